@@ -504,6 +504,33 @@ Widened widen_for_projection(fir_ctx& c, const Grid& g, const float* img)
   return Widened{d, d_t};
 }
 
+// The plan of a launch on transaxial tracks (column.cu), or tracks = 0 where
+// the LORs are traced one by one.
+ColumnPlan columns_for(fir_ctx& c, const Grid& g, const Sino& s, bool skip)
+{
+  ColumnPlan p = column_plan(g, s, c.scan_z.data(), c.block, skip);
+  if (!columns_pay(g, s, p, c.scan_z.data(), c.scan_diameter))
+  {
+    p.tracks = 0;
+  }
+  return p;
+}
+
+// The image's double copy and two zeroed accumulators in z columns, in context
+// scratch (acc may be null).
+const double* to_columns(fir_ctx& c, const Grid& g, const float* img, float** acc)
+{
+  const size_t n = (size_t)g.nxy * g.nz;
+  double* d = static_cast<double*>(c.wide.ensure(n * sizeof(double)));
+  if (acc != nullptr)
+  {
+    *acc = static_cast<float*>(c.bp_t.ensure(2 * n * sizeof(float)));
+  }
+  launch_to_columns(g, img, d, acc != nullptr ? *acc : nullptr, cfg_of(c));
+  after_launch(c);
+  return d;
+}
+
 // s with the compacted list of its bins whose measured value is not 0
 // (FIR_OPT_SKIP_ZERO_BINS), built on the context stream in context scratch.
 Sino nonzero_bins(fir_ctx& c, const Sino& s, const float* sino)
@@ -523,14 +550,39 @@ Sino nonzero_bins(fir_ctx& c, const Sino& s, const float* sino)
   return out;
 }
 
+// sino = the projection of img over s.
+void project_image(fir_ctx& c, const Grid& g, const Sino& s, const Tables& t, const float* img, float* sino,
+                   FwdEpilogue ep)
+{
+  const ColumnPlan plan = columns_for(c, g, s, false);
+  if (plan.tracks > 0)
+  {
+    const double* wide = to_columns(c, g, img, nullptr);
+    timed_launch(c, [&] { launch_column_forward(g, s, t, plan, wide, sino, ep, cfg_of(c)); });
+    return;
+  }
+  const Widened w = widen_for_projection(c, g, img);
+  timed_launch(c, [&] { launch_forward(g, s, t, w.img, w.img_t, sino, ep, cfg_of(c)); });
+}
+
 // img += backprojection of sino (nullptr: all ones) over the subset of s, in
 // the atomic mode; LORs running mostly along x accumulate in an x/y-exchanged
 // scratch image that is added into img afterwards, while both fit in L2.
 void backproject_subset(fir_ctx& c, const Grid& g, const Sino& s, const Tables& t, const float* sino, float* img,
                         bool skip_zero)
 {
-  float* img_t = nullptr;
+  const ColumnPlan plan = columns_for(c, g, s, skip_zero && sino != nullptr);
   const long long n = (long long)g.nxy * g.nz;
+  if (plan.tracks > 0)
+  {
+    float* acc = static_cast<float*>(c.bp_t.ensure(2 * (size_t)n * sizeof(float)));
+    cuda_ok(cudaMemsetAsync(acc, 0, 2 * (size_t)n * sizeof(float), c.stream), "cudaMemsetAsync");
+    timed_launch(c, [&] { launch_column_backward(g, s, t, plan, sino, acc, cfg_of(c)); });
+    launch_from_columns(g, acc, img, cfg_of(c));
+    after_launch(c);
+    return;
+  }
+  float* img_t = nullptr;
   if (use_exchanged(c, g, 8.0))
   {
     img_t = static_cast<float*>(c.bp_t.ensure((size_t)n * sizeof(float)));
@@ -546,6 +598,28 @@ void backproject_subset(fir_ctx& c, const Grid& g, const Sino& s, const Tables& 
   }
 }
 
+// Whether the fused sub-iteration runs on transaxial tracks; p is its plan.
+bool osem_columns(fir_ctx& c, const Grid& g, const Sino& s, ColumnPlan& p)
+{
+  if (c.backproj != FIR_BACKPROJ_ATOMIC || c.traversal != FIR_TRAVERSAL_EXACT)
+  {
+    return false;
+  }
+  p = columns_for(c, g, s, c.skip_zero != 0);
+  return p.tracks > 0;
+}
+
+// The backprojection of ratio_backproject in z columns (context scratch).
+const float* column_ratio_backproject(fir_ctx& c, const Grid& g, const Sino& s, const Tables& t,
+                                      const ColumnPlan& p, const float* img, const float* sino, const float* mult,
+                                      const float* bias)
+{
+  float* acc = nullptr;
+  const double* wide = to_columns(c, g, img, &acc);
+  timed_launch(c, [&] { launch_column_osem(g, s, t, p, wide, sino, mult, bias, acc, cfg_of(c)); });
+  return acc;
+}
+
 // bp (zeroed by the caller) += backprojection of sino / (projection of img +
 // bias) over the subset of s: the fused kernel, or in deterministic mode the
 // ratio kernel followed by the ordered scatter.  The fused kernel reads and
@@ -557,6 +631,14 @@ const float* ratio_backproject(fir_ctx& c, const Grid& g, const Sino& s_all, con
                                const float* sino, const float* mult, const float* bias, float* bp, long long nvox,
                                bool defer_merge = false)
 {
+  ColumnPlan plan;
+  if (osem_columns(c, g, s_all, plan))
+  {
+    const float* acc = column_ratio_backproject(c, g, s_all, t, plan, img, sino, mult, bias);
+    launch_from_columns(g, acc, bp, cfg_of(c));
+    after_launch(c);
+    return nullptr;
+  }
   // skipped bins: listed out of the atomic kernels' enumeration
   const bool listed = c.skip_zero != 0 && c.backproj == FIR_BACKPROJ_ATOMIC && s_all.n_enum > 0;
   const Sino s = listed ? nonzero_bins(c, s_all, sino) : s_all;
@@ -1022,17 +1104,26 @@ void osem_subiteration_device(fir_ctx& c, const ProjInfo& p, const Tables& t, co
                               const float* sens_frame, const fir_osem_params* prm, int subset,
                               int subiter)
 {
-  float* bp = static_cast<float*>(c.bp.ensure((size_t)v.nvox * sizeof(float)));
-  cuda_ok(cudaMemsetAsync(bp, 0, (size_t)v.nvox * sizeof(float), c.stream), "cudaMemsetAsync");
   const Sino s = sino_of(p, prm->n_subsets, subset);
-  const float* bp_t = ratio_backproject(c, g, s, t, img, sino, mult, bias, bp, v.nvox, true);
-  if (bp_t != nullptr)
+  ColumnPlan plan;
+  if (osem_columns(c, g, s, plan))
   {
-    launch_em_update_oriented(g.nx, g.ny, g.nz, img, bp, bp_t, sens_frame, cfg_of(c));
+    const float* acc = column_ratio_backproject(c, g, s, t, plan, img, sino, mult, bias);
+    launch_em_update_columns(g, img, acc, sens_frame, cfg_of(c));
   }
   else
   {
-    launch_em_update(v.nvox, img, bp, sens_frame, cfg_of(c));
+    float* bp = static_cast<float*>(c.bp.ensure((size_t)v.nvox * sizeof(float)));
+    cuda_ok(cudaMemsetAsync(bp, 0, (size_t)v.nvox * sizeof(float), c.stream), "cudaMemsetAsync");
+    const float* bp_t = ratio_backproject(c, g, s, t, img, sino, mult, bias, bp, v.nvox, true);
+    if (bp_t != nullptr)
+    {
+      launch_em_update_oriented(g.nx, g.ny, g.nz, img, bp, bp_t, sens_frame, cfg_of(c));
+    }
+    else
+    {
+      launch_em_update(v.nvox, img, bp, sens_frame, cfg_of(c));
+    }
   }
   after_launch(c);
   const bool conv = prm->convolution_interval > 0 && prm->fwhm_xyz[0] > 0.0 && prm->fwhm_xyz[1] > 0.0 &&
@@ -1587,6 +1678,8 @@ fir_status fir_ctx_set_scanner(fir_ctx* ctx, const fir_scanner_desc* scanner)
     c.z.ensure(s.z.size() * sizeof(double));
     cuda_ok(cudaMemcpy(c.xy.p, s.xy.data(), s.xy.size() * sizeof(double), cudaMemcpyHostToDevice), "cudaMemcpy");
     cuda_ok(cudaMemcpy(c.z.p, s.z.data(), s.z.size() * sizeof(double), cudaMemcpyHostToDevice), "cudaMemcpy");
+    c.scan_z = s.z;
+    c.scan_diameter = 2.0 * std::hypot(s.xy[0], s.xy[1]);
     c.scan_rings = s.n_rings;
     c.scan_cpr = s.n_cpr;
     c.have_scanner = true;
@@ -1615,9 +1708,7 @@ fir_status fir_forward(fir_ctx* ctx, const fir_vol_desc* vol, const float* img, 
     Stager st(c);
     const float* dimg = st.in(img, v.nvox);
     float* dsino = st.out(sino, p.g.n_bins);
-    const Sino s = sino_of(p, 1, 0);
-    const Widened w = widen_for_projection(c, g, dimg);
-    timed_launch(c, [&] { launch_forward(g, s, t, w.img, w.img_t, dsino, FwdEpilogue::None, cfg_of(c)); });
+    project_image(c, g, sino_of(p, 1, 0), t, dimg, dsino, FwdEpilogue::None);
     finish(c, st);
   });
 }
@@ -1634,9 +1725,7 @@ fir_status fir_forward_exp(fir_ctx* ctx, const fir_vol_desc* vol, const float* m
     Stager st(c);
     const float* dmu = st.in(mu, v.nvox);
     float* dacf = st.out(acf, p.g.n_bins);
-    const Sino s = sino_of(p, 1, 0);
-    const Widened w = widen_for_projection(c, g, dmu);
-    timed_launch(c, [&] { launch_forward(g, s, t, w.img, w.img_t, dacf, FwdEpilogue::Exp, cfg_of(c)); });
+    project_image(c, g, sino_of(p, 1, 0), t, dmu, dacf, FwdEpilogue::Exp);
     finish(c, st);
   });
 }

@@ -1,0 +1,774 @@
+// Projector kernels on transaxial tracks (column.cuh): forward projection,
+// backprojection and the fused OSEM sub-iteration, and the images in z
+// columns that they read and write.
+//
+// Blocks of 128 threads: with 256 the serial part of a track's construction
+// holds twice the warps (clinical forward projection 10.96 against 10.4 ms).
+// The projections run at 48 registers, the backprojection at 64: the gathers'
+// latency wants the warps (10.0 against 10.4 ms), the atomics do not (12.1
+// against 11.9).
+#include "column.cuh"
+
+#include <algorithm>
+#include <cmath>
+
+namespace fir
+{
+namespace
+{
+// One of a thread's two LORs: its ends in z and its bin.
+struct ColumnLor
+{
+  bool valid;
+  int pair;  // ring pair
+  int bin;
+  double z1, z2;
+};
+
+__device__ __forceinline__ int first_track(const ColumnPlan& p) { return blockIdx.x / p.blocks * p.per_block; }
+
+// The part of the launch that a warp's group (the block's warps that serve
+// its track) traces: ring pairs [begin, end) of one track.
+struct ColumnShare
+{
+  int group, warp;  // track within the block (the last one for warps past it), warp within the group
+  int sv, tang;
+  int begin, end;
+};
+
+__device__ __forceinline__ ColumnShare column_share(const Sino& s, const ColumnPlan& p, int first)
+{
+  const int warp = threadIdx.x >> 5;
+  ColumnShare c;
+  c.group = warp / p.warps;
+  c.warp = warp - c.group * p.warps;
+  const bool any = c.group < p.per_block && first + c.group < p.tracks;
+  c.group = min(c.group, p.per_block - 1);
+  const int vt = first + c.group;
+  c.sv = vt / s.n_tang;
+  c.tang = vt - c.sv * s.n_tang;
+  c.begin = (int)(blockIdx.x % p.blocks) * p.share;
+  c.end = any ? min(c.begin + p.share, p.pairs) : c.begin;
+  return c;
+}
+
+// Ring pair r of a track: its segment and plane.  The pairs are those of the
+// enumeration's segments in order; with p.interleave the planes of segments
+// 2k and 2k + 1 alternate, whose LORs lie half a ring spacing apart, so that
+// a warp's lanes share more of a column's sectors.
+__device__ __forceinline__ void ring_pair(const Sino& s, const ColumnPlan& p, int r, int& seg, int& axial)
+{
+  // the enumeration of a segment starts at tracks * its first ring pair
+  const int key = r * p.tracks;
+  int lo = 0, hi = s.n_segments;
+  while (hi - lo > 1)
+  {
+    const int mid = (lo + hi) >> 1;
+    if (s.enum_base[mid] <= key)
+      lo = mid;
+    else
+      hi = mid;
+  }
+  seg = lo;
+  axial = (key - s.enum_base[lo]) / p.tracks;
+  const int even = lo & ~1;
+  if (p.interleave && even + 1 < s.n_segments)
+  {
+    const int i = axial + (lo != even ? s.n_axial[even] : 0);
+    const int both = 2 * min(s.n_axial[even], s.n_axial[even + 1]);
+    // (the longer segment's last planes follow)
+    seg = i < both ? even + (i & 1) : (s.n_axial[even] > s.n_axial[even + 1] ? even : even + 1);
+    axial = i < both ? i >> 1 : i - (both >> 1);
+  }
+}
+
+__device__ __forceinline__ int column_bin(const Sino& s, const ColumnShare& c, int subset, int seg, int axial)
+{
+  return s.seg_base[seg] + ((c.sv * s.n_subsets + subset) * s.n_axial[seg] + axial) * s.n_tang + c.tang;
+}
+
+__device__ __forceinline__ ColumnLor column_lor(const Sino& s, const Tables& t, const ColumnPlan& p,
+                                                const ColumnShare& c, int subset, bool valid, int r)
+{
+  ColumnLor l{};
+  l.valid = valid;
+  if (valid)
+  {
+    int seg, axial, a1, a2;
+    l.pair = r;
+    ring_pair(s, p, r, seg, axial);
+    crystal_axial(s, seg - s.seg_offset, axial, a1, a2);
+    l.z1 = __ldg(t.z + a1);
+    l.z2 = __ldg(t.z + a2);
+    l.bin = column_bin(s, c, subset, seg, axial);
+  }
+  return l;
+}
+
+// Lists of the ring pairs whose bin is not 0, in shared memory: every warp
+// lists those of an equal part of its group's share, and counts them.
+struct NonzeroLists
+{
+  int* counts;           // of each warp
+  unsigned short* pairs; // share entries per group
+};
+
+__host__ __device__ constexpr int warp_part(int share, int warps) { return ((share + warps - 1) / warps + 31) / 32 * 32; }
+
+__device__ __forceinline__ void list_nonzero(const Sino& s, const ColumnPlan& p, const ColumnShare& c, int subset,
+                                             const float* __restrict__ sino, const NonzeroLists& l)
+{
+  const int lane = threadIdx.x & 31;
+  const int part = warp_part(p.share, p.warps);
+  unsigned short* list = l.pairs + (c.group * p.warps + c.warp) * part;
+  const int begin = c.begin + c.warp * part, end = min(begin + part, c.end);
+  int n = 0;
+  for (int r0 = begin; r0 < end; r0 += 32)
+  {
+    const int r = r0 + lane;
+    bool on = false;
+    if (r < end)
+    {
+      int seg, axial;
+      ring_pair(s, p, r, seg, axial);
+      on = __ldg(sino + column_bin(s, c, subset, seg, axial)) != 0.0f;
+    }
+    const unsigned mask = __ballot_sync(0xffffffffu, on);
+    if (on)
+    {
+      list[n + __popc(mask & ((1u << lane) - 1))] = (unsigned short)(r - c.begin);
+    }
+    n += __popc(mask);
+  }
+  if (lane == 0)
+  {
+    l.counts[threadIdx.x >> 5] = n;
+  }
+}
+
+// The LORs of a block that cannot use their track, in shared memory: they are
+// traced at the end, 32 to a warp, where a few of each warp's lanes would
+// hold up the others for a whole walk.
+struct Leftover
+{
+  int* count;
+  unsigned* lors;  // group << 16 | ring pair
+};
+
+__device__ __forceinline__ Leftover leftover(unsigned char* smem, const ColumnPlan& p)
+{
+  int* count = reinterpret_cast<int*>(smem + p.per_block * track_bytes(p.cap));
+  return Leftover{count, reinterpret_cast<unsigned*>(count + 4)};
+}
+
+// Calls trace(lor) for the warp's LORs, 64 at a time, two per lane: those of
+// its group's share in turn, or with kSkip those of them whose bin is not 0
+// (with a bin of 0 the ratio, or the value, is exactly 0, and so is every
+// contribution).  Every thread of the block calls this.
+template<bool kSkip, class Trace>
+__device__ __forceinline__ void column_each(const Sino& s, const Tables& t, const ColumnPlan& p,
+                                            const ColumnShare& c, int subset, const float* __restrict__ sino,
+                                            const NonzeroLists& lists, Trace&& trace)
+{
+  const int lane = threadIdx.x & 31;
+  int n = c.end - c.begin;
+  if (kSkip)
+  {
+    list_nonzero(s, p, c, subset, sino, lists);
+    __syncthreads();
+    n = 0;
+    for (int w = 0; w < p.warps && c.end > c.begin; ++w)
+    {
+      n += lists.counts[c.group * p.warps + w];
+    }
+  }
+  if constexpr (!kSkip)
+  {
+    ColumnLor lor[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+    {
+      const int i = c.warp * 64 + 32 * k + lane;
+      lor[k] = column_lor(s, t, p, c, subset, i < n, c.begin + i);
+    }
+    trace(lor);
+  }
+  else
+  {
+    for (int i0 = c.warp * 64; i0 < n; i0 += p.warps * 64)
+    {
+      ColumnLor lor[2];
+  #pragma unroll
+      for (int k = 0; k < 2; ++k)
+      {
+        int i = i0 + 32 * k + lane;
+        const bool valid = i < n;
+        if (valid)
+        {
+          int w = c.group * p.warps;
+          while (i >= lists.counts[w])
+          {
+            i -= lists.counts[w++];
+          }
+          i = lists.pairs[w * warp_part(p.share, p.warps) + i];
+        }
+        lor[k] = column_lor(s, t, p, c, subset, valid, c.begin + i);
+      }
+      trace(lor);
+    }
+  }
+}
+
+__device__ __forceinline__ NonzeroLists nonzero_lists(unsigned char* smem, const ColumnPlan& p)
+{
+  const Leftover l = leftover(smem, p);
+  int* counts = reinterpret_cast<int*>(l.lors + p.per_block * p.share);
+  return NonzeroLists{counts, reinterpret_cast<unsigned short*>(counts + 8)};
+}
+
+// The general walk in z columns, for the LORs that cannot use their track.
+// Not inlined: few lanes take it, and its registers are not the kernel's.
+// ok is false for a lane that hit the step bound.
+struct GeneralLine
+{
+  float line;
+  int ok;
+};
+
+__device__ __noinline__ GeneralLine general_line(const Grid& g, const TrackHead& h, double z1, double z2,
+                                           const double* __restrict__ img, int* check)
+{
+  const double e[6] = {h.x1, h.y1, z1, h.x2, h.y2, z2};
+  Walk w{};
+  const bool go = siddon_setup<true>(g, e, w);
+  float line = 0.0f;
+  const bool ok = siddon_walk<true>(g, w, go, [&](bool, int c, double len) {
+    line = accumulate(line, len, __ldg(img + (unsigned)c));
+  });
+  if (!ok)
+  {
+    flag(check, kCheckWalkGuard);
+  }
+  return GeneralLine{line, ok ? 1 : 0};
+}
+
+__device__ __noinline__ void general_scatter(const Grid& g, const TrackHead& h, double z1, double z2, double value,
+                                             float* acc, int* check)
+{
+  const double e[6] = {h.x1, h.y1, z1, h.x2, h.y2, z2};
+  Walk w{};
+  const bool go = siddon_setup<true>(g, e, w);
+  __builtin_assume(__isGlobal(acc));
+  const bool ok = siddon_walk<true>(g, w, go, [&](bool, int c, double len) {
+    atomicAdd(acc + c, __double2float_rn(dmul(len, value)));
+  });
+  if (!ok)
+  {
+    flag(check, kCheckWalkGuard);
+  }
+}
+
+// Sets up a lane's two LORs; go says which of them use the track.  Those that
+// need the general walk are left over.
+__device__ __forceinline__ void column_setup(const Grid& g, const Track& tr, const ColumnShare& c,
+                                             const ColumnLor lor[2], const Leftover& left, ColumnLane w[2],
+                                             bool go[2])
+{
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+  {
+    const int kind = lor[k].valid && tr.head->crosses ? lane_setup(g, *tr.head, lor[k].z1, lor[k].z2, w[k]) : kLorNone;
+    go[k] = kind == kLorColumn;
+    if (kind == kLorGeneral)
+    {
+      left.lors[atomicAdd(left.count, 1)] = (unsigned)c.group << 16 | (unsigned)lor[k].pair;
+    }
+  }
+}
+
+// Calls trace(lor, track) for the block's leftover LORs.  Every thread of the
+// block calls this.
+template<class Trace>
+__device__ __forceinline__ void column_leftover(const Sino& s, const Tables& t, const ColumnPlan& p, int subset,
+                                                int first, unsigned char* smem, const Leftover& left, Trace&& trace)
+{
+  __syncthreads();
+  for (int i = threadIdx.x; i < *left.count; i += blockDim.x)
+  {
+    const unsigned v = left.lors[i];
+    ColumnShare c;
+    c.group = (int)(v >> 16);
+    const int vt = first + c.group;
+    c.sv = vt / s.n_tang;
+    c.tang = vt - c.sv * s.n_tang;
+    trace(column_lor(s, t, p, c, subset, true, (int)(v & 0xffffu)), track_at(smem, p.cap, c.group));
+  }
+}
+
+// Line integrals of the image in z columns (VolData.cc:357-371).
+__device__ __forceinline__ void column_lines(const Track& tr, const bool go[2], const ColumnLane w[2],
+                                             const double* __restrict__ img, float line[2])
+{
+  LineSum sum[2] = {};
+  column_walk(
+    tr, w, go, [&](unsigned& at, ColumnState* st) { column_run_line(at, st, img, sum); },
+    [&](int k, int c, double len) {
+      sum[k].line = accumulate(sum[k].line, sum[k].len, sum[k].value);
+      sum[k].len = len;
+      sum[k].value = __ldg(img + (unsigned)c);
+    });
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+  {
+    line[k] = go[k] ? accumulate(sum[k].line, sum[k].len, sum[k].value) : 0.0f;
+  }
+}
+
+// acc += value along each LOR (VolData.cc:373-385).
+__device__ __forceinline__ void column_scatter(const Track& tr, const bool go[2], const ColumnLane w[2],
+                                               const double value[2], float* acc)
+{
+  __builtin_assume(__isGlobal(acc));
+  const bool all = __all_sync(0xffffffffu, go[0] && go[1]);
+  column_walk(
+    tr, w, go, [&](unsigned& at, ColumnState* st) { column_run_scatter(at, st, acc, value, go, all); },
+    [&](int k, int c, double len) { atomicAdd(acc + (unsigned)c, __double2float_rn(dmul(len, value[k]))); });
+}
+
+// exp evaluated in double and rounded once: the correctly rounded float
+// exponential that FIR's std::exp(float) returns (ProjData.cc:531).
+template<FwdEpilogue EP>
+__device__ __forceinline__ float epilogue(float line)
+{
+  if (EP == FwdEpilogue::Exp)
+  {
+    return (double)line > kEps ? __double2float_rn(exp((double)line)) : 1.0f;
+  }
+  return line;
+}
+
+// projections::forward (projections.cc:15-92), optionally with
+// ProjData::exponential (ProjData.cc:514-539).
+template<FwdEpilogue EP>
+__global__ void __launch_bounds__(256, 5) k_column_forward(const __grid_constant__ Grid g,
+                                                           const __grid_constant__ Sino s, Tables t, ColumnPlan p,
+                                                           const double* __restrict__ img, float* __restrict__ sino,
+                                                           int* check)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int first = first_track(p);
+  const Leftover left = leftover(smem, p);
+  build_tracks(g, s, t, p, s.subset, first, smem, left.count);
+  const ColumnShare c = column_share(s, p, first);
+  const Track tr = track_at(smem, p.cap, c.group);
+  column_each<false>(s, t, p, c, s.subset, nullptr, NonzeroLists{}, [&](const ColumnLor* lor) {
+    ColumnLane w[2] = {};
+    bool go[2];
+    float line[2];
+    column_setup(g, tr, c, lor, left, w, go);
+    column_lines(tr, go, w, img, line);
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+    {
+      if (lor[k].valid)
+      {
+        sino[lor[k].bin] = epilogue<EP>(line[k]);
+      }
+    }
+  });
+  column_leftover(s, t, p, s.subset, first, smem, left, [&](const ColumnLor& lor, const Track& own) {
+    sino[lor.bin] = epilogue<EP>(general_line(g, *own.head, lor.z1, lor.z2, img, check).line);
+  });
+}
+
+// A track's accumulator: tracks along x and along y add into one each, which
+// are summed at the end.  Each sum then rounds at half the size.
+__device__ __forceinline__ float* accumulator_of(const Grid& g, const TrackHead& h, float* acc)
+{
+  return acc + (h.crosses && h.along_x ? (size_t)g.nxy * g.nz : 0);
+}
+
+// projections::backward (projections.cc:94-184) into the accumulators in z
+// columns; sino == nullptr is the all-ones sinogram (projections.cc:186-197).
+template<bool kSkip>
+__global__ void __launch_bounds__(256, 4) k_column_backward(const __grid_constant__ Grid g,
+                                                            const __grid_constant__ Sino s, Tables t, ColumnPlan p,
+                                                            const float* __restrict__ sino, float* acc, int* check)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int first = first_track(p);
+  const Leftover left = leftover(smem, p);
+  build_tracks(g, s, t, p, s.subset, first, smem, left.count);
+  const ColumnShare c = column_share(s, p, first);
+  const Track tr = track_at(smem, p.cap, c.group);
+  column_each<kSkip>(s, t, p, c, s.subset, sino, nonzero_lists(smem, p), [&](const ColumnLor* lor) {
+    ColumnLane w[2] = {};
+    bool go[2];
+    double value[2];
+    column_setup(g, tr, c, lor, left, w, go);
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+    {
+      value[k] = lor[k].valid && sino != nullptr ? (double)__ldg(sino + lor[k].bin) : 1.0;
+    }
+    column_scatter(tr, go, w, value, accumulator_of(g, *tr.head, acc));
+  });
+  column_leftover(s, t, p, s.subset, first, smem, left, [&](const ColumnLor& lor, const Track& own) {
+    const double v = sino != nullptr ? (double)__ldg(sino + lor.bin) : 1.0;
+    general_scatter(g, *own.head, lor.z1, lor.z2, v, accumulator_of(g, *own.head, acc), check);
+  });
+}
+
+// measured / estimated of one bin (reconAlgos.cc:119-150, see osem_lor_body);
+// false where nothing is backprojected.
+template<bool kWeighted>
+__device__ __forceinline__ bool osem_ratio(float line, int bin, const float* __restrict__ sino,
+                                           const float* __restrict__ mult, const float* __restrict__ bias, double& q)
+{
+  const float m = kWeighted ? __ldg(mult + bin) : 1.0f;
+  if (kWeighted)
+  {
+    line = __fmul_rn(line, m);
+  }
+  if (bias != nullptr)
+  {
+    line = __fadd_rn(line, __ldg(bias + bin));
+  }
+  q = 0.0;
+  if (!((double)line > kEps))
+  {
+    return false;
+  }
+  const float r = __fdiv_rn(__ldg(sino + bin), line);
+  q = (double)(kWeighted ? __fmul_rn(r, m) : r);
+  return true;
+}
+
+// One OSEM sub-iteration (reconAlgos.cc:119-158, see osem_lor_body): image
+// and accumulators in z columns.
+template<bool kWeighted, bool kSkip>
+__global__ void __launch_bounds__(256, 5) k_column_osem(const __grid_constant__ Grid g,
+                                                        const __grid_constant__ Sino s, Tables t, ColumnPlan p,
+                                                        const double* __restrict__ img,
+                                                        const float* __restrict__ sino,
+                                                        const float* __restrict__ mult,
+                                                        const float* __restrict__ bias, float* acc, int* check)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int first = first_track(p);
+  const Leftover left = leftover(smem, p);
+  build_tracks(g, s, t, p, s.subset, first, smem, left.count);
+  const ColumnShare c = column_share(s, p, first);
+  const Track tr = track_at(smem, p.cap, c.group);
+  column_each<kSkip>(s, t, p, c, s.subset, sino, nonzero_lists(smem, p), [&](const ColumnLor* lor) {
+    ColumnLane w[2] = {};
+    bool go[2];
+    float line[2];
+    column_setup(g, tr, c, lor, left, w, go);
+    column_lines(tr, go, w, img, line);
+    double value[2] = {0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+    {
+      go[k] = go[k] && osem_ratio<kWeighted>(line[k], lor[k].bin, sino, mult, bias, value[k]);
+    }
+    column_scatter(tr, go, w, value, accumulator_of(g, *tr.head, acc));
+  });
+  column_leftover(s, t, p, s.subset, first, smem, left, [&](const ColumnLor& lor, const Track& own) {
+    const GeneralLine gl = general_line(g, *own.head, lor.z1, lor.z2, img, check);
+    double q;
+    if (osem_ratio<kWeighted>(gl.line, lor.bin, sino, mult, bias, q) && gl.ok)
+    {
+      general_scatter(g, *own.head, lor.z1, lor.z2, q, accumulator_of(g, *own.head, acc), check);
+    }
+  });
+}
+
+// Images between [z][y][x] and z columns, through 32 x 32 tiles of
+// (column, slice) in shared memory.  np = nx * ny.
+constexpr int kTile = 32, kTileRows = 8;
+
+dim3 column_tiles(int np, int nz)
+{
+  return dim3((unsigned)((np + kTile - 1) / kTile), (unsigned)((nz + kTile - 1) / kTile));
+}
+
+// out = the double copy of in in z columns; both accumulators at acc (or
+// null) = 0.
+__global__ void __launch_bounds__(kTile * kTileRows) k_to_columns(int np, int nz, const float* __restrict__ in,
+                                                                  double* __restrict__ out, float* __restrict__ acc)
+{
+  __shared__ float tile[kTile][kTile + 1];
+  const int p0 = blockIdx.x * kTile, z0 = blockIdx.y * kTile;
+  for (int j = threadIdx.y; j < kTile; j += kTileRows)
+  {
+    const int p = p0 + threadIdx.x, z = z0 + j;
+    if (p < np && z < nz)
+    {
+      tile[j][threadIdx.x] = in[(size_t)z * np + p];
+    }
+  }
+  __syncthreads();
+  for (int j = threadIdx.y; j < kTile; j += kTileRows)
+  {
+    const int z = z0 + threadIdx.x, p = p0 + j;
+    if (p < np && z < nz)
+    {
+      const size_t k = (size_t)p * nz + z;
+      out[k] = (double)tile[threadIdx.x][j];
+      if (acc != nullptr)
+      {
+        acc[k] = 0.0f;
+        acc[(size_t)np * nz + k] = 0.0f;
+      }
+    }
+  }
+}
+
+// out = the sum of the accumulators at acc in [z][y][x].
+__global__ void __launch_bounds__(kTile * kTileRows) k_from_columns(int np, int nz, const float* __restrict__ acc,
+                                                                    float* __restrict__ out)
+{
+  __shared__ float tile[kTile][kTile + 1];
+  const int p0 = blockIdx.x * kTile, z0 = blockIdx.y * kTile;
+  for (int j = threadIdx.y; j < kTile; j += kTileRows)
+  {
+    const int z = z0 + threadIdx.x, p = p0 + j;
+    if (p < np && z < nz)
+    {
+      tile[j][threadIdx.x] = __fadd_rn(acc[(size_t)p * nz + z], acc[(size_t)np * nz + (size_t)p * nz + z]);
+    }
+  }
+  __syncthreads();
+  for (int j = threadIdx.y; j < kTile; j += kTileRows)
+  {
+    const int p = p0 + threadIdx.x, z = z0 + j;
+    if (p < np && z < nz)
+    {
+      out[(size_t)z * np + p] = tile[threadIdx.x][j];
+    }
+  }
+}
+
+// k_em_update with the backprojection in z columns.
+__global__ void __launch_bounds__(kTile * kTileRows) k_em_update_columns(int np, int nz, float* __restrict__ img,
+                                                                         const float* __restrict__ acc,
+                                                                         const float* __restrict__ sens)
+{
+  __shared__ float tile[kTile][kTile + 1];
+  const int p0 = blockIdx.x * kTile, z0 = blockIdx.y * kTile;
+  for (int j = threadIdx.y; j < kTile; j += kTileRows)
+  {
+    const int z = z0 + threadIdx.x, p = p0 + j;
+    if (p < np && z < nz)
+    {
+      tile[j][threadIdx.x] = __fadd_rn(acc[(size_t)p * nz + z], acc[(size_t)np * nz + (size_t)p * nz + z]);
+    }
+  }
+  __syncthreads();
+  for (int j = threadIdx.y; j < kTile; j += kTileRows)
+  {
+    const int p = p0 + threadIdx.x, z = z0 + j;
+    if (p < np && z < nz)
+    {
+      const size_t k = (size_t)z * np + p;
+      const float b = tile[threadIdx.x][j];
+      const float sv = __ldg(sens + k);
+      const float q = ((double)b > kEps && (double)sv > kEps) ? __fdiv_rn(b, sv) : 0.0f;
+      const float v = img[k];
+      img[k] = ((double)v > kEps && (double)q > kEps) ? __fmul_rn(v, q) : 0.0f;
+    }
+  }
+}
+
+unsigned column_grid(const ColumnPlan& p)
+{
+  return (unsigned)((p.tracks + p.per_block - 1) / p.per_block * p.blocks);
+}
+
+// Shared memory above 48 KB is asked for once per kernel and call.
+template<typename K>
+void ask_shared(K kernel, size_t bytes)
+{
+  if (bytes > 48 * 1024)
+  {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  }
+}
+}  // namespace
+
+size_t column_smem(const ColumnPlan& p)
+{
+  const size_t lists = 8 * sizeof(int) + (size_t)(p.block / 32) * warp_part(p.share, p.warps) * sizeof(unsigned short);
+  return (size_t)p.per_block * (track_bytes(p.cap) + p.share * sizeof(unsigned)) + 4 * sizeof(int) +
+         (p.skip ? lists : 0);
+}
+
+ColumnPlan column_plan(const Grid& g, const Sino& s, const double* z, int block, bool skip)
+{
+  ColumnPlan p{};
+  for (int k = 0; k < s.n_segments; ++k)
+  {
+    p.pairs += s.n_axial[k];
+  }
+  p.tracks = p.pairs > 0 ? s.n_enum / p.pairs : 0;
+  p.cap = g.nx + g.ny;
+  p.skip = skip ? 1 : 0;
+  // neighbouring LORs of a segment lie one ring apart in z, or with a span half
+  // a ring
+  const double apart = s.n_rings > 1 ? std::fabs(z[2] - z[0]) * (s.span > 1 ? 0.5 : 1.0) : 0.0;
+  p.interleave = apart >= 1.6 * g.ext[2] ? 1 : 0;
+  // where bins are skipped a warp has room for two turns of 64: half of the
+  // bins are often 0, and warps without work would hold the block's registers
+  const int turn = skip ? 128 : 64;
+  const int warps = std::max((p.pairs + turn - 1) / turn, 1);
+  // a track's warps in equal blocks of nearly the wanted size: the count
+  // that leaves the fewest warps idle
+  const int want = block / 32;
+  int best = want, idle = 1 << 30;
+  for (int w : {want, want + 1, want - 1, want + 2})
+  {
+    if (w >= 1 && w <= 8)
+    {
+      const int off = warps >= w ? (warps + w - 1) / w * w - warps : (w % warps);
+      // (compared as a share of all warps)
+      if ((long long)off * 64 / std::max(warps, w) < idle)
+      {
+        idle = (int)((long long)off * 64 / std::max(warps, w));
+        best = w;
+      }
+    }
+  }
+  p.block = best * 32;
+  p.blocks = std::max((warps + best - 1) / best, 1);
+  p.warps = p.blocks > 1 ? best : warps;
+  p.share = p.blocks > 1 ? best * turn : std::max(p.pairs, 1);
+  p.per_block = best / p.warps;
+  return p;
+}
+
+// Share of the ring pairs whose LOR through the axis meets the volume but
+// enters or leaves it through an end face: those take the general walk.
+static double clipped_share(const Grid& g, const Sino& s, const double* z, double diameter)
+{
+  if (z[0] > g.low[2] && z[0] < g.high[2] && z[2 * s.n_rings - 2] > g.low[2] && z[2 * s.n_rings - 2] < g.high[2])
+  {
+    return 0.0;
+  }
+  const double across = std::max(g.high[0] - g.low[0], g.high[1] - g.low[1]);
+  const double in = std::max(0.5 * (diameter - across) / diameter, 0.0);
+  long long all = 0, clipped = 0;
+  for (int k = 0; k < s.n_segments; ++k)
+  {
+    for (int axial = 0; axial < s.n_axial[k]; ++axial)
+    {
+      int a1, a2;
+      crystal_axial(s, k - s.seg_offset, axial, a1, a2);
+      const double z1 = z[a1] + in * (z[a2] - z[a1]), z2 = z[a2] + in * (z[a1] - z[a2]);
+      const double lo = std::min(z1, z2), hi = std::max(z1, z2);
+      const bool meets = hi > g.low[2] && lo < g.high[2];
+      all += meets ? 1 : 0;
+      clipped += meets && (lo < g.low[2] || hi > g.high[2]) ? 1 : 0;
+    }
+  }
+  return all > 0 ? (double)clipped / all : 0.0;
+}
+
+// Mean number of z crossings that stop a warp's turn per crossing of its
+// track: the LORs of a segment cross together where their planes lie whole
+// voxels apart, so a segment counts once per distinct offset.
+static double stops_per_turn(const Grid& g, const Sino& s, const ColumnPlan& p, const double* z, double diameter)
+{
+  const double apart = s.n_rings > 1 ? std::fabs(z[2] - z[0]) * (s.span > 1 ? 0.5 : 1.0) / g.ext[2] : 0.0;
+  int offsets = 1;
+  while (offsets < 64 && std::fabs(offsets * apart - std::round(offsets * apart)) > 1e-3)
+  {
+    ++offsets;
+  }
+  // a line's mean step between transaxial crossings, and z's rise in it
+  const double step = 0.7853981633974483 * 0.5 * (g.ext[0] + g.ext[1]) / (diameter * g.ext[2]);
+  double sum = 0.0;
+  for (int k = 0; k < s.n_segments; ++k)
+  {
+    int a1, a2;
+    crystal_axial(s, k - s.seg_offset, s.n_axial[k] / 2, a1, a2);
+    sum += std::fabs(z[a2] - z[a1]) * step * std::min(offsets, s.n_axial[k]);
+  }
+  return sum / ((p.pairs + 63) / 64);
+}
+
+// Tracks need ring pairs to share them: below 48 most of a warp's 64 slots
+// are idle.  They also need about six warps per scheduler to hide the loops'
+// latency (a turn waits for its entry and test): the LOR-by-LOR kernels, with
+// twice the warps, are faster below that (measured 0.63x to 0.98x below 3000
+// warps, 1.3x and more above 8000).  A LOR clipped by the volume's ends walks
+// alone in its block's last pass (0.65x at 11 %, 1.14x at 2 %), and a stop
+// makes a turn nearly twice as long (1.1x at 3.2 stops per turn on small
+// volumes, 0.96x at 2.3 on a 320x320x128 one).
+bool columns_pay(const Grid& g, const Sino& s, const ColumnPlan& p, const double* z, double diameter)
+{
+  if (g.exact_only || p.pairs < 48 || (long long)p.tracks * ((p.pairs + 63) / 64) < 6 * 592 ||
+      column_smem(p) > 96 * 1024 || (long long)g.nxy * g.nz >= 1LL << 29)
+  {
+    return false;
+  }
+  return stops_per_turn(g, s, p, z, diameter) <= 2.2 && clipped_share(g, s, z, diameter) <= 0.04;
+}
+
+void launch_to_columns(const Grid& g, const float* in, double* out, float* acc, const LaunchCfg& cfg)
+{
+  k_to_columns<<<column_tiles(g.nxy, g.nz), dim3(kTile, kTileRows), 0, cfg.stream>>>(g.nxy, g.nz, in, out, acc);
+}
+
+void launch_from_columns(const Grid& g, const float* acc, float* out, const LaunchCfg& cfg)
+{
+  k_from_columns<<<column_tiles(g.nxy, g.nz), dim3(kTile, kTileRows), 0, cfg.stream>>>(g.nxy, g.nz, acc, out);
+}
+
+void launch_em_update_columns(const Grid& g, float* img, const float* acc, const float* sens, const LaunchCfg& cfg)
+{
+  k_em_update_columns<<<column_tiles(g.nxy, g.nz), dim3(kTile, kTileRows), 0, cfg.stream>>>(g.nxy, g.nz, img, acc,
+                                                                                            sens);
+}
+
+void launch_column_forward(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p, const double* img,
+                           float* sino, FwdEpilogue ep, const LaunchCfg& cfg)
+{
+  if (p.tracks == 0)
+  {
+    return;
+  }
+  const size_t bytes = column_smem(p);
+  auto* kernel = ep == FwdEpilogue::Exp ? k_column_forward<FwdEpilogue::Exp> : k_column_forward<FwdEpilogue::None>;
+  ask_shared(kernel, bytes);
+  kernel<<<column_grid(p), p.block, bytes, cfg.stream>>>(g, s, t, p, img, sino, cfg.check);
+}
+
+void launch_column_backward(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p, const float* sino,
+                            float* acc, const LaunchCfg& cfg)
+{
+  if (p.tracks == 0)
+  {
+    return;
+  }
+  const size_t bytes = column_smem(p);
+  auto* kernel = p.skip ? k_column_backward<true> : k_column_backward<false>;
+  ask_shared(kernel, bytes);
+  kernel<<<column_grid(p), p.block, bytes, cfg.stream>>>(g, s, t, p, sino, acc, cfg.check);
+}
+
+void launch_column_osem(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p, const double* img,
+                        const float* sino, const float* mult, const float* bias, float* acc, const LaunchCfg& cfg)
+{
+  if (p.tracks == 0)
+  {
+    return;
+  }
+  const size_t bytes = column_smem(p);
+  const bool skip = p.skip != 0;
+  auto* kernel = mult != nullptr ? (skip ? k_column_osem<true, true> : k_column_osem<true, false>)
+                                 : (skip ? k_column_osem<false, true> : k_column_osem<false, false>);
+  ask_shared(kernel, bytes);
+  kernel<<<column_grid(p), p.block, bytes, cfg.stream>>>(g, s, t, p, img, sino, mult, bias, acc, cfg.check);
+}
+}  // namespace fir

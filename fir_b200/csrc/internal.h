@@ -22,6 +22,25 @@ enum class FwdEpilogue
   Exp  // ProjData::exponential applied to the line integral (ACF)
 };
 
+// How a launch of column.cu deals LORs to threads.  Tracks are numbered
+// (view of the subset, tangential bin); a track's ring pairs in the
+// enumeration's order of (segment, axial plane).
+struct ColumnPlan
+{
+  int pairs;      // ring pairs per track
+  int tracks;     // tracks of the launch
+  int block;      // threads per block
+  int blocks;     // blocks per track
+  int share;      // ring pairs of a block's part of a track
+  int warps;      // warps of a block that serve one track
+  int per_block;  // tracks per block
+  int cap;        // crossings of a track: at most nx + ny
+  int skip;       // 1: bins that are 0 are skipped
+  int interleave; // 1: ring pairs of two neighbouring segments alternate
+};
+// Shared memory of one block.
+size_t column_smem(const ColumnPlan& p);
+
 struct LaunchCfg
 {
   int block;
@@ -49,6 +68,27 @@ void launch_osem_subset(const Grid& g, const Sino& s, const Tables& t, const dou
 void launch_osem_subset_float_image(const Grid& g, const Sino& s, const Tables& t, const float* img,
                                     const float* img_t, const float* sino, const float* mult, const float* bias,
                                     float* bp, float* bp_t, bool skip_zero, const LaunchCfg& cfg);
+// column.cu: the projectors on transaxial tracks (column.cuh), which read the
+// image as doubles in z columns ([y][x][z]) and add into two accumulators of
+// that layout, one after the other at acc, whose sum is the backprojection.
+// How a launch with blocks of about `block` threads deals the LORs of s (z: the
+// scanner's slice centres; skip: the projectors skip bins that are 0).
+ColumnPlan column_plan(const Grid& g, const Sino& s, const double* z, int block, bool skip);
+// Whether the launch is faster on tracks than LOR by LOR (z: the scanner's
+// slice centres, diameter: of a ring).
+bool columns_pay(const Grid& g, const Sino& s, const ColumnPlan& p, const double* z, double diameter);
+// out = the image's double copy in z columns; the accumulators (or null) = 0.
+void launch_to_columns(const Grid& g, const float* in, double* out, float* acc, const LaunchCfg& cfg);
+// out = the accumulators' sum in [z][y][x].
+void launch_from_columns(const Grid& g, const float* acc, float* out, const LaunchCfg& cfg);
+// launch_em_update with the backprojection in z columns (left as it is).
+void launch_em_update_columns(const Grid& g, float* img, const float* acc, const float* sens, const LaunchCfg& cfg);
+void launch_column_forward(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p, const double* img,
+                           float* sino, FwdEpilogue ep, const LaunchCfg& cfg);
+void launch_column_backward(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p, const float* sino,
+                            float* acc, const LaunchCfg& cfg);
+void launch_column_osem(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p, const double* img,
+                        const float* sino, const float* mult, const float* bias, float* acc, const LaunchCfg& cfg);
 // compact.cu: the enumerated indices of s (list null) whose bin of sino is
 // not 0, ascending, into list (s.n_enum entries), their number into *count
 // (device memory).  With temp null only *temp_bytes is set (CUB convention).

@@ -130,7 +130,7 @@ __device__ __forceinline__ int enum_index(const Sino& s, int i, bool& valid)
 }
 
 // ProjData::getCrystalAxialCoord (ProjData.cc:198-299): slice indices.
-__device__ __forceinline__ void crystal_axial(const Sino& s, int seg, int axial, int& a1, int& a2)
+__host__ __device__ __forceinline__ void crystal_axial(const Sino& s, int seg, int axial, int& a1, int& a2)
 {
   if (s.span == 1)
   {
@@ -284,8 +284,10 @@ struct Walk
 // Siddon::computePath setup (Siddon.cc:112-203 with dimSetup :260-317,
 // getEntryExit :319-334, getStartInd :336-350, prepareDim :352-377).
 // Returns false when the segment misses the volume.  With transpose the
-// linear index is that of the image with x and y exchanged ([z][x][y]); the
-// traversal itself is the same.
+// linear index is that of the image with x and y exchanged ([z][x][y]), with
+// kColumns that of the image in z columns ([y][x][z]); the traversal itself
+// is the same.
+template<bool kColumns = false>
 __device__ __forceinline__ bool siddon_setup(const Grid& g, const double e[6], Walk& w, bool transpose = false)
 {
   double diff[3], smin[3], smax[3], snext[3];
@@ -339,7 +341,8 @@ __device__ __forceinline__ bool siddon_setup(const Grid& g, const double e[6], W
     return false;
   }
   const int n[3] = {g.nx, g.ny, g.nz};
-  const int stride[3] = {transpose ? g.ny : 1, transpose ? 1 : g.nx, g.nxy};
+  const int stride[3] = {kColumns ? g.nz : (transpose ? g.ny : 1), kColumns ? g.nx * g.nz : (transpose ? 1 : g.nx),
+                         kColumns ? 1 : g.nxy};
   w.tr = transpose ? 1 : 0;
   double rdiff[3];
 #pragma unroll
@@ -434,10 +437,11 @@ __device__ __forceinline__ double walk_step(Walk& w, double prev, bool& more, Em
 
 // Advances left in each dimension, from the linear index (every index is
 // inside the volume when this is called).
+template<bool kColumns>
 __device__ __forceinline__ void left_from_index(const Grid& g, Walk& w)
 {
-  const int z = w.c / g.nxy;
-  const int rest = w.c - z * g.nxy;
+  const int z = kColumns ? w.c % g.nz : w.c / g.nxy;
+  const int rest = kColumns ? w.c / g.nz : w.c - z * g.nxy;
   const int slow = rest / (w.tr ? g.ny : g.nx);
   const int fast = rest - slow * (w.tr ? g.ny : g.nx);
   const int idx[3] = {w.tr ? slow : fast, w.tr ? fast : slow, z};
@@ -480,7 +484,7 @@ __device__ __forceinline__ void left_from_index(const Grid& g, Walk& w)
 // of these steps (a >= EPS, s < 2^-1042).  The running sums are therefore
 // FIR's, and one select of a 32-bit word replaces the compiler's select of
 // both words of a conditionally added alpha.
-template<class Emit>
+template<bool kColumns, class Emit>
 __device__ __forceinline__ void walk_loop_fast(const Grid& g, Walk& w, double& prev, bool active, Emit&& emit)
 {
   double end = w.amax;
@@ -535,7 +539,7 @@ __device__ __forceinline__ void walk_loop_fast(const Grid& g, Walk& w, double& p
       }
       step(m);
     }
-    left_from_index(g, w);
+    left_from_index<kColumns>(g, w);
   }
   bool more = active;
   while (more)
@@ -570,19 +574,20 @@ __device__ __forceinline__ void walk_loop_exact(Walk& w, double& prev, int& guar
 // this together (it votes on the tie form); a kernel that traverses twice
 // per lane calls __syncwarp() between the traversals.  Returns false for a
 // lane that hit the step bound, which only non-finite input can cause.
-template<class Emit>
+template<bool kColumns = false, class Emit>
 __device__ __forceinline__ bool siddon_walk(const Grid& g, Walk w, bool go, Emit&& emit)
 {
   double prev = w.amin;
   int guard = g.guard;
   const bool active = go && prev < w.amax;
-  // every alpha of the walk is >= the smallest initial one (alphas only
-  // grow, alphaMax > alphaMin), so this decides the tie form for the walk
-  const bool fast =
-    !active || (!g.exact_only && min_of(w.amin, min_of(w.a[0], min_of(w.a[1], w.a[2]))) >= kEps);
+  // the tie test compares crossings only, and they only grow (alphaMin, which
+  // is 0 where a crystal lies inside the volume, enters the first length
+  // alone; nothing is decided after a step that ends at alphaMax), so the
+  // smallest first crossing decides the tie form for the walk
+  const bool fast = !active || (!g.exact_only && min_of(w.a[0], min_of(w.a[1], w.a[2])) >= kEps);
   if (__all_sync(__activemask(), fast))
   {
-    walk_loop_fast(g, w, prev, active, emit);
+    walk_loop_fast<kColumns>(g, w, prev, active, emit);
   }
   else
   {
