@@ -117,20 +117,37 @@ __global__ void __launch_bounds__(256, 4) k_batch_osem(const BatchProblem* __res
   }
 }
 
+// A thread's voxel.  A unit is a block of kBatchBlock consecutive voxels, or
+// for a problem with columns a tile of 32 columns x 8 slices: a warp's 32
+// voxels are consecutive in x (and y) either way, and the tile's part of a
+// column is one sector.
 struct Voxel
 {
   const BatchProblem* pb;
   const BatchItem* item;
-  int j;  // linear voxel index within the problem; -1 past its end
+  int j;       // linear voxel index within the problem; -1 past its end
+  int p0, z0;  // first column and slice of the tile
 };
+
+constexpr int kTileColumns = 32, kTileSlices = kBatchBlock / kTileColumns;
 
 __device__ __forceinline__ Voxel voxel_of(const BatchProblem* P, const BatchItem* items, int n_items)
 {
   const int it = find_item(items, n_items, blockIdx.x);
-  Voxel v;
+  Voxel v{};
   v.item = items + it;
   v.pb = P + __ldg(&items[it].problem);
-  v.j = (blockIdx.x - __ldg(&items[it].unit_begin)) * kBatchBlock + threadIdx.x;
+  const int unit = blockIdx.x - __ldg(&items[it].unit_begin);
+  if (v.pb->columns)
+  {
+    const int across = (v.pb->g.nxy + kTileColumns - 1) / kTileColumns;
+    v.p0 = unit % across * kTileColumns;
+    v.z0 = unit / across * kTileSlices;
+    const int p = v.p0 + (int)(threadIdx.x & 31), z = v.z0 + (int)(threadIdx.x >> 5);
+    v.j = p < v.pb->g.nxy && z < v.pb->g.nz ? z * v.pb->g.nxy + p : -1;
+    return v;
+  }
+  v.j = unit * kBatchBlock + threadIdx.x;
   if (v.j >= v.pb->nvox)
   {
     v.j = -1;
@@ -147,6 +164,88 @@ __device__ __forceinline__ int exchanged(const BatchProblem& pb, int j)
   return (r / pb.g.ny * pb.g.nx + x) * pb.g.ny + y;
 }
 
+// A tile of a problem with columns, turned between the two orders of its
+// voxels: the block's threads along x, or along z within a column.
+struct Tile
+{
+  float v[kTileSlices][kTileColumns + 1];
+};
+
+// Element of the accumulators and the double copy that thread tid moves; -1
+// past the volume.
+__device__ __forceinline__ int tile_element(const Voxel& v, int& slice, int& column)
+{
+  slice = threadIdx.x % kTileSlices;
+  column = threadIdx.x / kTileSlices;
+  const int p = v.p0 + column, z = v.z0 + slice;
+  return p < v.pb->g.nxy && z < v.pb->g.nz ? p * v.pb->g.nz + z : -1;
+}
+
+// The projector's copies of the thread's voxel get its new value x.  Every
+// thread of a block with columns calls this.
+__device__ __forceinline__ void refresh(const Voxel& v, float x, Tile& tile)
+{
+  const BatchProblem& pb = *v.pb;
+  if (pb.columns)
+  {
+    tile.v[threadIdx.x >> 5][threadIdx.x & 31] = x;
+    __syncthreads();
+    int slice, column;
+    const int k = tile_element(v, slice, column);
+    if (k >= 0)
+    {
+      pb.wide[k] = (double)tile.v[slice][column];
+    }
+    return;
+  }
+  if (pb.wide != nullptr)
+  {
+    pb.wide[v.j] = (double)x;
+  }
+  if (pb.wide_t != nullptr)
+  {
+    pb.wide_t[exchanged(pb, v.j)] = (double)x;
+  }
+  if (pb.img_t != nullptr)
+  {
+    pb.img_t[exchanged(pb, v.j)] = x;
+  }
+}
+
+// The backprojection so far of the thread's voxel; clears it.  Every thread
+// of a block with columns calls this.
+__device__ __forceinline__ float take_backprojection(const Voxel& v, Tile& tile)
+{
+  const BatchProblem& pb = *v.pb;
+  if (pb.columns)
+  {
+    int slice, column;
+    const int k = tile_element(v, slice, column);
+    if (k >= 0)
+    {
+      float* const a = pb.bp + k;
+      float* const c = a + pb.nvox;
+      const float va = *a, vc = *c;
+      tile.v[slice][column] = __fadd_rn(va, vc);
+      *a = 0.0f;
+      *c = 0.0f;
+    }
+    __syncthreads();
+    const float b = tile.v[threadIdx.x >> 5][threadIdx.x & 31];
+    __syncthreads();
+    return b;
+  }
+  float b = pb.bp[v.j];
+  pb.bp[v.j] = 0.0f;
+  if (pb.bp_t != nullptr)
+  {
+    const int jt = exchanged(pb, v.j);
+    b = __fadd_rn(b, pb.bp_t[jt]);
+    pb.bp_t[jt] = 0.0f;
+  }
+  return b;
+}
+
 __device__ __forceinline__ double radius_at(const BatchProblem& pb, int j)
 {
   const int x = j % pb.g.nx;
@@ -160,39 +259,28 @@ __global__ void __launch_bounds__(kBatchBlock) k_batch_prepare(const BatchProble
                                                                const BatchItem* __restrict__ items, int n_items,
                                                                int write_img)
 {
+  __shared__ Tile tile;
   const Voxel v = voxel_of(P, items, n_items);
-  if (v.j < 0)
+  const BatchProblem& pb = *v.pb;
+  if (v.j < 0 && !pb.columns)
   {
     return;
   }
-  const BatchProblem& pb = *v.pb;
-  float x = pb.img[v.j];
-  if (pb.cut > 0.0f && radius_at(pb, v.j) > (double)pb.cut)
+  float x = 0.0f;
+  if (v.j >= 0)
   {
-    x = 0.0f;
-  }
-  if (write_img)
-  {
-    pb.img[v.j] = x;
-  }
-  if (pb.wide != nullptr)
-  {
-    pb.wide[v.j] = (double)x;
-  }
-  pb.bp[v.j] = 0.0f;
-  if (pb.bp_t != nullptr)
-  {
-    const int jt = exchanged(pb, v.j);
-    if (pb.wide_t != nullptr)
+    x = pb.img[v.j];
+    if (pb.cut > 0.0f && radius_at(pb, v.j) > (double)pb.cut)
     {
-      pb.wide_t[jt] = (double)x;
+      x = 0.0f;
     }
-    if (pb.img_t != nullptr)
+    if (write_img)
     {
-      pb.img_t[jt] = x;
+      pb.img[v.j] = x;
     }
-    pb.bp_t[jt] = 0.0f;
   }
+  take_backprojection(v, tile);
+  refresh(v, x, tile);
 }
 
 // reconAlgos.cc:161-166 (VolData::operator/= then operator*=, VolData.cc:
@@ -201,43 +289,39 @@ __global__ void __launch_bounds__(kBatchBlock) k_batch_prepare(const BatchProble
 __global__ void __launch_bounds__(kBatchBlock) k_batch_em(const BatchProblem* __restrict__ P,
                                                           const BatchItem* __restrict__ items, int n_items)
 {
+  __shared__ Tile tile;
   const Voxel v = voxel_of(P, items, n_items);
-  if (v.j < 0)
+  const BatchProblem& pb = *v.pb;
+  if (v.j < 0 && !pb.columns)
   {
     return;
   }
-  const BatchProblem& pb = *v.pb;
-  const int jt = pb.bp_t != nullptr ? exchanged(pb, v.j) : -1;
-  const float b = jt >= 0 ? __fadd_rn(pb.bp[v.j], pb.bp_t[jt]) : pb.bp[v.j];
-  const float s = __ldg(pb.sens + (size_t)__ldg(&v.item->subset) * pb.nvox + v.j);
-  const float q = ((double)b > kEps && (double)s > kEps) ? __fdiv_rn(b, s) : 0.0f;
-  const float x0 = pb.img[v.j];
-  float x = ((double)x0 > kEps && (double)q > kEps) ? __fmul_rn(x0, q) : 0.0f;
-  pb.bp[v.j] = 0.0f;
-  if (jt >= 0)
+  // (read ahead of the tile's turn, whose stores hold back what follows)
+  const int filter = __ldg(&v.item->filter);
+  float* const img = pb.img;
+  const float cut = pb.cut;
+  float s = 0.0f, x0 = 0.0f;
+  if (v.j >= 0)
   {
-    pb.bp_t[jt] = 0.0f;
+    s = __ldg(pb.sens + (size_t)__ldg(&v.item->subset) * pb.nvox + v.j);
+    x0 = img[v.j];
   }
-  if (!__ldg(&v.item->filter))
+  const float b = take_backprojection(v, tile);
+  float x = 0.0f;
+  if (v.j >= 0)
   {
-    if (pb.cut > 0.0f && radius_at(pb, v.j) > (double)pb.cut)
+    const float q = ((double)b > kEps && (double)s > kEps) ? __fdiv_rn(b, s) : 0.0f;
+    x = ((double)x0 > kEps && (double)q > kEps) ? __fmul_rn(x0, q) : 0.0f;
+    if (!filter && cut > 0.0f && radius_at(pb, v.j) > (double)cut)
     {
       x = 0.0f;
     }
-    if (pb.wide != nullptr)
-    {
-      pb.wide[v.j] = (double)x;
-    }
-    if (jt >= 0 && pb.wide_t != nullptr)
-    {
-      pb.wide_t[jt] = (double)x;
-    }
-    if (jt >= 0 && pb.img_t != nullptr)
-    {
-      pb.img_t[jt] = x;
-    }
+    img[v.j] = x;
   }
-  pb.img[v.j] = x;
+  if (!filter)
+  {
+    refresh(v, x, tile);
+  }
 }
 
 // One pass of operations::convolve (operations.cc:84-156).  The z pass
@@ -248,74 +332,71 @@ template<int AXIS>
 __global__ void __launch_bounds__(kBatchBlock) k_batch_filter(const BatchProblem* __restrict__ P,
                                                               const BatchItem* __restrict__ items, int n_items)
 {
+  __shared__ Tile tile;
   const Voxel v = voxel_of(P, items, n_items);
-  if (v.j < 0)
+  const BatchProblem& pb = *v.pb;
+  if (v.j < 0 && !(AXIS == 2 && pb.columns))
   {
     return;
   }
-  const BatchProblem& pb = *v.pb;
-  const int nx = pb.g.nx, ny = pb.g.ny, nz = pb.g.nz;
-  const int j = v.j;
-  const Taps& taps = AXIS == 0 ? pb.tx : (AXIS == 1 ? pb.ty : pb.tz);
-  const float* in = AXIS == 0 ? pb.img : (AXIS == 1 ? pb.t1 : pb.t2);
-  const int coord = AXIS == 0 ? j % nx : (AXIS == 1 ? (j / nx) % ny : j / (nx * ny));
-  const int len = AXIS == 0 ? nx : (AXIS == 1 ? ny : nz);
-  const int stride = AXIS == 0 ? 1 : (AXIS == 1 ? nx : nx * ny);
-  const int half = taps.half;
-  float sum = 0.0f, norm = 0.0f;
-  for (int k = -half; k <= half; ++k)
+  float x = 0.0f;
+  if (v.j >= 0)
   {
-    const int c = coord + k;
-    if (c >= 0 && c < len)
+    const int nx = pb.g.nx, ny = pb.g.ny, nz = pb.g.nz;
+    const int j = v.j;
+    const Taps& taps = AXIS == 0 ? pb.tx : (AXIS == 1 ? pb.ty : pb.tz);
+    const float* in = AXIS == 0 ? pb.img : (AXIS == 1 ? pb.t1 : pb.t2);
+    const int coord = AXIS == 0 ? j % nx : (AXIS == 1 ? (j / nx) % ny : j / (nx * ny));
+    const int len = AXIS == 0 ? nx : (AXIS == 1 ? ny : nz);
+    const int stride = AXIS == 0 ? 1 : (AXIS == 1 ? nx : nx * ny);
+    const int half = taps.half;
+    float sum = 0.0f, norm = 0.0f;
+    for (int k = -half; k <= half; ++k)
     {
-      const float kv = taps.w[half + k];
-      sum = __fadd_rn(sum, __fmul_rn(kv, __ldg(in + j + k * stride)));
-      norm = __fadd_rn(norm, kv);
-    }
-  }
-  if (AXIS == 0)
-  {
-    if (norm > 0.0f)
-    {
-      pb.t1[j] = __fdiv_rn(sum, norm);
-    }
-  }
-  else if (AXIS == 1)
-  {
-    if (norm > 0.0f)
-    {
-      pb.t2[j] = __fdiv_rn(sum, norm);
-    }
-  }
-  else
-  {
-    const float old = pb.img[j];
-    float x = norm > 0.0f ? __fdiv_rn(sum, norm) : old;
-    if (pb.cut > 0.0f)
-    {
-      const double r = radius_at(pb, j);
-      if (r >= __dsub_rn((double)pb.cut, __dmul_rn(5.0, (double)pb.fwhm)))
+      const int c = coord + k;
+      if (c >= 0 && c < len)
       {
-        x = old;
-      }
-      if (r > (double)pb.cut)
-      {
-        x = 0.0f;
+        const float kv = taps.w[half + k];
+        sum = __fadd_rn(sum, __fmul_rn(kv, __ldg(in + j + k * stride)));
+        norm = __fadd_rn(norm, kv);
       }
     }
-    pb.img[j] = x;
-    if (pb.wide != nullptr)
+    if (AXIS == 0)
     {
-      pb.wide[j] = (double)x;
+      if (norm > 0.0f)
+      {
+        pb.t1[j] = __fdiv_rn(sum, norm);
+      }
     }
-    if (pb.wide_t != nullptr)
+    else if (AXIS == 1)
     {
-      pb.wide_t[exchanged(pb, j)] = (double)x;
+      if (norm > 0.0f)
+      {
+        pb.t2[j] = __fdiv_rn(sum, norm);
+      }
     }
-    if (pb.img_t != nullptr)
+    else
     {
-      pb.img_t[exchanged(pb, j)] = x;
+      const float old = pb.img[j];
+      x = norm > 0.0f ? __fdiv_rn(sum, norm) : old;
+      if (pb.cut > 0.0f)
+      {
+        const double r = radius_at(pb, j);
+        if (r >= __dsub_rn((double)pb.cut, __dmul_rn(5.0, (double)pb.fwhm)))
+        {
+          x = old;
+        }
+        if (r > (double)pb.cut)
+        {
+          x = 0.0f;
+        }
+      }
+      pb.img[j] = x;
     }
+  }
+  if (AXIS == 2)
+  {
+    refresh(v, x, tile);
   }
 }
 }  // namespace
@@ -389,6 +470,15 @@ void launch_batch_filter(const BatchProblem* P, const BatchItem* items, int n_it
   {
     k_batch_filter<2><<<n_units, kBatchBlock, 0, stream>>>(P, items, n_items);
   }
+}
+
+long long batch_voxel_units(const BatchProblem& p)
+{
+  if (p.columns)
+  {
+    return (long long)((p.g.nxy + kTileColumns - 1) / kTileColumns) * ((p.g.nz + kTileSlices - 1) / kTileSlices);
+  }
+  return ((long long)p.nvox + kBatchBlock - 1) / kBatchBlock;
 }
 
 long long batch_bundles(const Sino& s, int axial_tile)

@@ -509,7 +509,7 @@ Widened widen_for_projection(fir_ctx& c, const Grid& g, const float* img)
 ColumnPlan columns_for(fir_ctx& c, const Grid& g, const Sino& s, bool skip)
 {
   ColumnPlan p = column_plan(g, s, c.scan_z.data(), c.block, skip);
-  if (!columns_pay(g, s, p, c.scan_z.data(), c.scan_diameter))
+  if (column_warps(p) < kColumnWarps || !columns_pay(g, s, p, c.scan_z.data(), c.scan_diameter))
   {
     p.tracks = 0;
   }

@@ -3,6 +3,7 @@
 #include "capi_common.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <memory>
 #include <vector>
@@ -48,6 +49,8 @@ struct fir_batch
     // the projector runs as fir_osem's kernel in launches of its own, its
     // descriptor as kernel parameters (kDirectLors)
     bool direct = false;
+    bool columns = false;  // the projector runs on transaxial tracks (column.cu)
+    ColumnPlan plan{};     // of its own launches (direct)
     double path = 0.0;  // nx + ny + nz: relative cost of a bundle
     size_t off_sino = 0, off_sens = 0, off_img = 0, off_wide = 0, off_bp = 0, off_wide_t = 0, off_bp_t = 0,
            off_img_t = 0, off_t1 = 0, off_t2 = 0, off_xy = 0, off_z = 0;
@@ -59,7 +62,7 @@ struct fir_batch
   };
   struct Step
   {
-    Launch proj, em, filt;
+    Launch proj, tracks, em, filt;  // proj: LOR by LOR; tracks: problems with columns
     std::vector<std::pair<int, int>> direct;  // (problem, subset) of the direct projector launches
   };
 
@@ -68,12 +71,16 @@ struct fir_batch
   int n_sms = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_in = nullptr, ev_out = nullptr;
+  cudaStream_t side = nullptr;  // the LOR-by-LOR projector beside the one on tracks
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   std::vector<Problem> pr;
   std::vector<BatchProblem> desc_host;
   DevBuf arena, desc, items, queue;
   Launch all;
   std::vector<Step> steps;
   BatchLaunch shape{128, 0, 1};
+  size_t track_bytes = 0;  // shared memory of the batched projector on tracks
+  bool skip_zero = false;
   // the last fir_batch_tune: every candidate shape with its best time (ms)
   std::vector<std::pair<BatchLaunch, double>> tuned;
   cudaGraph_t graph = nullptr;
@@ -135,9 +142,19 @@ void release_batch(fir_batch& b)
   {
     cudaEventDestroy(b.ev_out);
   }
-  if (b.stream != nullptr)
+  for (cudaEvent_t e : {b.ev_fork, b.ev_join})
   {
-    cudaStreamDestroy(b.stream);
+    if (e != nullptr)
+    {
+      cudaEventDestroy(e);
+    }
+  }
+  for (cudaStream_t s : {b.stream, b.side})
+  {
+    if (s != nullptr)
+    {
+      cudaStreamDestroy(s);
+    }
   }
 }
 
@@ -179,6 +196,16 @@ void batch_project(fir_batch& b, const fir_batch::Launch& L, int* queue, const B
   check_launch(s);
 }
 
+// Enqueues the step's batched projector on transaxial tracks.
+void batch_project_tracks(fir_batch& b, const fir_batch::Launch& L, cudaStream_t s)
+{
+  const auto* P = static_cast<const BatchProblem*>(b.desc.p);
+  const auto* I = static_cast<const BatchItem*>(b.items.p) + L.item_off;
+  launch_batch_column_osem(P, I, L.n_items, L.n_units, b.track_bytes, b.skip_zero,
+                           static_cast<int*>(b.ctx->check.p), s);
+  check_launch(s);
+}
+
 // Enqueues problem k's projector for one subset as fir_osem runs it (one
 // launch, two when it gathers floats); returns the number of launches.
 long long direct_project(fir_batch& b, int k, int subset, cudaStream_t s)
@@ -187,6 +214,12 @@ long long direct_project(fir_batch& b, int k, int subset, cudaStream_t s)
   Sino sub = d.s;
   sub.subset = subset;
   const LaunchCfg cfg{b.ctx->block, s, static_cast<int*>(b.ctx->check.p)};
+  if (b.pr[(size_t)k].columns)
+  {
+    launch_column_osem(d.g, sub, d.t, b.pr[(size_t)k].plan, d.wide, d.sino, nullptr, d.bias, d.bp, cfg);
+    check_launch(s);
+    return 1;
+  }
   if (b.pr[(size_t)k].gather_float)
   {
     launch_osem_subset_float_image(d.g, sub, d.t, d.img, d.img_t, d.sino, nullptr, d.bias, d.bp, d.bp_t,
@@ -213,8 +246,26 @@ long long batch_enqueue(fir_batch& b, cudaStream_t s)
   for (size_t t = 0; t < b.steps.size(); ++t)
   {
     const fir_batch::Step& st = b.steps[t];
-    batch_project(b, st.proj, queue + t, b.shape, s);
+    // the two projector launches write different problems: side by side,
+    // neither's last blocks leave SMs idle
+    const bool both = st.proj.n_items > 0 && st.tracks.n_items > 0;
+    if (both)
+    {
+      cuda_ok(cudaEventRecord(b.ev_fork, s), "cudaEventRecord");
+      cuda_ok(cudaStreamWaitEvent(b.side, b.ev_fork, 0), "cudaStreamWaitEvent");
+    }
+    batch_project(b, st.proj, queue + t, b.shape, both ? b.side : s);
+    if (both)
+    {
+      cuda_ok(cudaEventRecord(b.ev_join, b.side), "cudaEventRecord");
+    }
     n += st.proj.n_items > 0 ? 1 : 0;
+    batch_project_tracks(b, st.tracks, s);
+    if (both)
+    {
+      cuda_ok(cudaStreamWaitEvent(s, b.ev_join, 0), "cudaStreamWaitEvent");
+    }
+    n += st.tracks.n_items > 0 ? 1 : 0;
     for (const auto& ks : st.direct)
     {
       n += direct_project(b, ks.first, ks.second, s);
@@ -257,8 +308,9 @@ void build_schedule(fir_batch& b)
   {
     all[(size_t)k] = k;
   }
-  auto vox_units = [&](int k) { return (b.pr[(size_t)k].v.nvox + kBatchBlock - 1) / kBatchBlock; };
+  auto vox_units = [&](int k) { return batch_voxel_units(b.desc_host[(size_t)k]); };
   auto lor_units = [&](int k) { return batch_bundles(b.desc_host[(size_t)k].s, b.shape.axial_tile); };
+  auto track_units = [&](int k) { return (long long)column_blocks(b.desc_host[(size_t)k].plan); };
   b.all = add_launch(items, all, zeros, zeros, vox_units);
   std::vector<int> order = all;
   std::stable_sort(order.begin(), order.end(),
@@ -270,7 +322,7 @@ void build_schedule(fir_batch& b)
   }
   for (int t = 0; t < n_steps; ++t)
   {
-    std::vector<int> probs, subs, filts, fprobs, fsubs, fflags, dprobs, dsubs, dfilts;
+    std::vector<int> probs, subs, filts, fprobs, fsubs, fflags, dprobs, dsubs, dfilts, tprobs, tsubs, tfilts;
     fir_batch::Step st;
     for (int k : order)
     {
@@ -288,6 +340,12 @@ void build_schedule(fir_batch& b)
       {
         st.direct.emplace_back(k, t % q.n_subsets);
       }
+      else if (q.columns)
+      {
+        tprobs.push_back(k);
+        tsubs.push_back(t % q.n_subsets);
+        tfilts.push_back(f);
+      }
       else
       {
         dprobs.push_back(k);
@@ -302,6 +360,7 @@ void build_schedule(fir_batch& b)
       }
     }
     st.proj = add_launch(items, dprobs, dsubs, dfilts, lor_units);
+    st.tracks = add_launch(items, tprobs, tsubs, tfilts, track_units);
     st.em = add_launch(items, probs, subs, filts, vox_units);
     st.filt = add_launch(items, fprobs, fsubs, fflags, vox_units);
     b.steps.push_back(st);
@@ -315,7 +374,8 @@ void build_schedule(fir_batch& b)
   b.schedule_launches = 1;
   for (const auto& st : b.steps)
   {
-    b.schedule_launches += 1 + (st.proj.n_items > 0 ? 1 : 0) + (st.filt.n_items > 0 ? 3 : 0);
+    b.schedule_launches += 1 + (st.proj.n_items > 0 ? 1 : 0) + (st.tracks.n_items > 0 ? 1 : 0) +
+                           (st.filt.n_items > 0 ? 3 : 0);
     for (const auto& ks : st.direct)
     {
       const BatchProblem& d = b.desc_host[(size_t)ks.first];
@@ -410,17 +470,47 @@ fir_status fir_batch_create(fir_batch** out, fir_ctx* ctx, int n_problems, const
       q.filter = q.prm.convolution_interval > 0 && q.prm.fwhm_xyz[0] > 0.0f && q.prm.fwhm_xyz[1] > 0.0f &&
                  q.prm.fwhm_xyz[2] > 0.0f;
       q.path = (double)q.v.d.nx + q.v.d.ny + q.v.d.nz;
+    }
+    // the projector's plans on transaxial tracks, of the problems that they pay
+    // for; together they need the warps that a launch alone would (column.cu)
+    fir_ctx geo;
+    geo.geometry = c.geometry;
+    b->skip_zero = c.skip_zero != 0;
+    std::vector<ColumnPlan> plans((size_t)n_problems);
+    std::vector<char> pays((size_t)n_problems, 0);
+    long long track_warps = 0;
+    for (int k = 0; k < n_problems; ++k)
+    {
+      fir_batch::Problem& q = b->pr[(size_t)k];
+      const Grid g = grid_of(geo, q.v);
+      const Sino s = sino_of(q.p, q.n_subsets, 0);
+      const ScannerInfo& sc = scan[(size_t)k];
+      plans[(size_t)k] = column_plan(g, s, sc.z.data(), kBatchColumnBlock, b->skip_zero, true);
+      q.plan = column_plan(g, s, sc.z.data(), c.block, b->skip_zero);
+      if (columns_pay(g, s, plans[(size_t)k], sc.z.data(), 2.0 * std::hypot(sc.xy[0], sc.xy[1])))
+      {
+        pays[(size_t)k] = 1;
+        track_warps += column_warps(plans[(size_t)k]);
+      }
+    }
+    const bool use_columns = c.step_limit == 0 && track_warps >= kColumnWarps;
+    auto columns_of = [&](int k) { return pays[(size_t)k] != 0; };
+    for (int k = 0; k < n_problems; ++k)
+    {
+      fir_batch::Problem& q = b->pr[(size_t)k];
       const size_t nv = (size_t)q.v.nvox;
       q.off_sino = take((size_t)q.p.g.n_bins * sizeof(float));
       q.off_sens = take(nv * q.n_subsets * sizeof(float));
       q.off_img = take(nv * sizeof(float));
       {
         const Grid g = grid_of(c, q.v);
-        q.exchanged = use_exchanged(c, g);
-        q.gather_float = !q.exchanged && !use_exchanged(c, g, 12.0) && use_exchanged(c, g, 8.0);
+        q.columns = use_columns && columns_of(k);
+        q.exchanged = !q.columns && use_exchanged(c, g);
+        q.gather_float =
+          !q.columns && !q.exchanged && !use_exchanged(c, g, 12.0) && use_exchanged(c, g, 8.0);
       }
       q.off_wide = take(q.gather_float ? 0 : nv * sizeof(double));
-      q.off_bp = take(nv * sizeof(float));
+      q.off_bp = take((q.columns ? 2 : 1) * nv * sizeof(float));
       q.off_wide_t = take(q.exchanged ? nv * sizeof(double) : 0);
       q.off_bp_t = take(q.exchanged || q.gather_float ? nv * sizeof(float) : 0);
       q.off_img_t = take(q.gather_float ? nv * sizeof(float) : 0);
@@ -434,6 +524,9 @@ fir_status fir_batch_create(fir_batch** out, fir_ctx* ctx, int n_problems, const
     try
     {
       cuda_ok(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking), "cudaStreamCreate");
+      cuda_ok(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking), "cudaStreamCreate");
+      cuda_ok(cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming), "cudaEventCreate");
+      cuda_ok(cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming), "cudaEventCreate");
       cuda_ok(cudaEventCreateWithFlags(&b->ev_in, cudaEventDisableTiming), "cudaEventCreate");
       cuda_ok(cudaEventCreateWithFlags(&b->ev_out, cudaEventDisableTiming), "cudaEventCreate");
       auto* base = static_cast<unsigned char*>(b->arena.ensure(std::max<size_t>(off, 256)));
@@ -443,11 +536,15 @@ fir_status fir_batch_create(fir_batch** out, fir_ctx* ctx, int n_problems, const
         fir_batch::Problem& q = b->pr[(size_t)k];
         BatchProblem& d = b->desc_host[(size_t)k];
         std::memset(&d, 0, sizeof(d));
-        fir_ctx geo;
-        geo.geometry = c.geometry;
         d.g = grid_of(geo, q.v);
         d.s = sino_of(q.p, q.n_subsets, 0);
         q.n_enum = d.s.n_enum;
+        d.columns = q.columns ? 1 : 0;
+        d.plan = plans[(size_t)k];
+        if (q.columns)
+        {
+          b->track_bytes = std::max(b->track_bytes, column_smem(d.plan));
+        }
         q.direct = q.gather_float || (long long)q.n_enum >= kDirectLors;
         batch_copy(*b, base + q.off_xy, scan[(size_t)k].xy.data(), scan[(size_t)k].xy.size() * sizeof(double));
         batch_copy(*b, base + q.off_z, scan[(size_t)k].z.data(), scan[(size_t)k].z.size() * sizeof(double));
@@ -654,7 +751,7 @@ fir_status fir_batch_tune(fir_batch* batch, double* best_ms)
     // the first step whose projector batches problems (direct launches do
     // not use the shape)
     size_t t0 = 0;
-    while (t0 < b.steps.size() && b.steps[t0].proj.n_items == 0)
+    while (t0 < b.steps.size() && b.steps[t0].proj.n_items == 0 && b.steps[t0].tracks.n_items == 0)
     {
       ++t0;
     }
@@ -720,6 +817,7 @@ fir_status fir_batch_tune(fir_batch* batch, double* best_ms)
           cuda_ok(cudaMemsetAsync(queue, 0, sizeof(int), b.stream), "cudaMemsetAsync");
           cuda_ok(cudaEventRecord(e0, b.stream), "cudaEventRecord");
           batch_project(b, b.steps[t0].proj, queue, L, b.stream);
+          batch_project_tracks(b, b.steps[t0].tracks, b.stream);
           cuda_ok(cudaEventRecord(e1, b.stream), "cudaEventRecord");
           cuda_ok(cudaEventSynchronize(e1), "cudaEventSynchronize");
           float ms = 0.0f;

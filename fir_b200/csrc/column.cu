@@ -25,7 +25,8 @@ struct ColumnLor
   double z1, z2;
 };
 
-__device__ __forceinline__ int first_track(const ColumnPlan& p) { return blockIdx.x / p.blocks * p.per_block; }
+// The first track of the launch's block number `block`.
+__device__ __forceinline__ int first_track(const ColumnPlan& p, int block) { return block / p.blocks * p.per_block; }
 
 // The part of the launch that a warp's group (the block's warps that serve
 // its track) traces: ring pairs [begin, end) of one track.
@@ -36,7 +37,7 @@ struct ColumnShare
   int begin, end;
 };
 
-__device__ __forceinline__ ColumnShare column_share(const Sino& s, const ColumnPlan& p, int first)
+__device__ __forceinline__ ColumnShare column_share(const Sino& s, const ColumnPlan& p, int block, int first)
 {
   const int warp = threadIdx.x >> 5;
   ColumnShare c;
@@ -47,7 +48,7 @@ __device__ __forceinline__ ColumnShare column_share(const Sino& s, const ColumnP
   const int vt = first + c.group;
   c.sv = vt / s.n_tang;
   c.tang = vt - c.sv * s.n_tang;
-  c.begin = (int)(blockIdx.x % p.blocks) * p.share;
+  c.begin = block % p.blocks * p.share;
   c.end = any ? min(c.begin + p.share, p.pairs) : c.begin;
   return c;
 }
@@ -356,10 +357,10 @@ __global__ void __launch_bounds__(256, 5) k_column_forward(const __grid_constant
                                                            int* check)
 {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int first = first_track(p);
+  const int first = first_track(p, (int)blockIdx.x);
   const Leftover left = leftover(smem, p);
   build_tracks(g, s, t, p, s.subset, first, smem, left.count);
-  const ColumnShare c = column_share(s, p, first);
+  const ColumnShare c = column_share(s, p, (int)blockIdx.x, first);
   const Track tr = track_at(smem, p.cap, c.group);
   column_each<false>(s, t, p, c, s.subset, nullptr, NonzeroLists{}, [&](const ColumnLor* lor) {
     ColumnLane w[2] = {};
@@ -396,10 +397,10 @@ __global__ void __launch_bounds__(256, 4) k_column_backward(const __grid_constan
                                                             const float* __restrict__ sino, float* acc, int* check)
 {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int first = first_track(p);
+  const int first = first_track(p, (int)blockIdx.x);
   const Leftover left = leftover(smem, p);
   build_tracks(g, s, t, p, s.subset, first, smem, left.count);
-  const ColumnShare c = column_share(s, p, first);
+  const ColumnShare c = column_share(s, p, (int)blockIdx.x, first);
   const Track tr = track_at(smem, p.cap, c.group);
   column_each<kSkip>(s, t, p, c, s.subset, sino, nonzero_lists(smem, p), [&](const ColumnLor* lor) {
     ColumnLane w[2] = {};
@@ -444,23 +445,22 @@ __device__ __forceinline__ bool osem_ratio(float line, int bin, const float* __r
   return true;
 }
 
-// One OSEM sub-iteration (reconAlgos.cc:119-158, see osem_lor_body): image
-// and accumulators in z columns.
+// The LORs of block number `block` of one OSEM sub-iteration
+// (reconAlgos.cc:119-158, see osem_lor_body): image and accumulators in z
+// columns.
 template<bool kWeighted, bool kSkip>
-__global__ void __launch_bounds__(256, 5) k_column_osem(const __grid_constant__ Grid g,
-                                                        const __grid_constant__ Sino s, Tables t, ColumnPlan p,
-                                                        const double* __restrict__ img,
-                                                        const float* __restrict__ sino,
-                                                        const float* __restrict__ mult,
-                                                        const float* __restrict__ bias, float* acc, int* check)
+__device__ __forceinline__ void column_osem(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p,
+                                            int subset, int block, const double* __restrict__ img,
+                                            const float* __restrict__ sino, const float* __restrict__ mult,
+                                            const float* __restrict__ bias, float* acc, int* check,
+                                            unsigned char* smem)
 {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const int first = first_track(p);
+  const int first = first_track(p, block);
   const Leftover left = leftover(smem, p);
-  build_tracks(g, s, t, p, s.subset, first, smem, left.count);
-  const ColumnShare c = column_share(s, p, first);
+  build_tracks(g, s, t, p, subset, first, smem, left.count);
+  const ColumnShare c = column_share(s, p, block, first);
   const Track tr = track_at(smem, p.cap, c.group);
-  column_each<kSkip>(s, t, p, c, s.subset, sino, nonzero_lists(smem, p), [&](const ColumnLor* lor) {
+  column_each<kSkip>(s, t, p, c, subset, sino, nonzero_lists(smem, p), [&](const ColumnLor* lor) {
     ColumnLane w[2] = {};
     bool go[2];
     float line[2];
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(256, 5) k_column_osem(const __grid_constant__ 
     }
     column_scatter(tr, go, w, value, accumulator_of(g, *tr.head, acc));
   });
-  column_leftover(s, t, p, s.subset, first, smem, left, [&](const ColumnLor& lor, const Track& own) {
+  column_leftover(s, t, p, subset, first, smem, left, [&](const ColumnLor& lor, const Track& own) {
     const GeneralLine gl = general_line(g, *own.head, lor.z1, lor.z2, img, check);
     double q;
     if (osem_ratio<kWeighted>(gl.line, lor.bin, sino, mult, bias, q) && gl.ok)
@@ -482,6 +482,40 @@ __global__ void __launch_bounds__(256, 5) k_column_osem(const __grid_constant__ 
       general_scatter(g, *own.head, lor.z1, lor.z2, q, accumulator_of(g, *own.head, acc), check);
     }
   });
+}
+
+template<bool kWeighted, bool kSkip>
+__global__ void __launch_bounds__(256, 5) k_column_osem(const __grid_constant__ Grid g,
+                                                        const __grid_constant__ Sino s, Tables t, ColumnPlan p,
+                                                        const double* __restrict__ img,
+                                                        const float* __restrict__ sino,
+                                                        const float* __restrict__ mult,
+                                                        const float* __restrict__ bias, float* acc, int* check)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  column_osem<kWeighted, kSkip>(g, s, t, p, s.subset, (int)blockIdx.x, img, sino, mult, bias, acc, check, smem);
+}
+
+// The same for the items of a batch (batch.cu), whose work units are the
+// blocks of their problems' plans.
+template<bool kSkip>
+__global__ void __launch_bounds__(kBatchColumnBlock, 10)
+  k_batch_column_osem(const BatchProblem* __restrict__ P, const BatchItem* __restrict__ items, int n_items, int* check)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  int lo = 0, hi = n_items;
+  while (hi - lo > 1)
+  {
+    const int mid = (lo + hi) >> 1;
+    if (__ldg(&items[mid].unit_begin) <= (int)blockIdx.x)
+      lo = mid;
+    else
+      hi = mid;
+  }
+  const BatchProblem& pb = P[__ldg(&items[lo].problem)];
+  column_osem<false, kSkip>(pb.g, pb.s, pb.t, pb.plan, __ldg(&items[lo].subset),
+                            (int)blockIdx.x - __ldg(&items[lo].unit_begin), pb.wide, pb.sino, nullptr, pb.bias, pb.bp,
+                            check, smem);
 }
 
 // Images between [z][y][x] and z columns, through 32 x 32 tiles of
@@ -581,11 +615,6 @@ __global__ void __launch_bounds__(kTile * kTileRows) k_em_update_columns(int np,
   }
 }
 
-unsigned column_grid(const ColumnPlan& p)
-{
-  return (unsigned)((p.tracks + p.per_block - 1) / p.per_block * p.blocks);
-}
-
 // Shared memory above 48 KB is asked for once per kernel and call.
 template<typename K>
 void ask_shared(K kernel, size_t bytes)
@@ -604,7 +633,9 @@ size_t column_smem(const ColumnPlan& p)
          (p.skip ? lists : 0);
 }
 
-ColumnPlan column_plan(const Grid& g, const Sino& s, const double* z, int block, bool skip)
+int column_blocks(const ColumnPlan& p) { return (p.tracks + p.per_block - 1) / p.per_block * p.blocks; }
+
+ColumnPlan column_plan(const Grid& g, const Sino& s, const double* z, int block, bool skip, bool fixed)
 {
   ColumnPlan p{};
   for (int k = 0; k < s.n_segments; ++k)
@@ -628,7 +659,7 @@ ColumnPlan column_plan(const Grid& g, const Sino& s, const double* z, int block,
   int best = want, idle = 1 << 30;
   for (int w : {want, want + 1, want - 1, want + 2})
   {
-    if (w >= 1 && w <= 8)
+    if (w >= 1 && w <= 8 && (w == want || !fixed))
     {
       const int off = warps >= w ? (warps + w - 1) / w * w - warps : (w % warps);
       // (compared as a share of all warps)
@@ -697,8 +728,11 @@ static double stops_per_turn(const Grid& g, const Sino& s, const ColumnPlan& p, 
   return sum / ((p.pairs + 63) / 64);
 }
 
-// Tracks need ring pairs to share them: below 48 most of a warp's 64 slots
-// are idle.  They also need about six warps per scheduler to hide the loops'
+// Warps of the launch that have work.
+long long column_warps(const ColumnPlan& p) { return (long long)p.tracks * ((p.pairs + 63) / 64); }
+
+// Tracks need ring pairs to share them: below 30 most of a warp's 64 slots
+// are idle.  They also need about six warps per scheduler (kColumnWarps) to hide the loops'
 // latency (a turn waits for its entry and test): the LOR-by-LOR kernels, with
 // twice the warps, are faster below that (measured 0.63x to 0.98x below 3000
 // warps, 1.3x and more above 8000).  A LOR clipped by the volume's ends walks
@@ -707,8 +741,7 @@ static double stops_per_turn(const Grid& g, const Sino& s, const ColumnPlan& p, 
 // volumes, 0.96x at 2.3 on a 320x320x128 one).
 bool columns_pay(const Grid& g, const Sino& s, const ColumnPlan& p, const double* z, double diameter)
 {
-  if (g.exact_only || p.pairs < 48 || (long long)p.tracks * ((p.pairs + 63) / 64) < 6 * 592 ||
-      column_smem(p) > 96 * 1024 || (long long)g.nxy * g.nz >= 1LL << 29)
+  if (g.exact_only || p.pairs < 30 || column_smem(p) > 96 * 1024 || (long long)g.nxy * g.nz >= 1LL << 29)
   {
     return false;
   }
@@ -741,7 +774,7 @@ void launch_column_forward(const Grid& g, const Sino& s, const Tables& t, const 
   const size_t bytes = column_smem(p);
   auto* kernel = ep == FwdEpilogue::Exp ? k_column_forward<FwdEpilogue::Exp> : k_column_forward<FwdEpilogue::None>;
   ask_shared(kernel, bytes);
-  kernel<<<column_grid(p), p.block, bytes, cfg.stream>>>(g, s, t, p, img, sino, cfg.check);
+  kernel<<<(unsigned)column_blocks(p), p.block, bytes, cfg.stream>>>(g, s, t, p, img, sino, cfg.check);
 }
 
 void launch_column_backward(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p, const float* sino,
@@ -754,7 +787,19 @@ void launch_column_backward(const Grid& g, const Sino& s, const Tables& t, const
   const size_t bytes = column_smem(p);
   auto* kernel = p.skip ? k_column_backward<true> : k_column_backward<false>;
   ask_shared(kernel, bytes);
-  kernel<<<column_grid(p), p.block, bytes, cfg.stream>>>(g, s, t, p, sino, acc, cfg.check);
+  kernel<<<(unsigned)column_blocks(p), p.block, bytes, cfg.stream>>>(g, s, t, p, sino, acc, cfg.check);
+}
+
+void launch_batch_column_osem(const BatchProblem* P, const BatchItem* items, int n_items, int n_blocks, size_t bytes,
+                              bool skip, int* check, cudaStream_t stream)
+{
+  if (n_blocks <= 0)
+  {
+    return;
+  }
+  auto* kernel = skip ? k_batch_column_osem<true> : k_batch_column_osem<false>;
+  ask_shared(kernel, bytes);
+  kernel<<<(unsigned)n_blocks, kBatchColumnBlock, bytes, stream>>>(P, items, n_items, check);
 }
 
 void launch_column_osem(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p, const double* img,
@@ -769,6 +814,6 @@ void launch_column_osem(const Grid& g, const Sino& s, const Tables& t, const Col
   auto* kernel = mult != nullptr ? (skip ? k_column_osem<true, true> : k_column_osem<true, false>)
                                  : (skip ? k_column_osem<false, true> : k_column_osem<false, false>);
   ask_shared(kernel, bytes);
-  kernel<<<column_grid(p), p.block, bytes, cfg.stream>>>(g, s, t, p, img, sino, mult, bias, acc, cfg.check);
+  kernel<<<(unsigned)column_blocks(p), p.block, bytes, cfg.stream>>>(g, s, t, p, img, sino, mult, bias, acc, cfg.check);
 }
 }  // namespace fir

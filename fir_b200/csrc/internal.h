@@ -72,10 +72,16 @@ void launch_osem_subset_float_image(const Grid& g, const Sino& s, const Tables& 
 // image as doubles in z columns ([y][x][z]) and add into two accumulators of
 // that layout, one after the other at acc, whose sum is the backprojection.
 // How a launch with blocks of about `block` threads deals the LORs of s (z: the
-// scanner's slice centres; skip: the projectors skip bins that are 0).
-ColumnPlan column_plan(const Grid& g, const Sino& s, const double* z, int block, bool skip);
-// Whether the launch is faster on tracks than LOR by LOR (z: the scanner's
-// slice centres, diameter: of a ring).
+// scanner's slice centres; skip: the projectors skip bins that are 0;
+// fixed: with blocks of exactly that size).
+ColumnPlan column_plan(const Grid& g, const Sino& s, const double* z, int block, bool skip, bool fixed = false);
+int column_blocks(const ColumnPlan& p);
+// Warps of the launch that have work; below kColumnWarps a launch alone is
+// faster LOR by LOR.
+long long column_warps(const ColumnPlan& p);
+constexpr long long kColumnWarps = 6 * 592;
+// Whether a launch with enough warps is faster on tracks than LOR by LOR (z:
+// the scanner's slice centres, diameter: of a ring).
 bool columns_pay(const Grid& g, const Sino& s, const ColumnPlan& p, const double* z, double diameter);
 // out = the image's double copy in z columns; the accumulators (or null) = 0.
 void launch_to_columns(const Grid& g, const float* in, double* out, float* acc, const LaunchCfg& cfg);
@@ -193,9 +199,13 @@ struct BatchProblem
   // wide, img and bp with x and y exchanged ([z][x][y]), for LORs running
   // mostly along x; bp_t is added into bp by the EM step.  Problems with the
   // double copy have wide_t, those that gather floats img_t (null: none).
+  // With columns (column.cu) wide is in z columns, bp the two accumulators
+  // there, and these are null.
   double* wide_t;
   float* bp_t;
   float* img_t;
+  int columns;
+  ColumnPlan plan;
   float* t1;
   float* t2;
   int nvox;
@@ -221,6 +231,7 @@ struct BatchItem
 };
 
 constexpr int kBatchBlock = 256;
+constexpr int kBatchColumnBlock = 128;
 
 struct BatchLaunch
 {
@@ -236,6 +247,8 @@ struct BatchLaunch
 // Bundles of one subset of a problem with the given axial tile (0: linear).
 long long batch_bundles(const Sino& s, int axial_tile);
 void batch_bundle_bases(const Sino& s, int axial_tile, int* base);
+// Units of the image kernels.
+long long batch_voxel_units(const BatchProblem& p);
 
 // wide = cut(img), bp = 0 (and img = cut(img) when write_img).
 void launch_batch_prepare(const BatchProblem* P, const BatchItem* items, int n_items, int n_units,
@@ -245,6 +258,10 @@ void launch_batch_prepare(const BatchProblem* P, const BatchItem* items, int n_i
 // their double copies (wide).
 void launch_batch_project(const BatchProblem* P, const BatchItem* items, int n_items, int n_bundles,
                           int* queue, const BatchLaunch& L, int n_sms, int* check, cudaStream_t stream);
+// The same for items whose problems have columns: n_blocks blocks of their
+// plans, whose largest shared memory is `bytes` (column.cu).
+void launch_batch_column_osem(const BatchProblem* P, const BatchItem* items, int n_items, int n_blocks, size_t bytes,
+                              bool skip, int* check, cudaStream_t stream);
 // Gated EM update of img; bp <- 0.  Items without filtering also apply the
 // cut and refresh wide.
 void launch_batch_em(const BatchProblem* P, const BatchItem* items, int n_items, int n_units,

@@ -116,3 +116,40 @@ def test_weighted_osem_and_noncontiguous_subset():
         c.osem(proj, y, vol, img, sens, prm, bias=bias, mult=m)
         out.append(img.astype(np.float64))
     assert np.linalg.norm(out[0] - out[1]) <= 1e-5 * np.linalg.norm(out[1])
+
+
+@pytest.mark.parametrize("skip", [0, 1])
+def test_batch_on_tracks(skip):
+    """Problems on tracks beside one LOR by LOR (4 rings), against fir_osem."""
+    names = ["coincident_planes", "span_3", "interleaved"]
+    parts = [problem(n) for n in names]
+    parts.append((ScannerSpec.ring(4, 64, 120.0, 4.0), ProjSpec(4, 64, 7, 21), VolSpec.centred((32, 32, 8), (4.0, 4.0, 4.0))))
+    rng = np.random.default_rng(8)
+    prms = [OSEMParams(n_iterations=2, n_subsets=s, convolution_interval=f, fwhm_xyz=[5.0, 5.0, 5.0], cut_radius=cut)
+            for s, f, cut in ((2, 1, 0.0), (1, 0, 70.0), (3, 2, 60.0), (4, 1, 0.0))]
+    ctx = capi.Context(parts[0][0])
+    ctx.set_option(capi.FIR_OPT_SKIP_ZERO_BINS, skip)
+    batch = capi.Batch(ctx, [(s, p, v, q) for (s, p, v), q in zip(parts, prms)])
+    data = []
+    for k, ((s, p, v), q) in enumerate(zip(parts, prms)):
+        nb = capi.proj_geometry(p)["n_bins"]
+        y = rng.poisson(1.5, nb).astype(np.float32)
+        sens = np.zeros((q.n_subsets,) + v.shape_zyx, np.float32)
+        c = capi.Context(s)
+        c.sensitivity(p, v, sens, q.n_subsets)
+        bias = rng.random(nb, dtype=np.float32) + np.float32(0.1) if k != 1 else None
+        batch.set_data(k, y, sens, bias)
+        img = np.ones(v.shape_zyx, np.float32)
+        c.osem(p, y, v, img, sens, q, bias=bias)
+        data.append(img.astype(np.float64))
+        c.close()
+    for use_graph in (True, False, True):
+        for k, (_, _, v) in enumerate(parts):
+            batch.set_image(k, np.ones(v.shape_zyx, np.float32))
+        batch.osem(use_graph=use_graph)
+        for k, want in enumerate(data):
+            got = batch.get_image(k).astype(np.float64)
+            assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want), k
+    assert batch.tune() > 0
+    batch.close()
+    ctx.close()
