@@ -473,11 +473,12 @@ void det_backproject(fir_ctx& c, const Grid& g, const Sino& s, const Tables& t, 
   c.launches += launches;
 }
 
-// Double copy of a float image in context scratch, for the projector gathers.
-const double* widen(fir_ctx& c, const float* img, long long n)
+// Double copy of a float image in context scratch, for the projector gathers
+// (zero, or null, is cleared on the way).
+const double* widen(fir_ctx& c, const float* img, long long n, float* zero = nullptr)
 {
   double* d = static_cast<double*>(c.wide.ensure((size_t)n * sizeof(double)));
-  launch_widen(n, img, d, cfg_of(c));
+  launch_widen(n, img, d, zero, cfg_of(c));
   after_launch(c);
   return d;
 }
@@ -499,7 +500,7 @@ Widened widen_for_projection(fir_ctx& c, const Grid& g, const float* img)
   }
   double* d = static_cast<double*>(c.wide.ensure((size_t)n * sizeof(double)));
   double* d_t = static_cast<double*>(c.wide_t.ensure((size_t)n * sizeof(double)));
-  launch_widen_oriented(g.nx, g.ny, g.nz, img, d, d_t, cfg_of(c));
+  launch_widen_oriented(g.nx, g.ny, g.nz, img, d, d_t, nullptr, nullptr, cfg_of(c));
   after_launch(c);
   return Widened{d, d_t};
 }
@@ -620,8 +621,8 @@ const float* column_ratio_backproject(fir_ctx& c, const Grid& g, const Sino& s, 
   return acc;
 }
 
-// bp (zeroed by the caller) += backprojection of sino / (projection of img +
-// bias) over the subset of s: the fused kernel, or in deterministic mode the
+// bp (zeroed by the caller, or with defer_merge here) += backprojection of
+// sino / (projection of img + bias) over the subset of s: the fused kernel, or in deterministic mode the
 // ratio kernel followed by the ordered scatter.  The fused kernel reads and
 // accumulates LORs that run mostly along x in images with x and y exchanged
 // (double copy and accumulator in context scratch); the accumulator is added
@@ -638,6 +639,11 @@ const float* ratio_backproject(fir_ctx& c, const Grid& g, const Sino& s_all, con
     launch_from_columns(g, acc, bp, cfg_of(c));
     after_launch(c);
     return nullptr;
+  }
+  const bool exchanged = c.backproj == FIR_BACKPROJ_ATOMIC && c.traversal == FIR_TRAVERSAL_EXACT && use_exchanged(c, g);
+  if (defer_merge && !exchanged)
+  {
+    cuda_ok(cudaMemsetAsync(bp, 0, (size_t)nvox * sizeof(float), c.stream), "cudaMemsetAsync");
   }
   // skipped bins: listed out of the atomic kernels' enumeration
   const bool listed = c.skip_zero != 0 && c.backproj == FIR_BACKPROJ_ATOMIC && s_all.n_enum > 0;
@@ -718,8 +724,7 @@ const float* ratio_backproject(fir_ctx& c, const Grid& g, const Sino& s_all, con
   double* wimg = static_cast<double*>(c.wide.ensure(n * sizeof(double)));
   double* wimg_t = static_cast<double*>(c.wide_t.ensure(n * sizeof(double)));
   float* bp_t = static_cast<float*>(c.bp_t.ensure(n * sizeof(float)));
-  cuda_ok(cudaMemsetAsync(bp_t, 0, n * sizeof(float), c.stream), "cudaMemsetAsync");
-  launch_widen_oriented(g.nx, g.ny, g.nz, img, wimg, wimg_t, cfg_of(c));
+  launch_widen_oriented(g.nx, g.ny, g.nz, img, wimg, wimg_t, defer_merge ? bp : nullptr, bp_t, cfg_of(c));
   after_launch(c);
   timed_launch(c, [&] {
     launch_osem_subset(g, s, t, wimg, wimg_t, sino, mult, bias, bp, bp_t, c.skip_zero != 0, cfg_of(c));
@@ -1036,38 +1041,51 @@ Taps gauss_taps(float fwhm, double vox, bool double_sigma)
   return t;
 }
 
-// operations::convolve on device memory, all frames of vol.
-void convolve_device(fir_ctx& c, const VolInfo& v, float* img, const float fwhm[3], float cut)
+// The Gaussian of operations::convolve and its taps; wanted is false where FIR
+// does not filter.
+struct Filter
 {
+  Taps x, y, z;
+  float fwhm = 0.0f;  // of the edge's restore
+  bool wanted = false;
+};
+
+Filter filter_of(const VolInfo& v, const float fwhm[3])
+{
+  Filter f;
   if (!(fwhm[0] > 0.0 && fwhm[1] > 0.0 && fwhm[2] > 0.0))
   {
-    return;
+    return f;
   }
-  const Taps tx = gauss_taps(fwhm[0], v.d.voxel_x, false);
-  const Taps ty = gauss_taps(fwhm[1], v.d.voxel_y, false);
-  const Taps tz = gauss_taps(fwhm[2], v.d.voxel_z, true);
+  f.wanted = true;
+  f.x = gauss_taps(fwhm[0], v.d.voxel_x, false);
+  f.y = gauss_taps(fwhm[1], v.d.voxel_y, false);
+  f.z = gauss_taps(fwhm[2], v.d.voxel_z, true);
+  f.fwhm = fwhm[0] > fwhm[1] ? fwhm[0] : fwhm[1];
+  return f;
+}
+
+// One frame filtered in place in three passes; where r >= restore - 5 fwhm it
+// is kept (restore <= 0: nowhere), then 0 where r > cut (<= 0: nowhere).
+void filter_passes(fir_ctx& c, const VolInfo& v, const Filter& f, float restore, float cut, float* img)
+{
   const size_t bytes = (size_t)v.nvox * sizeof(float);
   float* t1 = static_cast<float*>(c.conv1.ensure(bytes));
   float* t2 = static_cast<float*>(c.conv2.ensure(bytes));
-  float* cp = cut > 0.0f ? static_cast<float*>(c.conv_copy.ensure(bytes)) : nullptr;
   const LaunchCfg cfg = cfg_of(c);
-  const float f = fwhm[0] > fwhm[1] ? fwhm[0] : fwhm[1];
-  for (int fr = 0; fr < v.d.n_frames; ++fr)
+  launch_conv_pass(v.d.nx, v.d.ny, v.d.nz, 0, f.x, img, t1, cfg);
+  launch_conv_pass(v.d.nx, v.d.ny, v.d.nz, 1, f.y, t1, t2, cfg);
+  launch_conv_last(v.d.nx, v.d.ny, v.d.nz, f.z, v.d.voxel_x, v.d.voxel_y, restore, f.fwhm, cut, t2, img, cfg);
+  after_launch(c, 3);
+}
+
+// operations::convolve on device memory, all frames of vol.
+void convolve_device(fir_ctx& c, const VolInfo& v, float* img, const float fwhm[3], float cut)
+{
+  const Filter f = filter_of(v, fwhm);
+  for (int fr = 0; f.wanted && fr < v.d.n_frames; ++fr)
   {
-    float* x = img + (size_t)fr * v.nvox;
-    if (cp != nullptr)
-    {
-      cuda_ok(cudaMemcpyAsync(cp, x, bytes, cudaMemcpyDeviceToDevice, c.stream), "cudaMemcpyAsync");
-    }
-    launch_conv_pass(v.d.nx, v.d.ny, v.d.nz, 0, tx, x, t1, cfg);
-    launch_conv_pass(v.d.nx, v.d.ny, v.d.nz, 1, ty, t1, t2, cfg);
-    launch_conv_pass(v.d.nx, v.d.ny, v.d.nz, 2, tz, t2, x, cfg);
-    after_launch(c, 3);
-    if (cp != nullptr)
-    {
-      launch_conv_restore(v.d.nx, v.d.ny, v.d.nz, v.d.voxel_x, v.d.voxel_y, cut, f, cp, x, cfg);
-      after_launch(c);
-    }
+    filter_passes(c, v, f, cut > 0.0f ? cut : 0.0f, 0.0f, img + (size_t)fr * v.nvox);
   }
 }
 
@@ -1105,34 +1123,48 @@ void osem_subiteration_device(fir_ctx& c, const ProjInfo& p, const Tables& t, co
                               int subiter)
 {
   const Sino s = sino_of(p, prm->n_subsets, subset);
+  Filter f;
+  if (prm->convolution_interval > 0 && subiter % prm->convolution_interval == 0)
+  {
+    f = filter_of(v, prm->fwhm_xyz);
+  }
+  // a small volume is filtered in one launch, from the EM step's scratch image
+  const bool fused = f.wanted && conv_fused_fits(g.nx, g.ny, g.nz, f.x, f.y, f.z);
+  float* out = fused ? static_cast<float*>(c.conv1.ensure((size_t)v.nvox * sizeof(float))) : img;
   ColumnPlan plan;
   if (osem_columns(c, g, s, plan))
   {
     const float* acc = column_ratio_backproject(c, g, s, t, plan, img, sino, mult, bias);
-    launch_em_update_columns(g, img, acc, sens_frame, cfg_of(c));
+    launch_em_update_columns(g, img, out, acc, sens_frame, cfg_of(c));
   }
   else
   {
     float* bp = static_cast<float*>(c.bp.ensure((size_t)v.nvox * sizeof(float)));
-    cuda_ok(cudaMemsetAsync(bp, 0, (size_t)v.nvox * sizeof(float), c.stream), "cudaMemsetAsync");
     const float* bp_t = ratio_backproject(c, g, s, t, img, sino, mult, bias, bp, v.nvox, true);
     if (bp_t != nullptr)
     {
-      launch_em_update_oriented(g.nx, g.ny, g.nz, img, bp, bp_t, sens_frame, cfg_of(c));
+      launch_em_update_oriented(g.nx, g.ny, g.nz, img, out, bp, bp_t, sens_frame, cfg_of(c));
     }
     else
     {
-      launch_em_update(v.nvox, img, bp, sens_frame, cfg_of(c));
+      launch_em_update(v.nvox, img, out, bp, sens_frame, cfg_of(c));
     }
   }
   after_launch(c);
-  const bool conv = prm->convolution_interval > 0 && prm->fwhm_xyz[0] > 0.0 && prm->fwhm_xyz[1] > 0.0 &&
-                    prm->fwhm_xyz[2] > 0.0;
-  if (conv && subiter % prm->convolution_interval == 0)
+  const float cut = prm->cut_radius > 0.0f ? prm->cut_radius : 0.0f;
+  if (fused)
   {
-    convolve_device(c, v, img, prm->fwhm_xyz, prm->cut_radius);
+    launch_conv_fused(g.nx, g.ny, g.nz, f.x, f.y, f.z, v.d.voxel_x, v.d.voxel_y, cut, f.fwhm, cut, out, img, cfg_of(c));
+    after_launch(c);
   }
-  cut_device(c, v, img, prm->cut_radius, 1);
+  else if (f.wanted)
+  {
+    filter_passes(c, v, f, cut, cut, img);
+  }
+  else
+  {
+    cut_device(c, v, img, prm->cut_radius, 1);
+  }
 }
 
 // One sub-iteration of the resolution-modelling OSEM: the Gaussian B of the
@@ -1151,7 +1183,7 @@ void osem_psf_subiteration_device(fir_ctx& c, const ProjInfo& p, const Tables& t
   const Sino s = sino_of(p, prm->n_subsets, subset);
   ratio_backproject(c, g, s, t, blur, sino, mult, bias, bp, v.nvox);
   convolve_device(c, v, bp, prm->fwhm_xyz, prm->cut_radius);
-  launch_em_update(v.nvox, img, bp, sens_frame, cfg_of(c));
+  launch_em_update(v.nvox, img, img, bp, sens_frame, cfg_of(c));
   after_launch(c);
   const bool conv = prm->convolution_interval > 0 && prm->fwhm_xyz[0] > 0.0 && prm->fwhm_xyz[1] > 0.0 &&
                     prm->fwhm_xyz[2] > 0.0;
@@ -1514,7 +1546,7 @@ fir_status fir_ctx_destroy(fir_ctx* c)
     }
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
-    for (DevBuf* b : {&c->xy, &c->z, &c->check, &c->bp, &c->conv1, &c->conv2, &c->conv_copy, &c->mu, &c->wide,
+    for (DevBuf* b : {&c->xy, &c->z, &c->check, &c->bp, &c->conv1, &c->conv2, &c->mu, &c->wide,
                       &c->det, &c->det_pairs, &c->ratio, &c->frames_il, &c->frames_acc, &c->psf_blur, &c->psf_sens, &c->rebin,
                       &c->wide_t, &c->bp_t, &c->img_t, &c->frames_il_t, &c->frames_acc_t, &c->compact})
     {
@@ -2034,7 +2066,7 @@ fir_status fir_em_update(fir_ctx* ctx, const fir_vol_desc* vol, float* img, floa
     float* dimg = st.inout(img, v.nvox);
     float* dbp = st.inout(bp, v.nvox);
     const float* dsens = st.in(sens_frame, v.nvox);
-    launch_em_update(v.nvox, dimg, dbp, dsens, cfg_of(c));
+    launch_em_update(v.nvox, dimg, dimg, dbp, dsens, cfg_of(c));
     after_launch(c);
     finish(c, st);
   });
@@ -2443,9 +2475,9 @@ extern "C" fir_status fir_osem_subiteration_noalloc(const fir_proj_desc* proj, c
 
     // the accumulator keeps the previous call's sums: clear it
     cuda_ok(cudaMemsetAsync(bp, 0, (size_t)v.nvox * sizeof(float), st), "cudaMemsetAsync");
-    launch_widen(v.nvox, img, wide, cfg);
+    launch_widen(v.nvox, img, wide, nullptr, cfg);
     launch_osem_subset(g, s, t, wide, nullptr, sino, nullptr, bias, bp, nullptr, false, cfg);
-    launch_em_update(v.nvox, img, bp, sens_frame, cfg);
+    launch_em_update(v.nvox, img, img, bp, sens_frame, cfg);
     const float* fwhm = params->fwhm_xyz;
     const bool conv = params->convolution_interval > 0 && fwhm[0] > 0.0 && fwhm[1] > 0.0 && fwhm[2] > 0.0;
     if (conv && subiter % params->convolution_interval == 0)

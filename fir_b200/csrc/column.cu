@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(kTile * kTileRows) k_from_columns(int np, int 
 }
 
 // k_em_update with the backprojection in z columns.
-__global__ void __launch_bounds__(kTile * kTileRows) k_em_update_columns(int np, int nz, float* __restrict__ img,
+__global__ void __launch_bounds__(kTile * kTileRows) k_em_update_columns(int np, int nz, const float* img, float* out,
                                                                          const float* __restrict__ acc,
                                                                          const float* __restrict__ sens)
 {
@@ -610,7 +610,7 @@ __global__ void __launch_bounds__(kTile * kTileRows) k_em_update_columns(int np,
       const float sv = __ldg(sens + k);
       const float q = ((double)b > kEps && (double)sv > kEps) ? __fdiv_rn(b, sv) : 0.0f;
       const float v = img[k];
-      img[k] = ((double)v > kEps && (double)q > kEps) ? __fmul_rn(v, q) : 0.0f;
+      out[k] = ((double)v > kEps && (double)q > kEps) ? __fmul_rn(v, q) : 0.0f;
     }
   }
 }
@@ -758,9 +758,10 @@ void launch_from_columns(const Grid& g, const float* acc, float* out, const Laun
   k_from_columns<<<column_tiles(g.nxy, g.nz), dim3(kTile, kTileRows), 0, cfg.stream>>>(g.nxy, g.nz, acc, out);
 }
 
-void launch_em_update_columns(const Grid& g, float* img, const float* acc, const float* sens, const LaunchCfg& cfg)
+void launch_em_update_columns(const Grid& g, const float* img, float* out, const float* acc, const float* sens,
+                              const LaunchCfg& cfg)
 {
-  k_em_update_columns<<<column_tiles(g.nxy, g.nz), dim3(kTile, kTileRows), 0, cfg.stream>>>(g.nxy, g.nz, img, acc,
+  k_em_update_columns<<<column_tiles(g.nxy, g.nz), dim3(kTile, kTileRows), 0, cfg.stream>>>(g.nxy, g.nz, img, out, acc,
                                                                                             sens);
 }
 

@@ -88,7 +88,8 @@ void launch_to_columns(const Grid& g, const float* in, double* out, float* acc, 
 // out = the accumulators' sum in [z][y][x].
 void launch_from_columns(const Grid& g, const float* acc, float* out, const LaunchCfg& cfg);
 // launch_em_update with the backprojection in z columns (left as it is).
-void launch_em_update_columns(const Grid& g, float* img, const float* acc, const float* sens, const LaunchCfg& cfg);
+void launch_em_update_columns(const Grid& g, const float* img, float* out, const float* acc, const float* sens,
+                              const LaunchCfg& cfg);
 void launch_column_forward(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p, const double* img,
                            float* sino, FwdEpilogue ep, const LaunchCfg& cfg);
 void launch_column_backward(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p, const float* sino,
@@ -137,24 +138,36 @@ struct Taps
   int half;
   float w[2 * kMaxHalfTaps + 1];
 };
-void launch_em_update(long long n, float* img, float* bp, const float* sens, const LaunchCfg& cfg);
+// out (may be img) = the gated EM update of img; bp holds the quotient then.
+void launch_em_update(long long n, const float* img, float* out, float* bp, const float* sens, const LaunchCfg& cfg);
 // The same after adding the x/y-exchanged accumulator bp_t into bp (one
 // launch in place of launch_merge_oriented and launch_em_update).
-void launch_em_update_oriented(int nx, int ny, int nz, float* img, float* bp, const float* bp_t, const float* sens,
-                               const LaunchCfg& cfg);
+void launch_em_update_oriented(int nx, int ny, int nz, const float* img, float* out, float* bp, const float* bp_t,
+                               const float* sens, const LaunchCfg& cfg);
 void launch_em_update_image_first(long long n, float* img, const float* bp, const float* sens,
                                   const LaunchCfg& cfg);
 // Exact widening of a float image to double for the projector gathers.
-void launch_widen(long long n, const float* in, double* out, const LaunchCfg& cfg);
+// zero (or null) is cleared on the way.
+void launch_widen(long long n, const float* in, double* out, float* zero, const LaunchCfg& cfg);
 // Double copies of an [nz][ny][nx] image: out in the same layout, out_t as
-// [nz][nx][ny].
-void launch_widen_oriented(int nx, int ny, int nz, const float* in, double* out, double* out_t,
-                           const LaunchCfg& cfg);
+// [nz][nx][ny]; zero and zero_t (each or null) are cleared on the way.
+void launch_widen_oriented(int nx, int ny, int nz, const float* in, double* out, double* out_t, float* zero,
+                           float* zero_t, const LaunchCfg& cfg);
 // bp[z][y][x] += bp_t[z][x][y].
 void launch_merge_oriented(int nx, int ny, int nz, float* bp, const float* bp_t, const LaunchCfg& cfg);
 // One separable pass of operations::convolve along axis (0=x, 1=y, 2=z).
 void launch_conv_pass(int nx, int ny, int nz, int axis, const Taps& taps, const float* in, float* out,
                       const LaunchCfg& cfg);
+// The z pass into img, which holds the pre-filter image: where r >= restore -
+// 5 fwhm that is kept (restore 0: nowhere), then 0 where r > cut (0: nowhere).
+void launch_conv_last(int nx, int ny, int nz, const Taps& taps, double vx, double vy, float restore, float fwhm,
+                      float cut, const float* in, float* img, const LaunchCfg& cfg);
+// The three passes and the same ending in one launch, in -> out, for volumes
+// where conv_fused_fits.
+constexpr long long kFusedFilterVoxels = 1LL << 20;
+bool conv_fused_fits(int nx, int ny, int nz, const Taps& tx, const Taps& ty, const Taps& tz);
+void launch_conv_fused(int nx, int ny, int nz, const Taps& tx, const Taps& ty, const Taps& tz, double vx, double vy,
+                       float restore, float fwhm, float cut, const float* in, float* out, const LaunchCfg& cfg);
 // Restore voxels with r >= cut - 5*fwhm from the pre-filter copy.
 void launch_conv_restore(int nx, int ny, int nz, double vx, double vy, float limit_base, float fwhm,
                          const float* copy, float* img, const LaunchCfg& cfg);
