@@ -23,6 +23,7 @@ from typing import Optional
 
 import torch
 
+from . import capi
 from .capi import Context, proj_geometry
 from .geometry import ProjSpec, ScannerSpec, VolSpec
 
@@ -119,10 +120,9 @@ _HALF26 = [(dz, dy, dx) for dz in (-1, 0, 1) for dy in (-1, 0, 1) for dx in (-1,
            if (dz, dy, dx) > (0, 0, 0)]
 
 
-def quadratic_penalty(x: torch.Tensor, beta: float) -> torch.Tensor:
-    """beta/2 * sum over 26-neighbour pairs (j, k) of (x_j - x_k)^2 / |j - k|,
-    |j - k| the centre distance in voxels (1, sqrt 2, sqrt 3); per frame,
-    summed over frames."""
+def _penalty_of_pairs(x: torch.Tensor, beta: float) -> torch.Tensor:
+    """The penalty as tensor operations over the 13 offsets: differentiable
+    any number of times, on any device and under any transform."""
     xs = x.reshape(-1, *x.shape[-3:])
     total = xs.new_zeros(())
     nz, ny, nx = xs.shape[-3:]
@@ -132,6 +132,49 @@ def quadratic_penalty(x: torch.Tensor, beta: float) -> torch.Tensor:
         w = 1.0 / math.sqrt(dz * dz + dy * dy + dx * dx)
         total = total + w * ((a - b) ** 2).sum()
     return 0.5 * beta * total
+
+
+class _Penalty(torch.autograd.Function):
+    """The penalty and its gradient by one kernel each."""
+
+    @staticmethod
+    def forward(ctx, x, beta):
+        ctx.save_for_backward(x)
+        ctx.beta = beta
+        return capi.quadratic_penalty(x.contiguous(), 0.5 * beta)[0].to(x.dtype)
+
+    @staticmethod
+    def backward(ctx, gy):
+        x, = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            # a gradient that is differentiated again
+            g, = torch.autograd.grad(_penalty_of_pairs(x, ctx.beta), x, create_graph=True)
+        else:
+            g = capi.quadratic_penalty(x.contiguous(), 0.5 * ctx.beta, value=False, grad=True)[1].view(x.shape)
+        return g * gy, None
+
+
+def _plain_cuda_image(x, beta) -> bool:
+    """Whether x is an ordinary CUDA image outside every transform (function
+    transforms, forward-mode duals, dispatch and torch-function modes, tracing)
+    and beta a number: only then a kernel may stand in for the operations."""
+    return (type(x) in (torch.Tensor, torch.nn.Parameter) and x.is_cuda and x.layout == torch.strided
+            and x.dtype in (torch.float32, torch.float64) and x.dim() >= 3 and 0 < x.numel() < 2 ** 31
+            and isinstance(beta, (int, float))
+            and torch._C._functorch.peek_interpreter_stack() is None
+            and not torch._C._functorch.is_functorch_wrapped_tensor(x)
+            and torch.autograd.forward_ad._current_level < 0
+            and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
+            and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
+
+
+def quadratic_penalty(x: torch.Tensor, beta: float) -> torch.Tensor:
+    """beta/2 * sum over 26-neighbour pairs (j, k) of (x_j - x_k)^2 / |j - k|,
+    |j - k| the centre distance in voxels (1, sqrt 2, sqrt 3); per frame,
+    summed over frames."""
+    if _plain_cuda_image(x, beta):
+        return _Penalty.apply(x, beta)
+    return _penalty_of_pairs(x, beta)
 
 
 def penalized_nll(x, y, op: SiddonProjector, beta: float, atten=None, bias=None):

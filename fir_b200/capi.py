@@ -149,6 +149,8 @@ _SIGS = {
                                      C.c_int]),
     "fir_backward_frames": (C.c_int, [C.c_void_p, C.POINTER(ProjDesc), C.c_void_p, C.POINTER(VolDesc), C.c_void_p,
                                       C.c_int]),
+    "fir_quadratic_penalty": (C.c_int, [C.POINTER(VolDesc), C.c_void_p, C.c_int, C.c_double, C.c_void_p, C.c_void_p,
+                                        C.c_void_p]),
     "fir_bin_coordinates": (C.c_int, [C.c_void_p, C.POINTER(ProjDesc), C.c_longlong, C.c_void_p, C.c_void_p,
                                       C.c_void_p]),
     "fir_proj_rebin_weight": (C.c_int, [C.c_void_p, C.POINTER(ProjDesc), C.c_void_p]),
@@ -295,6 +297,27 @@ def _dtype_of(x):
     except ImportError:
         pass
     return np.float64 if np.asarray(x).dtype == np.float64 else np.float32
+
+
+PENALTY_PARTIALS = 1024
+
+
+def quadratic_penalty(x, scale: float, value: bool = True, grad: bool = False):
+    """scale * the 26-neighbour quadratic penalty of the CUDA image x
+    ([F, nz, ny, nx], contiguous float32 or float64), on its device's current
+    stream: (value as a double tensor or None, gradient or None)."""
+    import torch
+
+    nz, ny, nx = x.shape[-3:]
+    d = VolDesc(nx, ny, nz, 1.0, 1.0, 1.0, 0.0, 0.0, 0.0, x.numel() // (nx * ny * nz))
+    dt = np.float64 if x.dtype == torch.float64 else np.float32
+    with torch.cuda.device(x.device):
+        part = torch.empty(PENALTY_PARTIALS, dtype=torch.float64, device=x.device) if value else None
+        g = torch.empty_like(x) if grad else None
+        _check(lib().fir_quadratic_penalty(C.byref(d), _ptr(x, dt), FIR_F64 if dt == np.float64 else FIR_F32,
+                                           float(scale), _ptr(part, np.float64), _ptr(g, dt),
+                                           C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    return (part.sum() if value else None), g
 
 
 class Context:

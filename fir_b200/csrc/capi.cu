@@ -2507,3 +2507,26 @@ extern "C" fir_status fir_osem_subiteration_noalloc(const fir_proj_desc* proj, c
     cuda_ok(cudaGetLastError(), "kernel launch");
   });
 }
+
+// The image's device, as the no-allocation entry point checks its pointers.
+extern "C" fir_status fir_quadratic_penalty(const fir_vol_desc* vol, const void* img, fir_dtype dtype, double scale,
+                                            double* partials, void* grad, void* stream)
+{
+  return guarded(__func__, [&] {
+    const VolInfo v = check_vol(vol);
+    const bool f64 = check_dtype(dtype);
+    if (img == nullptr)
+    {
+      fail(FIR_ERR_INVALID_ARGUMENT, "image must not be NULL");
+    }
+    int device = 0;
+    cuda_ok(cudaGetDevice(&device), "cudaGetDevice");
+    require_device(img, "img", device);
+    require_device(partials, "partials", device);
+    require_device(grad, "grad", device);
+    require_stream_on(static_cast<cudaStream_t>(stream), device);
+    launch_quadratic_penalty(v.d.nx, v.d.ny, v.d.nz, v.d.n_frames, img, f64, scale, partials, FIR_PENALTY_PARTIALS,
+                             grad, static_cast<cudaStream_t>(stream));
+    cuda_ok(cudaGetLastError(), "kernel launch");
+  });
+}

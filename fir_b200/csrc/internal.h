@@ -286,6 +286,11 @@ void launch_batch_filter(const BatchProblem* P, const BatchItem* items, int n_it
 // Resident blocks per SM of the projector at this block size.
 int batch_max_resident(int block);
 
+// penalty.cu: scale * the 26-neighbour quadratic penalty of nf frames as
+// n_partials partial sums, and its gradient (each or null).
+void launch_quadratic_penalty(int nx, int ny, int nz, int nf, const void* img, bool f64, double scale,
+                              double* partials, int n_partials, void* grad, cudaStream_t stream);
+
 // frames.cu: several frames per traversal, in groups of up to kMaxFramesPerPass
 // (measured on B200 at 8 frames of a clinical sinogram: two groups of 4 run
 // faster than one of 8, whose kernels need more registers).

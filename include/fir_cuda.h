@@ -394,6 +394,17 @@ fir_status fir_forward_frames(fir_ctx* ctx, const fir_vol_desc* vol, const void*
 fir_status fir_backward_frames(fir_ctx* ctx, const fir_proj_desc* proj, const void* sino, const fir_vol_desc* vol,
                                void* img, fir_dtype dtype);
 
+/* The quadratic smoothness penalty of the differentiable path over the
+ * n_frames frames of vol: with P = sum over frames and 26-neighbour pairs
+ * (j, k) of (x_j - x_k)^2 / |j - k| (|j - k| the centre distance in voxels),
+ * partials (FIR_PENALTY_PARTIALS doubles, or NULL) gets numbers whose sum is
+ * scale * P, and grad (or NULL, of img's type) the gradient of scale * P.  All
+ * pointers are memory of the current device; enqueued on stream (NULL: the
+ * default stream).  Differences, products and sums are double. */
+#define FIR_PENALTY_PARTIALS 1024
+fir_status fir_quadratic_penalty(const fir_vol_desc* vol, const void* img, fir_dtype dtype, double scale,
+                                 double* partials, void* grad, void* stream);
+
 /* ---- batched OSEM: many independent reconstructions at once ----
  *
  * No counterpart in FIR, which reconstructs one problem per process.  A
