@@ -777,7 +777,7 @@ def main():
         traffic = prof["dram_bytes_per_lor"] * (nb // nsub)
     roofline = {
         "bound": "hbm",
-        "kernel": "k_osem_subset (fused projection + ratio + backprojection)",
+        "kernel": "fused OSEM kernel (projection + ratio + backprojection): k_column_osem or k_osem_subset",
         "achieved": achieved,
         "peak": hbm,
         "unit": "GB/s",
