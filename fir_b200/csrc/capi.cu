@@ -2327,11 +2327,11 @@ fir_status fir_lor_paths(fir_ctx* ctx, const fir_proj_desc* proj, const fir_vol_
 
 // ====================================== OSEM sub-iteration without allocation
 //
-// fir_osem_subiteration_noalloc runs the same kernels as
-// fir_osem_subiteration, but takes its scratch memory (backprojection
+// fir_osem_subiteration_noalloc runs the sub-iteration LOR by LOR, with a
+// filter launch per axis, and takes its scratch memory (backprojection
 // accumulator, widened image, filter passes, pre-filter copy) from the
-// file-scope array below instead of from a context, and touches no host
-// memory, so it never allocates.  The array's device address is looked up
+// file-scope array below instead of from a context.  It touches no host
+// memory and never allocates.  The array's device address is looked up
 // once per device with cudaGetSymbolAddress; the name itself is only a host
 // stand-in and is never passed to a kernel.  This file defines no kernel, so
 // under CUDA's lazy module loading (the default) the array is reserved when
