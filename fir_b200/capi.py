@@ -87,6 +87,16 @@ class OsemParamsDesc(C.Structure):
     ]
 
 
+class TrackPlan(C.Structure):
+    """fir_track_plan_info."""
+
+    _fields_ = [
+        ("on_tracks", C.c_int), ("ring_pairs", C.c_int), ("tracks", C.c_int), ("threads", C.c_int),
+        ("block_pairs", C.c_int), ("block_tracks", C.c_int), ("shared_bytes", C.c_longlong),
+        ("warps", C.c_longlong), ("stops", C.c_double), ("clipped", C.c_double),
+    ]
+
+
 SAVE_FN = C.CFUNCTYPE(None, C.c_void_p, C.c_int, C.POINTER(C.c_float))
 
 _lib = None
@@ -149,6 +159,9 @@ _SIGS = {
                                      C.c_int]),
     "fir_backward_frames": (C.c_int, [C.c_void_p, C.POINTER(ProjDesc), C.c_void_p, C.POINTER(VolDesc), C.c_void_p,
                                       C.c_int]),
+    "fir_ctx_track_launch_count": (C.c_longlong, [C.c_void_p]),
+    "fir_track_plan": (C.c_int, [C.POINTER(ScannerDesc), C.POINTER(ProjDesc), C.POINTER(VolDesc), C.c_int, C.c_int,
+                                 C.c_int, C.c_int, C.c_int, C.POINTER(TrackPlan)]),
     "fir_quadratic_penalty": (C.c_int, [C.POINTER(VolDesc), C.c_void_p, C.c_int, C.c_double, C.c_void_p, C.c_void_p,
                                         C.c_void_p]),
     "fir_bin_coordinates": (C.c_int, [C.c_void_p, C.POINTER(ProjDesc), C.c_longlong, C.c_void_p, C.c_void_p,
@@ -299,6 +312,17 @@ def _dtype_of(x):
     return np.float64 if np.asarray(x).dtype == np.float64 else np.float32
 
 
+def track_plan(s: ScannerSpec, p: ProjSpec, v: VolSpec, n_subsets: int = 1, subset: int = 0,
+               geometry: int = FIR_GEOMETRY_REFERENCE, block_size: int = 0, skip_zero: bool = False) -> TrackPlan:
+    """How a projector launch over a subset would trace its LORs (no device
+    is needed)."""
+    out = TrackPlan()
+    _check(lib().fir_track_plan(C.byref(scanner_desc(s)), C.byref(proj_desc(p)), C.byref(vol_desc(v, 1)),
+                                int(n_subsets), int(subset), int(geometry), int(block_size), int(skip_zero),
+                                C.byref(out)))
+    return out
+
+
 PENALTY_PARTIALS = 1024
 
 
@@ -379,6 +403,11 @@ class Context:
     @property
     def launch_count(self) -> int:
         return int(lib().fir_ctx_launch_count(self._h))
+
+    @property
+    def track_launch_count(self) -> int:
+        """Projector launches that ran on transaxial tracks."""
+        return int(lib().fir_ctx_track_launch_count(self._h))
 
     def projector_time(self, reset: bool = True):
         """(device ms, launches) of projector kernels since the last reset

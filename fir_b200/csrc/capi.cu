@@ -560,6 +560,7 @@ void project_image(fir_ctx& c, const Grid& g, const Sino& s, const Tables& t, co
   {
     const double* wide = to_columns(c, g, img, nullptr);
     timed_launch(c, [&] { launch_column_forward(g, s, t, plan, wide, sino, ep, cfg_of(c)); });
+    ++c.track_launches;
     return;
   }
   const Widened w = widen_for_projection(c, g, img);
@@ -579,6 +580,7 @@ void backproject_subset(fir_ctx& c, const Grid& g, const Sino& s, const Tables& 
     float* acc = static_cast<float*>(c.bp_t.ensure(2 * (size_t)n * sizeof(float)));
     cuda_ok(cudaMemsetAsync(acc, 0, 2 * (size_t)n * sizeof(float), c.stream), "cudaMemsetAsync");
     timed_launch(c, [&] { launch_column_backward(g, s, t, plan, sino, acc, cfg_of(c)); });
+    ++c.track_launches;
     launch_from_columns(g, acc, img, cfg_of(c));
     after_launch(c);
     return;
@@ -618,6 +620,7 @@ const float* column_ratio_backproject(fir_ctx& c, const Grid& g, const Sino& s, 
   float* acc = nullptr;
   const double* wide = to_columns(c, g, img, &acc);
   timed_launch(c, [&] { launch_column_osem(g, s, t, p, wide, sino, mult, bias, acc, cfg_of(c)); });
+  ++c.track_launches;
   return acc;
 }
 
@@ -1727,6 +1730,44 @@ fir_status fir_ctx_synchronize(fir_ctx* ctx)
 }
 
 long long fir_ctx_launch_count(const fir_ctx* ctx) { return ctx != nullptr ? ctx->launches : -1; }
+
+long long fir_ctx_track_launch_count(const fir_ctx* ctx) { return ctx != nullptr ? ctx->track_launches : -1; }
+
+fir_status fir_track_plan(const fir_scanner_desc* scanner, const fir_proj_desc* proj, const fir_vol_desc* vol,
+                          int n_subsets, int subset, int geometry, int block_size, int skip_zero,
+                          fir_track_plan_info* out)
+{
+  return guarded(__func__, [&] {
+    const ScannerInfo sc = scanner_tables(scanner, true);
+    const ProjInfo p = check_proj(proj);
+    check_subsets(p, n_subsets);
+    const VolInfo v = check_vol(vol);
+    if (out == nullptr || subset < 0 || subset >= n_subsets || p.d.n_rings != sc.n_rings ||
+        p.d.n_crystals_per_ring != sc.n_cpr || block_size < 0 || block_size > 256 || block_size % 32 != 0 ||
+        (geometry != FIR_GEOMETRY_REFERENCE && geometry != FIR_GEOMETRY_EXACT))
+    {
+      fail(FIR_ERR_INVALID_ARGUMENT, "a plan needs a result, a subset, a sinogram of the scanner and valid options");
+    }
+    fir_ctx c;
+    c.geometry = geometry;
+    c.block = block_size > 0 ? block_size : c.block;
+    c.scan_z = sc.z;
+    c.scan_diameter = 2.0 * std::hypot(sc.xy[0], sc.xy[1]);
+    const Grid g = grid_of(c, v);
+    const Sino s = sino_of(p, n_subsets, subset);
+    const ColumnPlan plan = column_plan(g, s, c.scan_z.data(), c.block, skip_zero != 0);
+    out->on_tracks = columns_for(c, g, s, skip_zero != 0).tracks > 0 ? 1 : 0;
+    out->ring_pairs = plan.pairs;
+    out->tracks = plan.tracks;
+    out->threads = plan.block;
+    out->block_pairs = plan.share;
+    out->block_tracks = plan.per_block;
+    out->shared_bytes = (long long)column_smem(plan);
+    out->warps = column_warps(plan);
+    out->stops = column_stops(g, s, plan, c.scan_z.data(), c.scan_diameter);
+    out->clipped = column_clipped(g, s, c.scan_z.data(), c.scan_diameter);
+  });
+}
 
 fir_status fir_forward(fir_ctx* ctx, const fir_vol_desc* vol, const float* img, const fir_proj_desc* proj,
                        float* sino)

@@ -149,6 +149,7 @@ struct fir_ctx
   int step_limit = 0;  // FIR_OPT_STEP_LIMIT
   int traversal = FIR_TRAVERSAL_EXACT;  // FIR_OPT_TRAVERSAL
   long long launches = 0;
+  long long track_launches = 0;  // projector launches on transaxial tracks (column.cu)
   long long l2_bytes = 0;  // the device's L2 size, read on first use
 
   bool have_scanner = false;

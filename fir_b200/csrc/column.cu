@@ -153,7 +153,7 @@ __device__ __forceinline__ void list_nonzero(const Sino& s, const ColumnPlan& p,
 struct Leftover
 {
   int* count;
-  unsigned* lors;  // group << 16 | ring pair
+  unsigned* lors;  // their places (block_place)
 };
 
 __device__ __forceinline__ Leftover leftover(unsigned char* smem, const ColumnPlan& p)
@@ -271,8 +271,8 @@ __device__ __noinline__ void general_scatter(const Grid& g, const TrackHead& h, 
 
 // Sets up a lane's two LORs; go says which of them use the track.  Those that
 // need the general walk are left over.
-__device__ __forceinline__ void column_setup(const Grid& g, const Track& tr, const ColumnShare& c,
-                                             const ColumnLor lor[2], const Leftover& left, ColumnLane w[2],
+__device__ __forceinline__ void column_setup(const Grid& g, const ColumnPlan& p, const Track& tr,
+                                             const ColumnShare& c, const ColumnLor lor[2], const Leftover& left, ColumnLane w[2],
                                              bool go[2])
 {
 #pragma unroll
@@ -282,27 +282,29 @@ __device__ __forceinline__ void column_setup(const Grid& g, const Track& tr, con
     go[k] = kind == kLorColumn;
     if (kind == kLorGeneral)
     {
-      left.lors[atomicAdd(left.count, 1)] = (unsigned)c.group << 16 | (unsigned)lor[k].pair;
+      left.lors[atomicAdd(left.count, 1)] = block_place(p, BlockLor{c.group, lor[k].pair - c.begin});
     }
   }
 }
 
-// Calls trace(lor, track) for the block's leftover LORs.  Every thread of the
-// block calls this.
+// Calls trace(lor, track) for the leftover LORs of block number `block`.  Every
+// thread of the block calls this.
 template<class Trace>
 __device__ __forceinline__ void column_leftover(const Sino& s, const Tables& t, const ColumnPlan& p, int subset,
-                                                int first, unsigned char* smem, const Leftover& left, Trace&& trace)
+                                                int block, int first, unsigned char* smem, const Leftover& left,
+                                                Trace&& trace)
 {
   __syncthreads();
   for (int i = threadIdx.x; i < *left.count; i += blockDim.x)
   {
-    const unsigned v = left.lors[i];
+    const BlockLor l = block_lor(p, left.lors[i]);
     ColumnShare c;
-    c.group = (int)(v >> 16);
+    c.group = l.group;
     const int vt = first + c.group;
     c.sv = vt / s.n_tang;
     c.tang = vt - c.sv * s.n_tang;
-    trace(column_lor(s, t, p, c, subset, true, (int)(v & 0xffffu)), track_at(smem, p.cap, c.group));
+    trace(column_lor(s, t, p, c, subset, true, block % p.blocks * p.share + l.offset),
+          track_at(smem, p.cap, c.group));
   }
 }
 
@@ -366,7 +368,7 @@ __global__ void __launch_bounds__(256, 5) k_column_forward(const __grid_constant
     ColumnLane w[2] = {};
     bool go[2];
     float line[2];
-    column_setup(g, tr, c, lor, left, w, go);
+    column_setup(g, p, tr, c, lor, left, w, go);
     column_lines(tr, go, w, img, line);
 #pragma unroll
     for (int k = 0; k < 2; ++k)
@@ -377,7 +379,7 @@ __global__ void __launch_bounds__(256, 5) k_column_forward(const __grid_constant
       }
     }
   });
-  column_leftover(s, t, p, s.subset, first, smem, left, [&](const ColumnLor& lor, const Track& own) {
+  column_leftover(s, t, p, s.subset, (int)blockIdx.x, first, smem, left, [&](const ColumnLor& lor, const Track& own) {
     sino[lor.bin] = epilogue<EP>(general_line(g, *own.head, lor.z1, lor.z2, img, check).line);
   });
 }
@@ -406,7 +408,7 @@ __global__ void __launch_bounds__(256, 4) k_column_backward(const __grid_constan
     ColumnLane w[2] = {};
     bool go[2];
     double value[2];
-    column_setup(g, tr, c, lor, left, w, go);
+    column_setup(g, p, tr, c, lor, left, w, go);
 #pragma unroll
     for (int k = 0; k < 2; ++k)
     {
@@ -414,7 +416,7 @@ __global__ void __launch_bounds__(256, 4) k_column_backward(const __grid_constan
     }
     column_scatter(tr, go, w, value, accumulator_of(g, *tr.head, acc));
   });
-  column_leftover(s, t, p, s.subset, first, smem, left, [&](const ColumnLor& lor, const Track& own) {
+  column_leftover(s, t, p, s.subset, (int)blockIdx.x, first, smem, left, [&](const ColumnLor& lor, const Track& own) {
     const double v = sino != nullptr ? (double)__ldg(sino + lor.bin) : 1.0;
     general_scatter(g, *own.head, lor.z1, lor.z2, v, accumulator_of(g, *own.head, acc), check);
   });
@@ -464,7 +466,7 @@ __device__ __forceinline__ void column_osem(const Grid& g, const Sino& s, const 
     ColumnLane w[2] = {};
     bool go[2];
     float line[2];
-    column_setup(g, tr, c, lor, left, w, go);
+    column_setup(g, p, tr, c, lor, left, w, go);
     column_lines(tr, go, w, img, line);
     double value[2] = {0.0, 0.0};
 #pragma unroll
@@ -474,7 +476,7 @@ __device__ __forceinline__ void column_osem(const Grid& g, const Sino& s, const 
     }
     column_scatter(tr, go, w, value, accumulator_of(g, *tr.head, acc));
   });
-  column_leftover(s, t, p, subset, first, smem, left, [&](const ColumnLor& lor, const Track& own) {
+  column_leftover(s, t, p, subset, block, first, smem, left, [&](const ColumnLor& lor, const Track& own) {
     const GeneralLine gl = general_line(g, *own.head, lor.z1, lor.z2, img, check);
     double q;
     if (osem_ratio<kWeighted>(gl.line, lor.bin, sino, mult, bias, q) && gl.ok)
@@ -680,7 +682,7 @@ ColumnPlan column_plan(const Grid& g, const Sino& s, const double* z, int block,
 
 // Share of the ring pairs whose LOR through the axis meets the volume but
 // enters or leaves it through an end face: those take the general walk.
-static double clipped_share(const Grid& g, const Sino& s, const double* z, double diameter)
+double column_clipped(const Grid& g, const Sino& s, const double* z, double diameter)
 {
   if (z[0] > g.low[2] && z[0] < g.high[2] && z[2 * s.n_rings - 2] > g.low[2] && z[2 * s.n_rings - 2] < g.high[2])
   {
@@ -708,7 +710,7 @@ static double clipped_share(const Grid& g, const Sino& s, const double* z, doubl
 // Mean number of z crossings that stop a warp's turn per crossing of its
 // track: the LORs of a segment cross together where their planes lie whole
 // voxels apart, so a segment counts once per distinct offset.
-static double stops_per_turn(const Grid& g, const Sino& s, const ColumnPlan& p, const double* z, double diameter)
+double column_stops(const Grid& g, const Sino& s, const ColumnPlan& p, const double* z, double diameter)
 {
   const double apart = s.n_rings > 1 ? std::fabs(z[2] - z[0]) * (s.span > 1 ? 0.5 : 1.0) / g.ext[2] : 0.0;
   int offsets = 1;
@@ -745,7 +747,7 @@ bool columns_pay(const Grid& g, const Sino& s, const ColumnPlan& p, const double
   {
     return false;
   }
-  return stops_per_turn(g, s, p, z, diameter) <= 2.2 && clipped_share(g, s, z, diameter) <= 0.04;
+  return column_stops(g, s, p, z, diameter) <= 2.2 && column_clipped(g, s, z, diameter) <= 0.04;
 }
 
 void launch_to_columns(const Grid& g, const float* in, double* out, float* acc, const LaunchCfg& cfg)

@@ -41,6 +41,23 @@ struct ColumnPlan
 // Shared memory of one block.
 size_t column_smem(const ColumnPlan& p);
 
+// A LOR that its block leaves to the general walk, as the number of its place
+// in the block (places are below per_block * share, whatever the number of
+// ring pairs): the block's track, and the ring pair counted from the first
+// one of the block's part.
+struct BlockLor
+{
+  int group, offset;
+};
+__host__ __device__ inline unsigned block_place(const ColumnPlan& p, BlockLor l)
+{
+  return (unsigned)(l.group * p.share + l.offset);
+}
+__host__ __device__ inline BlockLor block_lor(const ColumnPlan& p, unsigned place)
+{
+  return BlockLor{(int)place / p.share, (int)place % p.share};
+}
+
 struct LaunchCfg
 {
   int block;
@@ -79,6 +96,9 @@ int column_blocks(const ColumnPlan& p);
 // Warps of the launch that have work; below kColumnWarps a launch alone is
 // faster LOR by LOR.
 long long column_warps(const ColumnPlan& p);
+// What columns_pay looks at: see there.
+double column_stops(const Grid& g, const Sino& s, const ColumnPlan& p, const double* z, double diameter);
+double column_clipped(const Grid& g, const Sino& s, const double* z, double diameter);
 constexpr long long kColumnWarps = 6 * 592;
 // Whether a launch with enough warps is faster on tracks than LOR by LOR (z:
 // the scanner's slice centres, diameter: of a ring).

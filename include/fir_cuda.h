@@ -218,6 +218,31 @@ fir_status fir_ctx_set_scanner(fir_ctx* ctx, const fir_scanner_desc* scanner);
 fir_status fir_ctx_synchronize(fir_ctx* ctx);
 /* Number of kernels this context launched since creation (all entry points). */
 long long fir_ctx_launch_count(const fir_ctx* ctx);
+/* Those of the projectors that ran on transaxial tracks (see fir_track_plan). */
+long long fir_ctx_track_launch_count(const fir_ctx* ctx);
+
+/* How a projector launch over one subset would trace its LORs.  On tracks the
+ * transaxial crossings of a view and tangential bin are listed once for all
+ * its ring pairs; otherwise every LOR is traced by itself.  Both give FIR's
+ * projections bit for bit.  Host arithmetic only: no device is needed. */
+typedef struct fir_track_plan_info
+{
+  int on_tracks;          /* 1: the launch runs on tracks */
+  int ring_pairs;         /* LORs that share a track */
+  int tracks;             /* (view, tangential bin) pairs of the subset */
+  int threads;            /* per block */
+  int block_pairs;        /* ring pairs of a block's part of a track, at most */
+  int block_tracks;       /* tracks of a block, at most */
+  long long shared_bytes; /* shared memory of a block */
+  long long warps;        /* of the launch */
+  double stops;           /* axial crossings that stop a warp, per transaxial one */
+  double clipped;         /* share of the LORs that take the general walk */
+} fir_track_plan_info;
+/* geometry: FIR_GEOMETRY_*; block_size: FIR_OPT_BLOCK_SIZE (0: the default);
+ * skip_zero: FIR_OPT_SKIP_ZERO_BINS. */
+fir_status fir_track_plan(const fir_scanner_desc* scanner, const fir_proj_desc* proj, const fir_vol_desc* vol,
+                          int n_subsets, int subset, int geometry, int block_size, int skip_zero,
+                          fir_track_plan_info* out);
 /* With FIR_OPT_TIMING on: waits for the recorded events and returns the total
  * device time (ms) and number of projector-kernel launches since the last
  * reset; reset != 0 clears the totals. */
