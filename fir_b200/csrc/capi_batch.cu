@@ -487,6 +487,10 @@ fir_status fir_batch_create(fir_batch** out, fir_ctx* ctx, int n_problems, const
       const ScannerInfo& sc = scan[(size_t)k];
       plans[(size_t)k] = column_plan(g, s, sc.z.data(), kBatchColumnBlock, b->skip_zero, true);
       q.plan = column_plan(g, s, sc.z.data(), c.block, b->skip_zero);
+      if (column_smem(q.plan) > kColumnSharedLimit)
+      {
+        q.plan = plans[(size_t)k];  // (columns_pay has looked at this one)
+      }
       if (columns_pay(g, s, plans[(size_t)k], sc.z.data(), 2.0 * std::hypot(sc.xy[0], sc.xy[1])))
       {
         pays[(size_t)k] = 1;

@@ -617,14 +617,15 @@ __global__ void __launch_bounds__(kTile * kTileRows) k_em_update_columns(int np,
   }
 }
 
-// Shared memory above 48 KB is asked for once per kernel and call.
+// Allows a kernel shared memory above 48 KB.  The limit belongs to the kernel,
+// which all contexts and threads share, so that it is always the same one: a
+// call that set its own need would take away a larger one that another thread
+// has just asked for.  False (and an error for cudaGetLastError) if it fails.
 template<typename K>
-void ask_shared(K kernel, size_t bytes)
+bool ask_shared(K kernel, size_t bytes)
 {
-  if (bytes > 48 * 1024)
-  {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  }
+  return bytes <= 48 * 1024 || cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                    (int)kColumnSharedLimit) == cudaSuccess;
 }
 }  // namespace
 
@@ -743,7 +744,7 @@ long long column_warps(const ColumnPlan& p) { return (long long)p.tracks * ((p.p
 // volumes, 0.96x at 2.3 on a 320x320x128 one).
 bool columns_pay(const Grid& g, const Sino& s, const ColumnPlan& p, const double* z, double diameter)
 {
-  if (g.exact_only || p.pairs < 30 || column_smem(p) > 96 * 1024 || (long long)g.nxy * g.nz >= 1LL << 29)
+  if (g.exact_only || p.pairs < 30 || column_smem(p) > kColumnSharedLimit || (long long)g.nxy * g.nz >= 1LL << 29)
   {
     return false;
   }
@@ -776,7 +777,10 @@ void launch_column_forward(const Grid& g, const Sino& s, const Tables& t, const 
   }
   const size_t bytes = column_smem(p);
   auto* kernel = ep == FwdEpilogue::Exp ? k_column_forward<FwdEpilogue::Exp> : k_column_forward<FwdEpilogue::None>;
-  ask_shared(kernel, bytes);
+  if (!ask_shared(kernel, bytes))
+  {
+    return;
+  }
   kernel<<<(unsigned)column_blocks(p), p.block, bytes, cfg.stream>>>(g, s, t, p, img, sino, cfg.check);
 }
 
@@ -789,7 +793,10 @@ void launch_column_backward(const Grid& g, const Sino& s, const Tables& t, const
   }
   const size_t bytes = column_smem(p);
   auto* kernel = p.skip ? k_column_backward<true> : k_column_backward<false>;
-  ask_shared(kernel, bytes);
+  if (!ask_shared(kernel, bytes))
+  {
+    return;
+  }
   kernel<<<(unsigned)column_blocks(p), p.block, bytes, cfg.stream>>>(g, s, t, p, sino, acc, cfg.check);
 }
 
@@ -801,7 +808,10 @@ void launch_batch_column_osem(const BatchProblem* P, const BatchItem* items, int
     return;
   }
   auto* kernel = skip ? k_batch_column_osem<true> : k_batch_column_osem<false>;
-  ask_shared(kernel, bytes);
+  if (!ask_shared(kernel, bytes))
+  {
+    return;
+  }
   kernel<<<(unsigned)n_blocks, kBatchColumnBlock, bytes, stream>>>(P, items, n_items, check);
 }
 
@@ -816,7 +826,10 @@ void launch_column_osem(const Grid& g, const Sino& s, const Tables& t, const Col
   const bool skip = p.skip != 0;
   auto* kernel = mult != nullptr ? (skip ? k_column_osem<true, true> : k_column_osem<true, false>)
                                  : (skip ? k_column_osem<false, true> : k_column_osem<false, false>);
-  ask_shared(kernel, bytes);
+  if (!ask_shared(kernel, bytes))
+  {
+    return;
+  }
   kernel<<<(unsigned)column_blocks(p), p.block, bytes, cfg.stream>>>(g, s, t, p, img, sino, mult, bias, acc, cfg.check);
 }
 }  // namespace fir

@@ -40,6 +40,8 @@ struct ColumnPlan
 };
 // Shared memory of one block.
 size_t column_smem(const ColumnPlan& p);
+// The most that a plan may ask for.
+constexpr size_t kColumnSharedLimit = 96 * 1024;
 
 // A LOR that its block leaves to the general walk, as the number of its place
 // in the block (places are below per_block * share, whatever the number of
