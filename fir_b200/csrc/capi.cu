@@ -517,19 +517,19 @@ ColumnPlan columns_for(fir_ctx& c, const Grid& g, const Sino& s, bool skip)
   return p;
 }
 
-// The image's double copy and two zeroed accumulators in z columns, in context
-// scratch (acc may be null).
-const double* to_columns(fir_ctx& c, const Grid& g, const float* img, float** acc)
+// Writes the image's double copy in z columns to context scratch and clears
+// the two accumulators at acc (or null).
+const double* to_columns(fir_ctx& c, const Grid& g, const float* img, float* acc)
 {
-  const size_t n = (size_t)g.nxy * g.nz;
-  double* d = static_cast<double*>(c.wide.ensure(n * sizeof(double)));
-  if (acc != nullptr)
-  {
-    *acc = static_cast<float*>(c.bp_t.ensure(2 * n * sizeof(float)));
-  }
-  launch_to_columns(g, img, d, acc != nullptr ? *acc : nullptr, cfg_of(c));
+  double* d = static_cast<double*>(c.wide.ensure((size_t)g.nxy * g.nz * sizeof(double)));
+  launch_to_columns(g, img, d, acc, cfg_of(c));
   after_launch(c);
   return d;
+}
+
+float* column_accumulators(fir_ctx& c, const Grid& g)
+{
+  return static_cast<float*>(c.bp_t.ensure(2 * (size_t)g.nxy * g.nz * sizeof(float)));
 }
 
 // s with the compacted list of its bins whose measured value is not 0
@@ -567,17 +567,17 @@ void project_image(fir_ctx& c, const Grid& g, const Sino& s, const Tables& t, co
   timed_launch(c, [&] { launch_forward(g, s, t, w.img, w.img_t, sino, ep, cfg_of(c)); });
 }
 
-// img += backprojection of sino (nullptr: all ones) over the subset of s, in
-// the atomic mode; LORs running mostly along x accumulate in an x/y-exchanged
-// scratch image that is added into img afterwards, while both fit in L2.
-void backproject_subset(fir_ctx& c, const Grid& g, const Sino& s, const Tables& t, const float* sino, float* img,
-                        bool skip_zero)
+// img = backprojection of sino (nullptr: all ones) over the subset of s, in the
+// atomic mode: on the tracks of plan, or (plan.tracks = 0) LOR by LOR, where
+// LORs running mostly along x accumulate in an x/y-exchanged scratch image that
+// is added into img afterwards, while both fit in L2.
+void backproject_subset(fir_ctx& c, const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& plan,
+                        const float* sino, float* img, bool skip_zero)
 {
-  const ColumnPlan plan = columns_for(c, g, s, skip_zero && sino != nullptr);
   const long long n = (long long)g.nxy * g.nz;
   if (plan.tracks > 0)
   {
-    float* acc = static_cast<float*>(c.bp_t.ensure(2 * (size_t)n * sizeof(float)));
+    float* acc = column_accumulators(c, g);
     cuda_ok(cudaMemsetAsync(acc, 0, 2 * (size_t)n * sizeof(float), c.stream), "cudaMemsetAsync");
     timed_launch(c, [&] { launch_column_backward(g, s, t, plan, sino, acc, cfg_of(c)); });
     ++c.track_launches;
@@ -585,6 +585,7 @@ void backproject_subset(fir_ctx& c, const Grid& g, const Sino& s, const Tables& 
     after_launch(c);
     return;
   }
+  cuda_ok(cudaMemsetAsync(img, 0, (size_t)n * sizeof(float), c.stream), "cudaMemsetAsync");
   float* img_t = nullptr;
   if (use_exchanged(c, g, 8.0))
   {
@@ -601,15 +602,39 @@ void backproject_subset(fir_ctx& c, const Grid& g, const Sino& s, const Tables& 
   }
 }
 
-// Whether the fused sub-iteration runs on transaxial tracks; p is its plan.
-bool osem_columns(fir_ctx& c, const Grid& g, const Sino& s, ColumnPlan& p)
+// Frame k of img = backprojection of sino (nullptr: all ones) over subset k.
+void backproject_subsets(fir_ctx& c, const ProjInfo& p, const VolInfo& v, const Grid& g, const Tables& t,
+                         const float* sino, float* img, int n_subsets)
+{
+  const bool skip = c.skip_zero != 0 && sino != nullptr;
+  ColumnPlan plan{};
+  if (c.backproj == FIR_BACKPROJ_ATOMIC)
+  {
+    plan = columns_for(c, g, sino_of(p, n_subsets, 0), skip);
+  }
+  for (int k = 0; k < n_subsets; ++k)
+  {
+    const Sino s = sino_of(p, n_subsets, k);
+    float* out = img + (size_t)k * v.nvox;
+    if (c.backproj == FIR_BACKPROJ_DETERMINISTIC)
+    {
+      cuda_ok(cudaMemsetAsync(out, 0, (size_t)v.nvox * sizeof(float), c.stream), "cudaMemsetAsync");
+      det_backproject(c, g, s, t, sino, false, out, v.nvox);
+      continue;
+    }
+    backproject_subset(c, g, s, t, plan, sino, out, skip);
+  }
+}
+
+// The plan of the fused sub-iteration's launches.  The subsets of one call have the same
+// number of views, and so one plan.
+ColumnPlan osem_columns(fir_ctx& c, const Grid& g, const Sino& s)
 {
   if (c.backproj != FIR_BACKPROJ_ATOMIC || c.traversal != FIR_TRAVERSAL_EXACT)
   {
-    return false;
+    return ColumnPlan{};
   }
-  p = columns_for(c, g, s, c.skip_zero != 0);
-  return p.tracks > 0;
+  return columns_for(c, g, s, c.skip_zero != 0);
 }
 
 // The backprojection of ratio_backproject in z columns (context scratch).
@@ -617,37 +642,35 @@ const float* column_ratio_backproject(fir_ctx& c, const Grid& g, const Sino& s, 
                                       const ColumnPlan& p, const float* img, const float* sino, const float* mult,
                                       const float* bias)
 {
-  float* acc = nullptr;
-  const double* wide = to_columns(c, g, img, &acc);
+  float* acc = column_accumulators(c, g);
+  const double* wide = to_columns(c, g, img, acc);
   timed_launch(c, [&] { launch_column_osem(g, s, t, p, wide, sino, mult, bias, acc, cfg_of(c)); });
   ++c.track_launches;
   return acc;
 }
 
-// bp (zeroed by the caller, or with defer_merge here) += backprojection of
-// sino / (projection of img + bias) over the subset of s: the fused kernel, or in deterministic mode the
-// ratio kernel followed by the ordered scatter.  The fused kernel reads and
+// bp = backprojection of sino / (projection of img + bias) over the subset of
+// s: the fused kernel, on the tracks of plan or (plan.tracks = 0) LOR by LOR, or
+// in deterministic mode the ratio kernel followed by the ordered scatter.  LOR
+// by LOR, the fused kernel reads and
 // accumulates LORs that run mostly along x in images with x and y exchanged
 // (double copy and accumulator in context scratch); the accumulator is added
 // back into bp after the kernel, or, with defer_merge, returned (null: none)
 // for the caller to add (launch_em_update_oriented).
-const float* ratio_backproject(fir_ctx& c, const Grid& g, const Sino& s_all, const Tables& t, const float* img,
-                               const float* sino, const float* mult, const float* bias, float* bp, long long nvox,
-                               bool defer_merge = false)
+const float* ratio_backproject(fir_ctx& c, const Grid& g, const Sino& s_all, const Tables& t, const ColumnPlan& plan,
+                               const float* img, const float* sino, const float* mult, const float* bias, float* bp,
+                               long long nvox, bool defer_merge = false)
 {
-  ColumnPlan plan;
-  if (osem_columns(c, g, s_all, plan))
+  if (plan.tracks > 0)
   {
     const float* acc = column_ratio_backproject(c, g, s_all, t, plan, img, sino, mult, bias);
     launch_from_columns(g, acc, bp, cfg_of(c));
     after_launch(c);
     return nullptr;
   }
-  const bool exchanged = c.backproj == FIR_BACKPROJ_ATOMIC && c.traversal == FIR_TRAVERSAL_EXACT && use_exchanged(c, g);
-  if (defer_merge && !exchanged)
-  {
+  auto clear_bp = [&] {
     cuda_ok(cudaMemsetAsync(bp, 0, (size_t)nvox * sizeof(float), c.stream), "cudaMemsetAsync");
-  }
+  };
   // skipped bins: listed out of the atomic kernels' enumeration
   const bool listed = c.skip_zero != 0 && c.backproj == FIR_BACKPROJ_ATOMIC && s_all.n_enum > 0;
   const Sino s = listed ? nonzero_bins(c, s_all, sino) : s_all;
@@ -656,6 +679,7 @@ const float* ratio_backproject(fir_ctx& c, const Grid& g, const Sino& s_all, con
   {
     // the opt-in float loop: float images in both orientations while they
     // and the accumulators fit in L2 (16 B per voxel)
+    clear_bp();
     const size_t n = (size_t)nvox;
     float* img_t = nullptr;
     float* bp_t = nullptr;
@@ -683,7 +707,7 @@ const float* ratio_backproject(fir_ctx& c, const Grid& g, const Sino& s_all, con
   }
   if (c.backproj == FIR_BACKPROJ_DETERMINISTIC)
   {
-    const double* wimg = widen(c, img, nvox);
+    const double* wimg = widen(c, img, nvox, bp);
     // the ratio and, from the same walks, the pair count of every LOR
     const size_t ne = (size_t)std::max(s.n_enum, 1);
     float* ratio = static_cast<float*>(c.ratio.ensure(ne * (sizeof(float) + sizeof(int))));
@@ -699,6 +723,7 @@ const float* ratio_backproject(fir_ctx& c, const Grid& g, const Sino& s_all, con
       // the double copy and the accumulator (12 B/voxel) overflow L2, the
       // float image and the accumulator (8 B/voxel) fit: gather floats, one
       // launch per orientation, each with its own image and accumulator
+      clear_bp();
       const size_t n = (size_t)nvox;
       float* img_t = static_cast<float*>(c.img_t.ensure(n * sizeof(float)));
       float* bp_t = static_cast<float*>(c.bp_t.ensure(n * sizeof(float)));
@@ -717,7 +742,7 @@ const float* ratio_backproject(fir_ctx& c, const Grid& g, const Sino& s_all, con
       after_launch(c);
       return nullptr;
     }
-    const double* wimg = widen(c, img, nvox);
+    const double* wimg = widen(c, img, nvox, bp);
     timed_launch(c, [&] {
       launch_osem_subset(g, s, t, wimg, nullptr, sino, mult, bias, bp, nullptr, c.skip_zero != 0, cfg_of(c));
     });
@@ -727,7 +752,7 @@ const float* ratio_backproject(fir_ctx& c, const Grid& g, const Sino& s_all, con
   double* wimg = static_cast<double*>(c.wide.ensure(n * sizeof(double)));
   double* wimg_t = static_cast<double*>(c.wide_t.ensure(n * sizeof(double)));
   float* bp_t = static_cast<float*>(c.bp_t.ensure(n * sizeof(float)));
-  launch_widen_oriented(g.nx, g.ny, g.nz, img, wimg, wimg_t, defer_merge ? bp : nullptr, bp_t, cfg_of(c));
+  launch_widen_oriented(g.nx, g.ny, g.nz, img, wimg, wimg_t, bp, bp_t, cfg_of(c));
   after_launch(c);
   timed_launch(c, [&] {
     launch_osem_subset(g, s, t, wimg, wimg_t, sino, mult, bias, bp, bp_t, c.skip_zero != 0, cfg_of(c));
@@ -1120,7 +1145,7 @@ void check_osem_params(const fir_osem_params* prm, const ProjInfo& p)
 }
 
 // Device-pointer body of one OSEM sub-iteration.
-void osem_subiteration_device(fir_ctx& c, const ProjInfo& p, const Tables& t, const Grid& g,
+void osem_subiteration_device(fir_ctx& c, const ProjInfo& p, const Tables& t, const Grid& g, const ColumnPlan& plan,
                               const VolInfo& v, const float* sino, const float* mult, const float* bias, float* img,
                               const float* sens_frame, const fir_osem_params* prm, int subset,
                               int subiter)
@@ -1134,8 +1159,7 @@ void osem_subiteration_device(fir_ctx& c, const ProjInfo& p, const Tables& t, co
   // a small volume is filtered in one launch, from the EM step's scratch image
   const bool fused = f.wanted && conv_fused_fits(g.nx, g.ny, g.nz, f.x, f.y, f.z);
   float* out = fused ? static_cast<float*>(c.conv1.ensure((size_t)v.nvox * sizeof(float))) : img;
-  ColumnPlan plan;
-  if (osem_columns(c, g, s, plan))
+  if (plan.tracks > 0)
   {
     const float* acc = column_ratio_backproject(c, g, s, t, plan, img, sino, mult, bias);
     launch_em_update_columns(g, img, out, acc, sens_frame, cfg_of(c));
@@ -1143,7 +1167,7 @@ void osem_subiteration_device(fir_ctx& c, const ProjInfo& p, const Tables& t, co
   else
   {
     float* bp = static_cast<float*>(c.bp.ensure((size_t)v.nvox * sizeof(float)));
-    const float* bp_t = ratio_backproject(c, g, s, t, img, sino, mult, bias, bp, v.nvox, true);
+    const float* bp_t = ratio_backproject(c, g, s, t, plan, img, sino, mult, bias, bp, v.nvox, true);
     if (bp_t != nullptr)
     {
       launch_em_update_oriented(g.nx, g.ny, g.nz, img, out, bp, bp_t, sens_frame, cfg_of(c));
@@ -1174,17 +1198,16 @@ void osem_subiteration_device(fir_ctx& c, const ProjInfo& p, const Tables& t, co
 // parameters is part of the system model (projection of B x, B applied to
 // the backprojection, sens_frame already blurred).
 void osem_psf_subiteration_device(fir_ctx& c, const ProjInfo& p, const Tables& t, const Grid& g,
-                                  const VolInfo& v, const float* sino, const float* mult, const float* bias, float* img,
+                                  const ColumnPlan& plan, const VolInfo& v, const float* sino, const float* mult, const float* bias, float* img,
                                   const float* sens_frame, const fir_osem_params* prm, int subset, int subiter)
 {
   const size_t bytes = (size_t)v.nvox * sizeof(float);
   float* bp = static_cast<float*>(c.bp.ensure(bytes));
   float* blur = static_cast<float*>(c.psf_blur.ensure(bytes));
-  cuda_ok(cudaMemsetAsync(bp, 0, bytes, c.stream), "cudaMemsetAsync");
   cuda_ok(cudaMemcpyAsync(blur, img, bytes, cudaMemcpyDeviceToDevice, c.stream), "cudaMemcpyAsync");
   convolve_device(c, v, blur, prm->fwhm_xyz, prm->cut_radius);
   const Sino s = sino_of(p, prm->n_subsets, subset);
-  ratio_backproject(c, g, s, t, blur, sino, mult, bias, bp, v.nvox);
+  ratio_backproject(c, g, s, t, plan, blur, sino, mult, bias, bp, v.nvox);
   convolve_device(c, v, bp, prm->fwhm_xyz, prm->cut_radius);
   launch_em_update(v.nvox, img, img, bp, sens_frame, cfg_of(c));
   after_launch(c);
@@ -1333,6 +1356,7 @@ void osem_run(fir_ctx& c, const fir_proj_desc* proj, const float* sino, const fl
   }
   std::vector<float> host_copy;
   cut_device(c, v, dimg, params->cut_radius, 1);
+  const ColumnPlan plan = osem_columns(c, g, sino_of(p, params->n_subsets, 0));
   const int nsub_total = params->n_iterations * params->n_subsets;
   for (int iter = 0; iter < params->n_iterations; ++iter)
   {
@@ -1346,11 +1370,11 @@ void osem_run(fir_ctx& c, const fir_proj_desc* proj, const float* sino, const fl
       }
       if (psf)
       {
-        osem_psf_subiteration_device(c, p, t, g, v, dsino, dmult, dbias, dimg, sframe, params, subset, subiter);
+        osem_psf_subiteration_device(c, p, t, g, plan, v, dsino, dmult, dbias, dimg, sframe, params, subset, subiter);
       }
       else
       {
-        osem_subiteration_device(c, p, t, g, v, dsino, dmult, dbias, dimg, sframe, params, subset, subiter);
+        osem_subiteration_device(c, p, t, g, plan, v, dsino, dmult, dbias, dimg, sframe, params, subset, subiter);
       }
       if (save != nullptr && params->save_interval > 0 && subiter % params->save_interval == 0 &&
           subiter != nsub_total)
@@ -1409,6 +1433,7 @@ void osem_reso_reco_run(fir_ctx& c, const fir_proj_desc* proj, const float* sino
   convolve_device(c, frames, dsens, params->fwhm_xyz, params->cut_radius);
   const bool conv = params->convolution_interval > 0 && params->fwhm_xyz[0] > 0.0 &&
                     params->fwhm_xyz[1] > 0.0 && params->fwhm_xyz[2] > 0.0;
+  const ColumnPlan plan = osem_columns(c, g, sino_of(p, params->n_subsets, 0));
   const int nsub_total = params->n_iterations * params->n_subsets;
   std::vector<float> host_copy;
   for (int iter = 0; iter < params->n_iterations; ++iter)
@@ -1416,9 +1441,8 @@ void osem_reso_reco_run(fir_ctx& c, const fir_proj_desc* proj, const float* sino
     for (int subset = 0; subset < params->n_subsets; ++subset)
     {
       const int subiter = iter * params->n_subsets + subset + 1;
-      cuda_ok(cudaMemsetAsync(bp, 0, bytes, c.stream), "cudaMemsetAsync");
       const Sino s = sino_of(p, params->n_subsets, subset);
-      ratio_backproject(c, g, s, t, dimg, dsino, nullptr, dbias, bp, v.nvox);
+      ratio_backproject(c, g, s, t, plan, dimg, dsino, nullptr, dbias, bp, v.nvox);
       convolve_device(c, v, bp, params->fwhm_xyz, params->cut_radius);
       launch_em_update_image_first(v.nvox, dimg, bp, dsens + (size_t)subset * v.nvox, cfg_of(c));
       after_launch(c);
@@ -1814,24 +1838,14 @@ fir_status fir_backward(fir_ctx* ctx, const fir_proj_desc* proj, const float* si
     check_frames(v, n_subsets);
     const Tables t = tables_of(c, p);
     const Grid g = grid_of(c, v);
-    if (sino == nullptr)
+    if (sino == nullptr || img == nullptr)
     {
-      fail(FIR_ERR_INVALID_ARGUMENT, "sinogram is NULL");
+      fail(FIR_ERR_INVALID_ARGUMENT, sino == nullptr ? "sinogram is NULL" : "image is NULL");
     }
     Stager st(c);
     const float* dsino = st.in(sino, p.g.n_bins);
     float* dimg = st.out(img, v.nvox * n_subsets);
-    cuda_ok(cudaMemsetAsync(dimg, 0, (size_t)(v.nvox * n_subsets) * sizeof(float), c.stream), "cudaMemsetAsync");
-    for (int s = 0; s < n_subsets; ++s)
-    {
-      const Sino ss = sino_of(p, n_subsets, s);
-      if (c.backproj == FIR_BACKPROJ_DETERMINISTIC)
-      {
-        det_backproject(c, g, ss, t, dsino, false, dimg + (size_t)s * v.nvox, v.nvox);
-        continue;
-      }
-      backproject_subset(c, g, ss, t, dsino, dimg + (size_t)s * v.nvox, c.skip_zero != 0);
-    }
+    backproject_subsets(c, p, v, g, t, dsino, dimg, n_subsets);
     finish(c, st);
   });
 }
@@ -1938,19 +1952,13 @@ fir_status fir_sensitivity(fir_ctx* ctx, const fir_proj_desc* proj, const fir_vo
     check_frames(v, n_subsets);
     const Tables t = tables_of(c, p);
     const Grid g = grid_of(c, v);
+    if (sens == nullptr)
+    {
+      fail(FIR_ERR_INVALID_ARGUMENT, "sensitivity is NULL");
+    }
     Stager st(c);
     float* dsens = st.out(sens, v.nvox * n_subsets);
-    cuda_ok(cudaMemsetAsync(dsens, 0, (size_t)(v.nvox * n_subsets) * sizeof(float), c.stream), "cudaMemsetAsync");
-    for (int s = 0; s < n_subsets; ++s)
-    {
-      const Sino ss = sino_of(p, n_subsets, s);
-      if (c.backproj == FIR_BACKPROJ_DETERMINISTIC)
-      {
-        det_backproject(c, g, ss, t, nullptr, false, dsens + (size_t)s * v.nvox, v.nvox);
-        continue;
-      }
-      backproject_subset(c, g, ss, t, nullptr, dsens + (size_t)s * v.nvox, false);
-    }
+    backproject_subsets(c, p, v, g, t, nullptr, dsens, n_subsets);
     finish(c, st);
   });
 }
@@ -1980,7 +1988,8 @@ fir_status fir_osem_subiteration(fir_ctx* ctx, const fir_proj_desc* proj, const 
     const float* dbias = st.in(bias, p.g.n_bins);
     const float* dsens = st.in(sens_frame, v.nvox);
     float* dimg = st.inout(img, v.nvox);
-    osem_subiteration_device(c, p, t, g, v, dsino, nullptr, dbias, dimg, dsens, params, subset, subiter);
+    const ColumnPlan plan = osem_columns(c, g, sino_of(p, params->n_subsets, subset));
+    osem_subiteration_device(c, p, t, g, plan, v, dsino, nullptr, dbias, dimg, dsens, params, subset, subiter);
     finish(c, st);
   });
 }
@@ -2051,9 +2060,8 @@ fir_status fir_ratio_backprojection(fir_ctx* ctx, const fir_proj_desc* proj, con
     const float* dbias = st.in(bias, p.g.n_bins);
     const float* dimg = st.in(img, v.nvox);
     float* dbp = st.out(bp, v.nvox);
-    cuda_ok(cudaMemsetAsync(dbp, 0, (size_t)v.nvox * sizeof(float), c.stream), "cudaMemsetAsync");
     const Sino s = sino_of(p, n_subsets, subset);
-    ratio_backproject(c, g, s, t, dimg, dsino, nullptr, dbias, dbp, v.nvox);
+    ratio_backproject(c, g, s, t, osem_columns(c, g, s), dimg, dsino, nullptr, dbias, dbp, v.nvox);
     finish(c, st);
   });
 }
@@ -2087,12 +2095,15 @@ fir_status fir_ratio_backprojection_shard(fir_ctx* ctx, const fir_proj_desc* pro
     const float* dbias = st.in(bias, p.g.n_bins);
     const float* dimg = st.in(img, v.nvox);
     float* dbp = st.out(bp, v.nvox);
-    cuda_ok(cudaMemsetAsync(dbp, 0, (size_t)v.nvox * sizeof(float), c.stream), "cudaMemsetAsync");
     // the subset's views subset + n_subsets * k with k % n_shards == shard
     const Sino s = sino_of_views(p, n_subsets * n_shards, subset + n_subsets * shard);
     if (s.n_enum > 0)
     {
-      ratio_backproject(c, g, s, t, dimg, dsino, nullptr, dbias, dbp, v.nvox);
+      ratio_backproject(c, g, s, t, osem_columns(c, g, s), dimg, dsino, nullptr, dbias, dbp, v.nvox);
+    }
+    else
+    {
+      cuda_ok(cudaMemsetAsync(dbp, 0, (size_t)v.nvox * sizeof(float), c.stream), "cudaMemsetAsync");
     }
     finish(c, st);
   });

@@ -42,3 +42,41 @@ def test_more_ring_pairs_than_16_bits_number():
     got, want = forward_both(track, single, proj, vol, x)
     np.testing.assert_array_equal(got, want)
     assert np.count_nonzero(want) > want.size / 2
+
+
+def test_outputs_are_overwritten_and_null_is_refused():
+    """Every route writes its output whole, whatever it held (the sums do not
+    add to it), and refuses a missing one."""
+    scanner, proj, vol = (ScannerSpec.ring(13, 96, 130.0, 4.0), ProjSpec(13, 96, 25, 25),
+                          VolSpec.centred((40, 40, 30), (4.0, 4.0, 2.0)))
+    assert capi.track_plan(scanner, proj, vol).on_tracks
+    nb = capi.proj_geometry(proj)["n_bins"]
+    rng = np.random.default_rng(2)
+    y = rng.poisson(1.0, nb).astype(np.float32)
+    x = rng.random(vol.shape_zyx, dtype=np.float32) + np.float32(0.1)
+    track, single = contexts(scanner)
+    ordered = capi.Context(scanner)
+    ordered.set_option(capi.FIR_OPT_BACKPROJ_MODE, capi.FIR_BACKPROJ_DETERMINISTIC)
+    floats = capi.Context(scanner)
+    floats.set_option(capi.FIR_OPT_TRAVERSAL, capi.FIR_TRAVERSAL_FLOAT)
+    import torch
+
+    for c in (track, single, ordered, floats):
+        for n_subsets in (1, 4):
+            out = []
+            for fill in (0.0, 1e6):
+                b = torch.full((n_subsets,) + vol.shape_zyx, fill, device="cuda")
+                s = torch.full_like(b, fill)
+                r = torch.full(vol.shape_zyx, fill, device="cuda")
+                dy, dx = torch.from_numpy(y).cuda(), torch.from_numpy(x).cuda()
+                c.backward(proj, dy, vol, b, n_subsets)
+                c.sensitivity(proj, vol, s, n_subsets)
+                c.ratio_backprojection(proj, dy, vol, dx, r, n_subsets=n_subsets, subset=n_subsets - 1)
+                c.synchronize()
+                out.append([t.double() for t in (b, s, r)])
+            for a, b in zip(*out):
+                assert float((a - b).norm()) <= 1e-6 * float(a.norm())
+    L, pd, vd = capi.lib(), capi.C.byref(capi.proj_desc(proj)), capi.C.byref(capi.vol_desc(vol, 1))
+    refused = 1  # FIR_ERR_INVALID_ARGUMENT
+    assert L.fir_sensitivity(track.handle, pd, vd, None, 1) == refused
+    assert L.fir_backward(track.handle, pd, capi._ptr(y), vd, None, 1) == refused
