@@ -506,12 +506,64 @@ Widened widen_for_projection(fir_ctx& c, const Grid& g, const float* img)
 }
 
 // The plan of a launch on transaxial tracks (column.cu), or tracks = 0 where
-// the LORs are traced one by one.
-ColumnPlan columns_for(fir_ctx& c, const Grid& g, const Sino& s, bool skip)
+// LOR by LOR is faster.
+ColumnPlan columns_for(const fir_ctx& c, const Grid& g, const Sino& s, bool skip)
 {
   ColumnPlan p = column_plan(g, s, c.scan_z.data(), c.block, skip);
   if (column_warps(p) < kColumnWarps || !columns_pay(g, s, p, c.scan_z.data(), c.scan_diameter))
   {
+    p.tracks = 0;
+  }
+  return p;
+}
+
+// Whether b holds n bytes, or can be made to: not while the stream is being
+// captured (an allocation would end the capture), nor where the device has no
+// room for them.
+bool can_hold(const fir_ctx& c, DevBuf& b, size_t n)
+{
+  if (b.bytes >= n)
+  {
+    return true;
+  }
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c.stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone)
+  {
+    cudaGetLastError();
+    return false;
+  }
+  try
+  {
+    b.ensure(n);
+    return true;
+  }
+  catch (const Failure&)
+  {
+    cudaGetLastError();
+    return false;
+  }
+}
+
+// The same plan for a launch of this context, which also needs scratch: the
+// image's double copy (image) and the accumulators (acc) in z columns.  Calls
+// that the LOR-by-LOR kernels can serve without it must not fail for the lack
+// of it, so without room for it the plan has tracks = 0.
+ColumnPlan columns_here(fir_ctx& c, const Grid& g, const Sino& s, bool skip, bool image, bool acc)
+{
+  ColumnPlan p = columns_for(c, g, s, skip);
+  const size_t n = (size_t)g.nxy * g.nz;
+  if (p.tracks == 0)
+  {
+    return p;
+  }
+  const size_t had = c.wide.bytes;
+  if ((image && !can_hold(c, c.wide, n * sizeof(double))) ||
+      (acc && !can_hold(c, c.column_acc, 2 * n * sizeof(float))))
+  {
+    if (c.wide.bytes > had)
+    {
+      c.wide.release();  // the other kernels may need the room
+    }
     p.tracks = 0;
   }
   return p;
@@ -529,7 +581,7 @@ const double* to_columns(fir_ctx& c, const Grid& g, const float* img, float* acc
 
 float* column_accumulators(fir_ctx& c, const Grid& g)
 {
-  return static_cast<float*>(c.bp_t.ensure(2 * (size_t)g.nxy * g.nz * sizeof(float)));
+  return static_cast<float*>(c.column_acc.ensure(2 * (size_t)g.nxy * g.nz * sizeof(float)));
 }
 
 // s with the compacted list of its bins whose measured value is not 0
@@ -555,7 +607,7 @@ Sino nonzero_bins(fir_ctx& c, const Sino& s, const float* sino)
 void project_image(fir_ctx& c, const Grid& g, const Sino& s, const Tables& t, const float* img, float* sino,
                    FwdEpilogue ep)
 {
-  const ColumnPlan plan = columns_for(c, g, s, false);
+  const ColumnPlan plan = columns_here(c, g, s, false, true, false);
   if (plan.tracks > 0)
   {
     const double* wide = to_columns(c, g, img, nullptr);
@@ -610,7 +662,7 @@ void backproject_subsets(fir_ctx& c, const ProjInfo& p, const VolInfo& v, const 
   ColumnPlan plan{};
   if (c.backproj == FIR_BACKPROJ_ATOMIC)
   {
-    plan = columns_for(c, g, sino_of(p, n_subsets, 0), skip);
+    plan = columns_here(c, g, sino_of(p, n_subsets, 0), skip, false, true);
   }
   for (int k = 0; k < n_subsets; ++k)
   {
@@ -634,7 +686,7 @@ ColumnPlan osem_columns(fir_ctx& c, const Grid& g, const Sino& s)
   {
     return ColumnPlan{};
   }
-  return columns_for(c, g, s, c.skip_zero != 0);
+  return columns_here(c, g, s, c.skip_zero != 0, true, true);
 }
 
 // The backprojection of ratio_backproject in z columns (context scratch).
@@ -1158,7 +1210,14 @@ void osem_subiteration_device(fir_ctx& c, const ProjInfo& p, const Tables& t, co
   }
   // a small volume is filtered in one launch, from the EM step's scratch image
   const bool fused = f.wanted && conv_fused_fits(g.nx, g.ny, g.nz, f.x, f.y, f.z);
-  float* out = fused ? static_cast<float*>(c.conv1.ensure((size_t)v.nvox * sizeof(float))) : img;
+  float* out = img;
+  if (fused)
+  {
+    out = static_cast<float*>(c.conv1.ensure((size_t)v.nvox * sizeof(float)));
+    // (a captured fir_convolve after this call finds its scratch, as after one
+    // that filters in passes)
+    c.conv2.ensure((size_t)v.nvox * sizeof(float));
+  }
   if (plan.tracks > 0)
   {
     const float* acc = column_ratio_backproject(c, g, s, t, plan, img, sino, mult, bias);
@@ -1575,7 +1634,7 @@ fir_status fir_ctx_destroy(fir_ctx* c)
     cudaStreamSynchronize(c->stream);
     for (DevBuf* b : {&c->xy, &c->z, &c->check, &c->bp, &c->conv1, &c->conv2, &c->mu, &c->wide,
                       &c->det, &c->det_pairs, &c->ratio, &c->frames_il, &c->frames_acc, &c->psf_blur, &c->psf_sens, &c->rebin,
-                      &c->wide_t, &c->bp_t, &c->img_t, &c->frames_il_t, &c->frames_acc_t, &c->compact})
+                      &c->wide_t, &c->bp_t, &c->column_acc, &c->img_t, &c->frames_il_t, &c->frames_acc_t, &c->compact})
     {
       b->release();
     }

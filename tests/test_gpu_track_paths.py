@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 
 from fir_b200 import capi
-from fir_b200.geometry import ProjSpec, ScannerSpec, VolSpec
+from fir_b200.geometry import OSEMParams, ProjSpec, ScannerSpec, VolSpec
 from test_track_plan import MANY_RINGS
 
 pytestmark = pytest.mark.gpu
@@ -80,3 +80,76 @@ def test_outputs_are_overwritten_and_null_is_refused():
     refused = 1  # FIR_ERR_INVALID_ARGUMENT
     assert L.fir_sensitivity(track.handle, pd, vd, None, 1) == refused
     assert L.fir_backward(track.handle, pd, capi._ptr(y), vd, None, 1) == refused
+
+
+def test_first_backprojection_may_be_captured_above_l2():
+    """Above L2 the LOR-by-LOR backprojection needs no scratch, so a context's
+    first call can be captured; tracks need scratch and step back."""
+    import torch
+
+    scanner, proj = ScannerSpec.ring(16, 256, 300.0, 4.0), ProjSpec(16, 256, 31, 99)
+    l2 = torch.cuda.get_device_properties(0).L2_cache_size
+    nz = int(l2 / 8 / (280 * 280)) + 2
+    vol = VolSpec.centred((280, 280, nz), (2.0, 2.0, 2.0))
+    assert capi.track_plan(scanner, proj, vol).on_tracks
+    nb = capi.proj_geometry(proj)["n_bins"]
+    y = torch.rand(nb, device="cuda")
+    out = torch.zeros(vol.shape_zyx, device="cuda")
+    eager, first = capi.Context(scanner), capi.Context(scanner)
+    eager.backward(proj, y, vol, out)
+    eager.synchronize()
+    assert eager.track_launch_count == 1
+    want = out.double()
+    out.zero_()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        first.backward(proj, y, vol, out)
+    assert first.track_launch_count == 0
+    graph.replay()
+    torch.cuda.synchronize()
+    assert float((out.double() - want).norm()) <= 1e-6 * float(want.norm())
+    # with its scratch the context's next calls run on tracks, captured ones too
+    first.backward(proj, y, vol, out)
+    assert first.track_launch_count == 1
+    again = torch.cuda.CUDAGraph()
+    out.zero_()
+    with torch.cuda.graph(again):
+        first.backward(proj, y, vol, out)
+    assert first.track_launch_count == 2
+    again.replay()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert float((out.double() - want).norm()) <= 1e-6 * float(want.norm())
+
+
+def test_captured_launch_keeps_its_scratch():
+    """A later call on tracks leaves the scratch of a captured LOR-by-LOR
+    sub-iteration in place."""
+    import torch
+
+    scanner, proj, vol = (ScannerSpec.ring(13, 96, 130.0, 4.0), ProjSpec(13, 96, 25, 25),
+                          VolSpec.centred((40, 40, 30), (4.0, 4.0, 2.0)))
+    assert capi.track_plan(scanner, proj, vol).on_tracks
+    assert not capi.track_plan(scanner, proj, vol, n_subsets=4).on_tracks
+    nb = capi.proj_geometry(proj)["n_bins"]
+    rng = np.random.default_rng(3)
+    y = torch.from_numpy(rng.poisson(2.0, nb).astype(np.float32)).cuda()
+    x0 = torch.from_numpy(rng.random(vol.shape_zyx, dtype=np.float32) + np.float32(0.1)).cuda()
+    sens = torch.ones(vol.shape_zyx, device="cuda")
+    prm = OSEMParams(n_subsets=4)
+    ctx = capi.Context(scanner)
+    x = x0.clone()
+    ctx.osem_subiteration(proj, y, vol, x, sens, prm, 1, 1)
+    want = x.double()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ctx.osem_subiteration(proj, y, vol, x, sens, prm, 1, 1)
+    assert ctx.track_launch_count == 0
+    full = torch.empty(vol.shape_zyx, device="cuda")
+    ctx.sensitivity(proj, vol, full)
+    ctx.synchronize()
+    assert ctx.track_launch_count == 1
+    x.copy_(x0)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert float((x.double() - want).norm()) <= 1e-6 * float(want.norm())
