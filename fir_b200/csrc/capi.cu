@@ -544,6 +544,24 @@ bool can_hold(const fir_ctx& c, DevBuf& b, size_t n)
   }
 }
 
+// The queue of a launch on tracks, in context scratch; none without skipped
+// bins.
+size_t queue_bytes(const Sino& s) { return ((size_t)queue_room(s) + 1) * sizeof(int); }
+
+LorQueue queue_for(fir_ctx& c, const Sino& s, const ColumnPlan& p, const float* sino)
+{
+  if (p.skip == 0)
+  {
+    return LorQueue{};
+  }
+  int* base = static_cast<int*>(c.compact.ensure(queue_bytes(s)));
+  const LorQueue q{base + 1, base, queue_room(s)};
+  cuda_ok(cudaMemsetAsync(base, 0, sizeof(int), c.stream), "cudaMemsetAsync");
+  launch_list_nonzero(s, p, sino, q, cfg_of(c));
+  after_launch(c);
+  return q;
+}
+
 // The same plan for a launch of this context, which also needs scratch: the
 // image's double copy (image) and the accumulators (acc) in z columns.  Calls
 // that the LOR-by-LOR kernels can serve without it must not fail for the lack
@@ -552,13 +570,14 @@ ColumnPlan columns_here(fir_ctx& c, const Grid& g, const Sino& s, bool skip, boo
 {
   ColumnPlan p = columns_for(c, g, s, skip);
   const size_t n = (size_t)g.nxy * g.nz;
+  const size_t queue = queue_bytes(s);
   if (p.tracks == 0)
   {
     return p;
   }
   const size_t had = c.wide.bytes;
   if ((image && !can_hold(c, c.wide, n * sizeof(double))) ||
-      (acc && !can_hold(c, c.column_acc, 2 * n * sizeof(float))))
+      (acc && !can_hold(c, c.column_acc, 2 * n * sizeof(float))) || (skip && !can_hold(c, c.compact, queue)))
   {
     if (c.wide.bytes > had)
     {
@@ -631,7 +650,15 @@ void backproject_subset(fir_ctx& c, const Grid& g, const Sino& s, const Tables& 
   {
     float* acc = column_accumulators(c, g);
     cuda_ok(cudaMemsetAsync(acc, 0, 2 * (size_t)n * sizeof(float), c.stream), "cudaMemsetAsync");
-    timed_launch(c, [&] { launch_column_backward(g, s, t, plan, sino, acc, cfg_of(c)); });
+    const LorQueue queue = queue_for(c, s, plan, sino);
+    timed_launch(c, [&] {
+      launch_column_backward(g, s, t, plan, sino, acc, queue, cfg_of(c));
+      if (queue.list != nullptr)
+      {
+        launch_queue_backward(g, s, t, sino, acc, queue, cfg_of(c));
+      }
+    });
+    c.launches += queue.list != nullptr ? 1 : 0;
     ++c.track_launches;
     launch_from_columns(g, acc, img, cfg_of(c));
     after_launch(c);
@@ -696,7 +723,15 @@ const float* column_ratio_backproject(fir_ctx& c, const Grid& g, const Sino& s, 
 {
   float* acc = column_accumulators(c, g);
   const double* wide = to_columns(c, g, img, acc);
-  timed_launch(c, [&] { launch_column_osem(g, s, t, p, wide, sino, mult, bias, acc, cfg_of(c)); });
+  const LorQueue queue = queue_for(c, s, p, sino);
+  timed_launch(c, [&] {
+    launch_column_osem(g, s, t, p, wide, sino, mult, bias, acc, queue, cfg_of(c));
+    if (queue.list != nullptr)
+    {
+      launch_queue_osem(g, s, t, wide, sino, mult, bias, acc, queue, cfg_of(c));
+    }
+  });
+  c.launches += queue.list != nullptr ? 1 : 0;
   ++c.track_launches;
   return acc;
 }

@@ -216,7 +216,8 @@ long long direct_project(fir_batch& b, int k, int subset, cudaStream_t s)
   const LaunchCfg cfg{b.ctx->block, s, static_cast<int*>(b.ctx->check.p)};
   if (b.pr[(size_t)k].columns)
   {
-    launch_column_osem(d.g, sub, d.t, b.pr[(size_t)k].plan, d.wide, d.sino, nullptr, d.bias, d.bp, cfg);
+    launch_column_osem(d.g, sub, d.t, b.pr[(size_t)k].plan, d.wide, d.sino, nullptr, d.bias, d.bp,
+                       LorQueue{}, cfg);
     check_launch(s);
     return 1;
   }

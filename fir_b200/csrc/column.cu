@@ -106,47 +106,6 @@ __device__ __forceinline__ ColumnLor column_lor(const Sino& s, const Tables& t, 
   return l;
 }
 
-// Lists of the ring pairs whose bin is not 0, in shared memory: every warp
-// lists those of an equal part of its group's share, and counts them.
-struct NonzeroLists
-{
-  int* counts;           // of each warp
-  unsigned short* pairs; // share entries per group
-};
-
-__host__ __device__ constexpr int warp_part(int share, int warps) { return ((share + warps - 1) / warps + 31) / 32 * 32; }
-
-__device__ __forceinline__ void list_nonzero(const Sino& s, const ColumnPlan& p, const ColumnShare& c, int subset,
-                                             const float* __restrict__ sino, const NonzeroLists& l)
-{
-  const int lane = threadIdx.x & 31;
-  const int part = warp_part(p.share, p.warps);
-  unsigned short* list = l.pairs + (c.group * p.warps + c.warp) * part;
-  const int begin = c.begin + c.warp * part, end = min(begin + part, c.end);
-  int n = 0;
-  for (int r0 = begin; r0 < end; r0 += 32)
-  {
-    const int r = r0 + lane;
-    bool on = false;
-    if (r < end)
-    {
-      int seg, axial;
-      ring_pair(s, p, r, seg, axial);
-      on = __ldg(sino + column_bin(s, c, subset, seg, axial)) != 0.0f;
-    }
-    const unsigned mask = __ballot_sync(0xffffffffu, on);
-    if (on)
-    {
-      list[n + __popc(mask & ((1u << lane) - 1))] = (unsigned short)(r - c.begin);
-    }
-    n += __popc(mask);
-  }
-  if (lane == 0)
-  {
-    l.counts[threadIdx.x >> 5] = n;
-  }
-}
-
 // The LORs of a block that cannot use their track, in shared memory: they are
 // traced at the end, 32 to a warp, where a few of each warp's lanes would
 // hold up the others for a whole walk.
@@ -162,70 +121,32 @@ __device__ __forceinline__ Leftover leftover(unsigned char* smem, const ColumnPl
   return Leftover{count, reinterpret_cast<unsigned*>(count + 4)};
 }
 
-// Calls trace(lor) for the warp's LORs, 64 at a time, two per lane: those of
-// its group's share in turn, or with kSkip those of them whose bin is not 0
-// (with a bin of 0 the ratio, or the value, is exactly 0, and so is every
-// contribution).  Every thread of the block calls this.
-template<bool kSkip, class Trace>
-__device__ __forceinline__ void column_each(const Sino& s, const Tables& t, const ColumnPlan& p,
-                                            const ColumnShare& c, int subset, const float* __restrict__ sino,
-                                            const NonzeroLists& lists, Trace&& trace)
+// The lane's two LORs of the warp's 64.
+__device__ __forceinline__ void column_lors(const Sino& s, const Tables& t, const ColumnPlan& p,
+                                            const ColumnShare& c, int subset, ColumnLor lor[2])
 {
-  const int lane = threadIdx.x & 31;
-  int n = c.end - c.begin;
-  if (kSkip)
-  {
-    list_nonzero(s, p, c, subset, sino, lists);
-    __syncthreads();
-    n = 0;
-    for (int w = 0; w < p.warps && c.end > c.begin; ++w)
-    {
-      n += lists.counts[c.group * p.warps + w];
-    }
-  }
-  if constexpr (!kSkip)
-  {
-    ColumnLor lor[2];
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
-    {
-      const int i = c.warp * 64 + 32 * k + lane;
-      lor[k] = column_lor(s, t, p, c, subset, i < n, c.begin + i);
-    }
-    trace(lor);
-  }
-  else
+  for (int k = 0; k < 2; ++k)
   {
-    for (int i0 = c.warp * 64; i0 < n; i0 += p.warps * 64)
-    {
-      ColumnLor lor[2];
-  #pragma unroll
-      for (int k = 0; k < 2; ++k)
-      {
-        int i = i0 + 32 * k + lane;
-        const bool valid = i < n;
-        if (valid)
-        {
-          int w = c.group * p.warps;
-          while (i >= lists.counts[w])
-          {
-            i -= lists.counts[w++];
-          }
-          i = lists.pairs[w * warp_part(p.share, p.warps) + i];
-        }
-        lor[k] = column_lor(s, t, p, c, subset, valid, c.begin + i);
-      }
-      trace(lor);
-    }
+    const int r = c.begin + c.warp * 64 + 32 * k + (int)(threadIdx.x & 31);
+    lor[k] = column_lor(s, t, p, c, subset, r < c.end, r);
   }
 }
 
-__device__ __forceinline__ NonzeroLists nonzero_lists(unsigned char* smem, const ColumnPlan& p)
-{
-  const Leftover l = leftover(smem, p);
-  int* counts = reinterpret_cast<int*>(l.lors + p.per_block * p.share);
-  return NonzeroLists{counts, reinterpret_cast<unsigned short*>(counts + 8)};
-}
+// Where bins that are 0 are skipped and less than this share of them is left,
+// the launch leaves those to the queue, one LOR per thread of its own kernel: a
+// block would build its tracks for a few LORs, most of its warps' lanes idle.
+// Otherwise all LORs go along their tracks as without skipping, those of zero
+// bins idle.  (Decided block by block, the two kernels of a launch are each too
+// short to fill the GPU: 58 % of a span-3 subset, 281 us against 245 and 239.)
+// Sub-iterations of Poisson data, tracks against queue: clinical scanner
+// 1.21 ms against 0.44 at 10 % non-zero, 0.69 at 25 %, 1.32 at 61 %; 17 rings
+// 365 us against 158 at 9 %, 246 at 25 %, 415 at 55 %; 24 rings 770 us against
+// 479 at 25 %, 862 at 59 %.
+constexpr int kQueuePercent = 50;
+
+// Whether the launch that skips zero bins leaves the others to the queue.
+__device__ __forceinline__ bool queued(const LorQueue& q) { return q.list != nullptr && __ldg(q.count) < q.room; }
 
 // The general walk in z columns, for the LORs that cannot use their track.
 // Not inlined: few lanes take it, and its registers are not the kernel's.
@@ -269,16 +190,18 @@ __device__ __noinline__ void general_scatter(const Grid& g, const TrackHead& h, 
   }
 }
 
-// Sets up a lane's two LORs; go says which of them use the track.  Those that
-// need the general walk are left over.
+// Sets up a lane's two LORs, those that are on; go says which of them use the
+// track.  Those that need the general walk are left over.
 __device__ __forceinline__ void column_setup(const Grid& g, const ColumnPlan& p, const Track& tr,
-                                             const ColumnShare& c, const ColumnLor lor[2], const Leftover& left, ColumnLane w[2],
-                                             bool go[2])
+                                             const ColumnShare& c, const ColumnLor lor[2], const bool on[2],
+                                             const Leftover& left, ColumnLane w[2], bool go[2])
 {
 #pragma unroll
   for (int k = 0; k < 2; ++k)
   {
-    const int kind = lor[k].valid && tr.head->crosses ? lane_setup(g, *tr.head, lor[k].z1, lor[k].z2, w[k]) : kLorNone;
+    const int kind = on[k] && lor[k].valid && tr.head->crosses
+                       ? lane_setup(g, *tr.head, lor[k].z1, lor[k].z2, w[k])
+                       : kLorNone;
     go[k] = kind == kLorColumn;
     if (kind == kLorGeneral)
     {
@@ -364,23 +287,24 @@ __global__ void __launch_bounds__(256, 5) k_column_forward(const __grid_constant
   build_tracks(g, s, t, p, s.subset, first, smem, left.count);
   const ColumnShare c = column_share(s, p, (int)blockIdx.x, first);
   const Track tr = track_at(smem, p.cap, c.group);
-  column_each<false>(s, t, p, c, s.subset, nullptr, NonzeroLists{}, [&](const ColumnLor* lor) {
-    ColumnLane w[2] = {};
-    bool go[2];
-    float line[2];
-    column_setup(g, p, tr, c, lor, left, w, go);
-    column_lines(tr, go, w, img, line);
+  ColumnLor lor[2];
+  column_lors(s, t, p, c, s.subset, lor);
+  ColumnLane w[2] = {};
+  bool go[2];
+  float line[2];
+  const bool on[2] = {true, true};
+  column_setup(g, p, tr, c, lor, on, left, w, go);
+  column_lines(tr, go, w, img, line);
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
+  for (int k = 0; k < 2; ++k)
+  {
+    if (lor[k].valid)
     {
-      if (lor[k].valid)
-      {
-        sino[lor[k].bin] = epilogue<EP>(line[k]);
-      }
+      sino[lor[k].bin] = epilogue<EP>(line[k]);
     }
-  });
-  column_leftover(s, t, p, s.subset, (int)blockIdx.x, first, smem, left, [&](const ColumnLor& lor, const Track& own) {
-    sino[lor.bin] = epilogue<EP>(general_line(g, *own.head, lor.z1, lor.z2, img, check).line);
+  }
+  column_leftover(s, t, p, s.subset, (int)blockIdx.x, first, smem, left, [&](const ColumnLor& l, const Track& own) {
+    sino[l.bin] = epilogue<EP>(general_line(g, *own.head, l.z1, l.z2, img, check).line);
   });
 }
 
@@ -396,29 +320,36 @@ __device__ __forceinline__ float* accumulator_of(const Grid& g, const TrackHead&
 template<bool kSkip>
 __global__ void __launch_bounds__(256, 4) k_column_backward(const __grid_constant__ Grid g,
                                                             const __grid_constant__ Sino s, Tables t, ColumnPlan p,
-                                                            const float* __restrict__ sino, float* acc, int* check)
+                                                            const float* __restrict__ sino, float* acc,
+                                                            LorQueue queue, int* check)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   const int first = first_track(p, (int)blockIdx.x);
+  const ColumnShare c = column_share(s, p, (int)blockIdx.x, first);
+  if (kSkip && queued(queue))
+  {
+    return;
+  }
   const Leftover left = leftover(smem, p);
   build_tracks(g, s, t, p, s.subset, first, smem, left.count);
-  const ColumnShare c = column_share(s, p, (int)blockIdx.x, first);
   const Track tr = track_at(smem, p.cap, c.group);
-  column_each<kSkip>(s, t, p, c, s.subset, sino, nonzero_lists(smem, p), [&](const ColumnLor* lor) {
-    ColumnLane w[2] = {};
-    bool go[2];
-    double value[2];
-    column_setup(g, p, tr, c, lor, left, w, go);
+  ColumnLor lor[2];
+  column_lors(s, t, p, c, s.subset, lor);
+  ColumnLane w[2] = {};
+  bool go[2];
+  double value[2];
+  bool on[2] = {true, true};
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
-    {
-      value[k] = lor[k].valid && sino != nullptr ? (double)__ldg(sino + lor[k].bin) : 1.0;
-    }
-    column_scatter(tr, go, w, value, accumulator_of(g, *tr.head, acc));
-  });
-  column_leftover(s, t, p, s.subset, (int)blockIdx.x, first, smem, left, [&](const ColumnLor& lor, const Track& own) {
-    const double v = sino != nullptr ? (double)__ldg(sino + lor.bin) : 1.0;
-    general_scatter(g, *own.head, lor.z1, lor.z2, v, accumulator_of(g, *own.head, acc), check);
+  for (int k = 0; k < 2; ++k)
+  {
+    value[k] = lor[k].valid && sino != nullptr ? (double)__ldg(sino + lor[k].bin) : 1.0;
+    on[k] = !kSkip || value[k] != 0.0;
+  }
+  column_setup(g, p, tr, c, lor, on, left, w, go);
+  column_scatter(tr, go, w, value, accumulator_of(g, *tr.head, acc));
+  column_leftover(s, t, p, s.subset, (int)blockIdx.x, first, smem, left, [&](const ColumnLor& l, const Track& own) {
+    const double v = sino != nullptr ? (double)__ldg(sino + l.bin) : 1.0;
+    general_scatter(g, *own.head, l.z1, l.z2, v, accumulator_of(g, *own.head, acc), check);
   });
 }
 
@@ -454,34 +385,44 @@ template<bool kWeighted, bool kSkip>
 __device__ __forceinline__ void column_osem(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p,
                                             int subset, int block, const double* __restrict__ img,
                                             const float* __restrict__ sino, const float* __restrict__ mult,
-                                            const float* __restrict__ bias, float* acc, int* check,
-                                            unsigned char* smem)
+                                            const float* __restrict__ bias, float* acc, const LorQueue& queue,
+                                            int* check, unsigned char* smem)
 {
   const int first = first_track(p, block);
+  const ColumnShare c = column_share(s, p, block, first);
+  if (kSkip && queued(queue))
+  {
+    return;
+  }
   const Leftover left = leftover(smem, p);
   build_tracks(g, s, t, p, subset, first, smem, left.count);
-  const ColumnShare c = column_share(s, p, block, first);
   const Track tr = track_at(smem, p.cap, c.group);
-  column_each<kSkip>(s, t, p, c, subset, sino, nonzero_lists(smem, p), [&](const ColumnLor* lor) {
-    ColumnLane w[2] = {};
-    bool go[2];
-    float line[2];
-    column_setup(g, p, tr, c, lor, left, w, go);
-    column_lines(tr, go, w, img, line);
-    double value[2] = {0.0, 0.0};
+  ColumnLor lor[2];
+  column_lors(s, t, p, c, subset, lor);
+  ColumnLane w[2] = {};
+  bool go[2];
+  float line[2];
+  bool on[2] = {true, true};
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
-    {
-      go[k] = go[k] && osem_ratio<kWeighted>(line[k], lor[k].bin, sino, mult, bias, value[k]);
-    }
-    column_scatter(tr, go, w, value, accumulator_of(g, *tr.head, acc));
-  });
-  column_leftover(s, t, p, subset, block, first, smem, left, [&](const ColumnLor& lor, const Track& own) {
-    const GeneralLine gl = general_line(g, *own.head, lor.z1, lor.z2, img, check);
+  for (int k = 0; k < 2; ++k)
+  {
+    on[k] = !kSkip || (lor[k].valid && __ldg(sino + lor[k].bin) != 0.0f);
+  }
+  column_setup(g, p, tr, c, lor, on, left, w, go);
+  column_lines(tr, go, w, img, line);
+  double value[2] = {0.0, 0.0};
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+  {
+    go[k] = go[k] && osem_ratio<kWeighted>(line[k], lor[k].bin, sino, mult, bias, value[k]);
+  }
+  column_scatter(tr, go, w, value, accumulator_of(g, *tr.head, acc));
+  column_leftover(s, t, p, subset, block, first, smem, left, [&](const ColumnLor& l, const Track& own) {
+    const GeneralLine gl = general_line(g, *own.head, l.z1, l.z2, img, check);
     double q;
-    if (osem_ratio<kWeighted>(gl.line, lor.bin, sino, mult, bias, q) && gl.ok)
+    if (osem_ratio<kWeighted>(gl.line, l.bin, sino, mult, bias, q) && gl.ok)
     {
-      general_scatter(g, *own.head, lor.z1, lor.z2, q, accumulator_of(g, *own.head, acc), check);
+      general_scatter(g, *own.head, l.z1, l.z2, q, accumulator_of(g, *own.head, acc), check);
     }
   });
 }
@@ -492,10 +433,133 @@ __global__ void __launch_bounds__(256, 5) k_column_osem(const __grid_constant__ 
                                                         const double* __restrict__ img,
                                                         const float* __restrict__ sino,
                                                         const float* __restrict__ mult,
-                                                        const float* __restrict__ bias, float* acc, int* check)
+                                                        const float* __restrict__ bias, float* acc,
+                                                        LorQueue queue, int* check)
 {
   extern __shared__ __align__(16) unsigned char smem[];
-  column_osem<kWeighted, kSkip>(g, s, t, p, s.subset, (int)blockIdx.x, img, sino, mult, bias, acc, check, smem);
+  column_osem<kWeighted, kSkip>(g, s, t, p, s.subset, (int)blockIdx.x, img, sino, mult, bias, acc, queue, check, smem);
+}
+
+// The queue: the enumerated indices of the subset's non-zero bins, as far as
+// there is room, and their number.  A block takes a tile of 32 ring pairs x 32
+// tangential bins: its warps read along the latter, eight pairs each, and it
+// appends track by track, since the LORs of a track run through the same columns.
+constexpr int kListPairs = 8, kListWarps = 4;
+
+__global__ void __launch_bounds__(32 * kListWarps) k_list_nonzero(const __grid_constant__ Sino s, ColumnPlan p,
+                                                                  const float* __restrict__ sino, LorQueue q)
+{
+  constexpr unsigned kAll = 0xffffffffu;
+  __shared__ int counts[kListWarps][32];
+  __shared__ int place;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int across = (s.n_tang + 31) / 32;
+  const int tiles = across * ((p.pairs + kListWarps * kListPairs - 1) / (kListWarps * kListPairs));
+  const int sv = (int)blockIdx.x / tiles, tile = (int)blockIdx.x - sv * tiles;
+  const int tang = tile % across * 32 + lane;
+  const int first = (tile / across * kListWarps + warp) * kListPairs;
+  int seg, axial;
+  ring_pair(s, p, min(first + (lane & (kListPairs - 1)), p.pairs - 1), seg, axial);
+  const int bin = s.seg_base[seg] + ((sv * s.n_subsets + s.subset) * s.n_axial[seg] + axial) * s.n_tang;
+  const int key = s.enum_base[seg] + (sv * s.n_axial[seg] + axial) * s.n_tang;
+  float y[kListPairs];
+#pragma unroll
+  for (int k = 0; k < kListPairs; ++k)
+  {
+    const int row = __shfl_sync(kAll, bin, k);
+    y[k] = tang < s.n_tang && first + k < p.pairs ? __ldg(sino + row + tang) : 0.0f;
+  }
+  int n = 0;
+#pragma unroll
+  for (int k = 0; k < kListPairs; ++k)
+  {
+    n += y[k] != 0.0f ? 1 : 0;
+  }
+  counts[warp][lane] = n;
+  __syncthreads();
+  int own = 0, before = 0;  // entries of the lane's track, and of the warps before this one
+#pragma unroll
+  for (int w = 0; w < kListWarps; ++w)
+  {
+    own += counts[w][lane];
+    before += w < warp ? counts[w][lane] : 0;
+  }
+  int end = own;
+#pragma unroll
+  for (int d = 1; d < 32; d *= 2)
+  {
+    const int below = __shfl_up_sync(kAll, end, d);
+    end += lane >= d ? below : 0;
+  }
+  if (threadIdx.x == 31)
+  {
+    place = end > 0 ? atomicAdd(q.count, end) : 0;
+  }
+  __syncthreads();
+  int at = place + end - own + before;
+#pragma unroll
+  for (int k = 0; k < kListPairs; ++k)
+  {
+    const int index = __shfl_sync(kAll, key, k) + tang;
+    if (y[k] != 0.0f)
+    {
+      if (at < q.room)
+      {
+        q.list[at] = index;
+      }
+      ++at;
+    }
+  }
+}
+
+// The queued LORs (s.list), one per thread, on the same images.  The LORs of a
+// track lie side by side in the queue and run through the same columns.
+template<bool kWeighted>
+__global__ void __launch_bounds__(128, 8) k_queue_osem(const __grid_constant__ Grid g, const __grid_constant__ Sino s,
+                                                       Tables t, const double* __restrict__ img,
+                                                       const float* __restrict__ sino, const float* __restrict__ mult,
+                                                       const float* __restrict__ bias, float* acc, LorQueue queue,
+                                                       int* check)
+{
+  if (!queued(queue))
+  {
+    return;
+  }
+  osem_lor_body<kWeighted, double, true>(g, s, s.subset, t, img, img, sino, mult, bias, acc,
+                                         acc + (size_t)g.nxy * g.nz, true, blockIdx.x * blockDim.x + threadIdx.x,
+                                         check);
+}
+
+__global__ void __launch_bounds__(128, 8) k_queue_backward(const __grid_constant__ Grid g,
+                                                           const __grid_constant__ Sino s, Tables t,
+                                                           const float* __restrict__ sino, float* acc, LorQueue queue,
+                                                           int* check)
+{
+  if (!queued(queue))
+  {
+    return;
+  }
+  bool valid = false;
+  const int i = enum_index(s, blockIdx.x * blockDim.x + threadIdx.x, valid);
+  Walk w{};
+  bool go = false;
+  double value = 0.0;
+  float* to = acc;
+  if (valid)
+  {
+    const Lor l = decode_bin(s, i);
+    double e[6];
+    lor_ends(s, t, l, e);
+    go = siddon_setup<true>(g, e, w);
+    value = (double)__ldg(sino + l.bin);
+    to += fabs(dsub(e[3], e[0])) > fabs(dsub(e[4], e[1])) ? (size_t)g.nxy * g.nz : 0;
+  }
+  const bool ok = siddon_walk<true>(
+    g, w, go, [&](bool, int c, double len) { atomicAdd(to + c, __double2float_rn(dmul(len, value))); });
+  if (!ok)
+  {
+    flag(check, kCheckWalkGuard);
+  }
 }
 
 // The same for the items of a batch (batch.cu), whose work units are the
@@ -517,7 +581,7 @@ __global__ void __launch_bounds__(kBatchColumnBlock, 10)
   const BatchProblem& pb = P[__ldg(&items[lo].problem)];
   column_osem<false, kSkip>(pb.g, pb.s, pb.t, pb.plan, __ldg(&items[lo].subset),
                             (int)blockIdx.x - __ldg(&items[lo].unit_begin), pb.wide, pb.sino, nullptr, pb.bias, pb.bp,
-                            check, smem);
+                            LorQueue{}, check, smem);
 }
 
 // Images between [z][y][x] and z columns, through 32 x 32 tiles of
@@ -631,9 +695,7 @@ bool ask_shared(K kernel, size_t bytes)
 
 size_t column_smem(const ColumnPlan& p)
 {
-  const size_t lists = 8 * sizeof(int) + (size_t)(p.block / 32) * warp_part(p.share, p.warps) * sizeof(unsigned short);
-  return (size_t)p.per_block * (track_bytes(p.cap) + p.share * sizeof(unsigned)) + 4 * sizeof(int) +
-         (p.skip ? lists : 0);
+  return (size_t)p.per_block * (track_bytes(p.cap) + p.share * sizeof(unsigned)) + 4 * sizeof(int);
 }
 
 int column_blocks(const ColumnPlan& p) { return (p.tracks + p.per_block - 1) / p.per_block * p.blocks; }
@@ -652,10 +714,7 @@ ColumnPlan column_plan(const Grid& g, const Sino& s, const double* z, int block,
   // a ring
   const double apart = s.n_rings > 1 ? std::fabs(z[2] - z[0]) * (s.span > 1 ? 0.5 : 1.0) : 0.0;
   p.interleave = apart >= 1.6 * g.ext[2] ? 1 : 0;
-  // where bins are skipped a warp has room for two turns of 64: half of the
-  // bins are often 0, and warps without work would hold the block's registers
-  const int turn = skip ? 128 : 64;
-  const int warps = std::max((p.pairs + turn - 1) / turn, 1);
+  const int warps = std::max((p.pairs + 63) / 64, 1);
   // a track's warps in equal blocks of nearly the wanted size: the count
   // that leaves the fewest warps idle
   const int want = block / 32;
@@ -676,7 +735,7 @@ ColumnPlan column_plan(const Grid& g, const Sino& s, const double* z, int block,
   p.block = best * 32;
   p.blocks = std::max((warps + best - 1) / best, 1);
   p.warps = p.blocks > 1 ? best : warps;
-  p.share = p.blocks > 1 ? best * turn : std::max(p.pairs, 1);
+  p.share = p.blocks > 1 ? best * 64 : std::max(p.pairs, 1);
   p.per_block = best / p.warps;
   return p;
 }
@@ -785,7 +844,7 @@ void launch_column_forward(const Grid& g, const Sino& s, const Tables& t, const 
 }
 
 void launch_column_backward(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p, const float* sino,
-                            float* acc, const LaunchCfg& cfg)
+                            float* acc, const LorQueue& queue, const LaunchCfg& cfg)
 {
   if (p.tracks == 0)
   {
@@ -797,7 +856,41 @@ void launch_column_backward(const Grid& g, const Sino& s, const Tables& t, const
   {
     return;
   }
-  kernel<<<(unsigned)column_blocks(p), p.block, bytes, cfg.stream>>>(g, s, t, p, sino, acc, cfg.check);
+  kernel<<<(unsigned)column_blocks(p), p.block, bytes, cfg.stream>>>(g, s, t, p, sino, acc, queue, cfg.check);
+}
+
+int queue_room(const Sino& s) { return (int)((long long)s.n_enum * kQueuePercent / 100) + 1; }
+
+void launch_list_nonzero(const Sino& s, const ColumnPlan& p, const float* sino, const LorQueue& queue,
+                         const LaunchCfg& cfg)
+{
+  constexpr int deep = kListWarps * kListPairs;
+  const int tiles = (s.n_tang + 31) / 32 * ((p.pairs + deep - 1) / deep);
+  k_list_nonzero<<<(unsigned)(tiles * (p.tracks / s.n_tang)), 32 * kListWarps, 0, cfg.stream>>>(s, p, sino, queue);
+}
+
+// s with the queue as its enumeration.
+static Sino queue_of(const Sino& s, const LorQueue& queue)
+{
+  Sino q = s;
+  q.list = queue.list;
+  q.list_n = queue.count;
+  return q;
+}
+
+void launch_queue_backward(const Grid& g, const Sino& s, const Tables& t, const float* sino, float* acc,
+                           const LorQueue& queue, const LaunchCfg& cfg)
+{
+  k_queue_backward<<<(unsigned)(queue.room + 127) / 128, 128, 0, cfg.stream>>>(g, queue_of(s, queue), t, sino, acc,
+                                                                                 queue, cfg.check);
+}
+
+void launch_queue_osem(const Grid& g, const Sino& s, const Tables& t, const double* img, const float* sino,
+                       const float* mult, const float* bias, float* acc, const LorQueue& queue, const LaunchCfg& cfg)
+{
+  auto* kernel = mult != nullptr ? k_queue_osem<true> : k_queue_osem<false>;
+  kernel<<<(unsigned)(queue.room + 127) / 128, 128, 0, cfg.stream>>>(g, queue_of(s, queue), t, img, sino, mult, bias,
+                                                                       acc, queue, cfg.check);
 }
 
 void launch_batch_column_osem(const BatchProblem* P, const BatchItem* items, int n_items, int n_blocks, size_t bytes,
@@ -816,7 +909,8 @@ void launch_batch_column_osem(const BatchProblem* P, const BatchItem* items, int
 }
 
 void launch_column_osem(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p, const double* img,
-                        const float* sino, const float* mult, const float* bias, float* acc, const LaunchCfg& cfg)
+                        const float* sino, const float* mult, const float* bias, float* acc, const LorQueue& queue,
+                        const LaunchCfg& cfg)
 {
   if (p.tracks == 0)
   {
@@ -830,6 +924,7 @@ void launch_column_osem(const Grid& g, const Sino& s, const Tables& t, const Col
   {
     return;
   }
-  kernel<<<(unsigned)column_blocks(p), p.block, bytes, cfg.stream>>>(g, s, t, p, img, sino, mult, bias, acc, cfg.check);
+  kernel<<<(unsigned)column_blocks(p), p.block, bytes, cfg.stream>>>(g, s, t, p, img, sino, mult, bias, acc, queue,
+                                                                     cfg.check);
 }
 }  // namespace fir

@@ -87,6 +87,16 @@ void launch_osem_subset(const Grid& g, const Sino& s, const Tables& t, const dou
 void launch_osem_subset_float_image(const Grid& g, const Sino& s, const Tables& t, const float* img,
                                     const float* img_t, const float* sino, const float* mult, const float* bias,
                                     float* bp, float* bp_t, bool skip_zero, const LaunchCfg& cfg);
+// The non-zero bins that a launch on tracks with skipped bins leaves to the
+// general walk where they are fewer than room: the enumerated indices of the
+// first of them and the number of all.  list null: it leaves none.
+struct LorQueue
+{
+  int* list;
+  int* count;
+  int room;
+};
+int queue_room(const Sino& s);
 // column.cu: the projectors on transaxial tracks (column.cuh), which read the
 // image as doubles in z columns ([y][x][z]) and add into two accumulators of
 // that layout, one after the other at acc, whose sum is the backprojection.
@@ -115,9 +125,18 @@ void launch_em_update_columns(const Grid& g, const float* img, float* out, const
 void launch_column_forward(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p, const double* img,
                            float* sino, FwdEpilogue ep, const LaunchCfg& cfg);
 void launch_column_backward(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p, const float* sino,
-                            float* acc, const LaunchCfg& cfg);
+                            float* acc, const LorQueue& queue, const LaunchCfg& cfg);
 void launch_column_osem(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p, const double* img,
-                        const float* sino, const float* mult, const float* bias, float* acc, const LaunchCfg& cfg);
+                        const float* sino, const float* mult, const float* bias, float* acc, const LorQueue& queue,
+                        const LaunchCfg& cfg);
+// Fills the queue (its count is 0) with the non-zero bins of sino; traces its
+// LORs, where the launch on tracks leaves them to it.
+void launch_list_nonzero(const Sino& s, const ColumnPlan& p, const float* sino, const LorQueue& queue,
+                         const LaunchCfg& cfg);
+void launch_queue_backward(const Grid& g, const Sino& s, const Tables& t, const float* sino, float* acc,
+                           const LorQueue& queue, const LaunchCfg& cfg);
+void launch_queue_osem(const Grid& g, const Sino& s, const Tables& t, const double* img, const float* sino,
+                       const float* mult, const float* bias, float* acc, const LorQueue& queue, const LaunchCfg& cfg);
 // compact.cu: the enumerated indices of s (list null) whose bin of sino is
 // not 0, ascending, into list (s.n_enum entries), their number into *count
 // (device memory).  With temp null only *temp_bytes is set (CUB convention).

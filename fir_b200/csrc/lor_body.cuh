@@ -38,7 +38,10 @@ __device__ __forceinline__ void flag(int* check, int bit)
 // TImg: the image the projection gathers from, the double copy or the float
 // image itself (widened per step, exact; for volumes whose double copy does
 // not fit in L2 beside the accumulator).
-template<bool kWeighted, typename TImg = double>
+//
+// kColumns: the images are in z columns (column.cuh); img_t is img, and bp_t
+// the second of the two accumulators.
+template<bool kWeighted, typename TImg = double, bool kColumns = false>
 __device__ __forceinline__ void osem_lor_body(const Grid& g, const Sino& s, int subset, const Tables& t,
                                               const TImg* __restrict__ img, const TImg* __restrict__ img_t,
                                               const float* __restrict__ sino, const float* __restrict__ mult,
@@ -66,7 +69,7 @@ __device__ __forceinline__ void osem_lor_body(const Grid& g, const Sino& s, int 
       // orient 0 or 1: this launch takes only the LORs of that orientation
       if (orient < 0 || (tr ? 1 : 0) == orient)
       {
-        go = siddon_setup(g, e, w, tr);
+        go = siddon_setup<kColumns>(g, e, w, !kColumns && tr);
       }
     }
   }
@@ -81,7 +84,7 @@ __device__ __forceinline__ void osem_lor_body(const Grid& g, const Sino& s, int 
   // order; the first call adds 0 * 0 to the zero sum, which leaves it 0.
   float line = 0.0f;
   double pl = 0.0, pv = 0.0;
-  bool ok = siddon_walk(g, w, go, [&](bool inside, int c, double len) {
+  bool ok = siddon_walk<kColumns>(g, w, go, [&](bool inside, int c, double len) {
     if (inside)
     {
       line = accumulate(line, pl, pv);
@@ -107,7 +110,7 @@ __device__ __forceinline__ void osem_lor_body(const Grid& g, const Sino& s, int 
     q = __fmul_rn(q, m);
   }
   const double ratio = (double)q;
-  ok = siddon_walk(g, w, back, [&](bool inside, int c, double len) {
+  ok = siddon_walk<kColumns>(g, w, back, [&](bool inside, int c, double len) {
          if (inside)
          {
            atomicAdd(b + c, __double2float_rn(dmul(len, ratio)));

@@ -153,3 +153,41 @@ def test_captured_launch_keeps_its_scratch():
     graph.replay()
     torch.cuda.synchronize()
     assert float((x.double() - want).norm()) <= 1e-6 * float(want.norm())
+
+
+# Sums of floats in another order: 1e-6 as in the repository's other
+# comparisons of float atomics.
+@pytest.mark.parametrize("occupied", [0.0, 1e-4, 0.1, 0.49, 0.51, 1.0])
+@pytest.mark.parametrize("span", [1, 3])
+def test_skipped_bins_at_any_occupancy(occupied, span):
+    """Below half of the bins non-zero a launch on tracks leaves them to the
+    general walk, above it traces all; both equal the LOR-by-LOR route."""
+    if span == 1:
+        scanner, proj, vol = (ScannerSpec.ring(15, 96, 150.0, 5.0), ProjSpec(15, 96, 29, 27),
+                              VolSpec.centred((50, 46, 40), (3.0, 3.0, 2.0)))
+    else:
+        scanner, proj, vol = (ScannerSpec.ring(16, 128, 160.0, 4.0), ProjSpec(16, 128, 9, 31, 3),
+                              VolSpec.centred((47, 51, 17), (4.0, 4.0, 4.0)))
+    assert capi.track_plan(scanner, proj, vol, skip_zero=True).on_tracks
+    nb = capi.proj_geometry(proj)["n_bins"]
+    rng = np.random.default_rng(4)
+    y = rng.poisson(3.0, nb).astype(np.float32) + np.float32(1)
+    keep = int(round(occupied * nb))
+    y[rng.permutation(nb)[keep:]] = 0
+    m = rng.random(nb, dtype=np.float32) + np.float32(0.2)
+    x = rng.random(vol.shape_zyx, dtype=np.float32) + np.float32(0.1)
+    track, single = contexts(scanner)
+    track.set_option(capi.FIR_OPT_SKIP_ZERO_BINS, 1)
+    sens = np.ones((1,) + vol.shape_zyx, np.float32)
+    out = []
+    for c in (track, single):
+        back, ratio, osem = (np.zeros(vol.shape_zyx, np.float32) for _ in range(3))
+        c.backward(proj, y, vol, back)
+        c.ratio_backprojection(proj, y, vol, x, ratio)
+        osem[:] = x
+        c.osem(proj, y, vol, osem, sens, OSEMParams(n_iterations=1, n_subsets=1), mult=m)
+        out.append([a.astype(np.float64) for a in (back, ratio, osem)])
+    assert track.track_launch_count == 3 and single.track_launch_count == 0
+    for a, b in zip(*out):
+        assert np.linalg.norm(a - b) <= 1e-6 * np.linalg.norm(b)
+        assert np.array_equal(a > 0, b > 0)
