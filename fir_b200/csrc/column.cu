@@ -133,6 +133,9 @@ __device__ __forceinline__ void column_lors(const Sino& s, const Tables& t, cons
   }
 }
 
+// Ring pairs of a warp where a batch skips zero bins.
+constexpr int kPackedTurn = 128;
+
 // Where bins that are 0 are skipped and less than this share of them is left,
 // the launch leaves those to the queue, one LOR per thread of its own kernel: a
 // block would build its tracks for a few LORs, most of its warps' lanes idle.
@@ -144,6 +147,70 @@ __device__ __forceinline__ void column_lors(const Sino& s, const Tables& t, cons
 // 365 us against 158 at 9 %, 246 at 25 %, 415 at 55 %; 24 rings 770 us against
 // 479 at 25 %, 862 at 59 %.
 constexpr int kQueuePercent = 50;
+
+// A batch has no queue.  Its blocks pack the ring pairs of their tracks'
+// non-zero bins instead, and have twice the pairs, as half of the bins are often
+// 0 (12 problems of 1e5 counts: 11.1 ms; with the zero bins' lanes idle 13.2).
+// counts and pairs are in shared memory.
+struct PackedPairs
+{
+  int* counts;            // of each warp
+  unsigned short* pairs;  // of each group, counted from the block's first
+};
+
+__device__ __forceinline__ PackedPairs packed_pairs(unsigned char* smem, const ColumnPlan& p)
+{
+  const Leftover l = leftover(smem, p);
+  int* counts = reinterpret_cast<int*>(l.lors + p.per_block * p.share);
+  return PackedPairs{counts, reinterpret_cast<unsigned short*>(counts + 8)};
+}
+
+// Packs them; returns the number of the group's.  Every thread of the block
+// calls this.
+__device__ __forceinline__ int pack_nonzero(const Sino& s, const ColumnPlan& p, const ColumnShare& c, int subset,
+                                            const float* __restrict__ sino, const PackedPairs& q)
+{
+  const int lane = threadIdx.x & 31;
+  unsigned mask[kPackedTurn / 32];
+  int n = 0;
+#pragma unroll
+  for (int k = 0; k < kPackedTurn / 32; ++k)
+  {
+    const int i = c.warp * kPackedTurn + 32 * k + lane;
+    int seg, axial;
+    bool on = false;
+    if (c.begin + i < c.end)
+    {
+      ring_pair(s, p, c.begin + i, seg, axial);
+      on = __ldg(sino + column_bin(s, c, subset, seg, axial)) != 0.0f;
+    }
+    mask[k] = __ballot_sync(0xffffffffu, on);
+    n += __popc(mask[k]);
+  }
+  if (lane == 0)
+  {
+    q.counts[threadIdx.x >> 5] = n;
+  }
+  __syncthreads();
+  int all = 0, at = c.group * p.share;
+  for (int w = 0; w < p.warps && c.end > c.begin; ++w)
+  {
+    const int m = q.counts[c.group * p.warps + w];
+    all += m;
+    at += w < c.warp ? m : 0;
+  }
+#pragma unroll
+  for (int k = 0; k < kPackedTurn / 32; ++k)
+  {
+    if (mask[k] >> lane & 1)
+    {
+      q.pairs[at + __popc(mask[k] & ((1u << lane) - 1))] = (unsigned short)(c.warp * kPackedTurn + 32 * k + lane);
+    }
+    at += __popc(mask[k]);
+  }
+  __syncthreads();
+  return all;
+}
 
 // Whether the launch that skips zero bins leaves the others to the queue.
 __device__ __forceinline__ bool queued(const LorQueue& q) { return q.list != nullptr && __ldg(q.count) < q.room; }
@@ -381,7 +448,14 @@ __device__ __forceinline__ bool osem_ratio(float line, int bin, const float* __r
 // The LORs of block number `block` of one OSEM sub-iteration
 // (reconAlgos.cc:119-158, see osem_lor_body): image and accumulators in z
 // columns.
-template<bool kWeighted, bool kSkip>
+enum class ZeroBins
+{
+  Trace,  // not skipped
+  Queue,  // their lanes idle, or (see kQueuePercent) the others queued
+  Pack    // the others packed
+};
+
+template<bool kWeighted, ZeroBins kZero>
 __device__ __forceinline__ void column_osem(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p,
                                             int subset, int block, const double* __restrict__ img,
                                             const float* __restrict__ sino, const float* __restrict__ mult,
@@ -390,33 +464,54 @@ __device__ __forceinline__ void column_osem(const Grid& g, const Sino& s, const 
 {
   const int first = first_track(p, block);
   const ColumnShare c = column_share(s, p, block, first);
-  if (kSkip && queued(queue))
+  if (kZero == ZeroBins::Queue && queued(queue))
   {
     return;
   }
   const Leftover left = leftover(smem, p);
   build_tracks(g, s, t, p, subset, first, smem, left.count);
   const Track tr = track_at(smem, p.cap, c.group);
+  auto trace = [&](const ColumnLor lor[2], const bool on[2]) {
+    ColumnLane w[2] = {};
+    bool go[2];
+    float line[2];
+    column_setup(g, p, tr, c, lor, on, left, w, go);
+    column_lines(tr, go, w, img, line);
+    double value[2] = {0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+    {
+      go[k] = go[k] && osem_ratio<kWeighted>(line[k], lor[k].bin, sino, mult, bias, value[k]);
+    }
+    column_scatter(tr, go, w, value, accumulator_of(g, *tr.head, acc));
+  };
   ColumnLor lor[2];
-  column_lors(s, t, p, c, subset, lor);
-  ColumnLane w[2] = {};
-  bool go[2];
-  float line[2];
   bool on[2] = {true, true};
-#pragma unroll
-  for (int k = 0; k < 2; ++k)
+  if constexpr (kZero == ZeroBins::Pack)
   {
-    on[k] = !kSkip || (lor[k].valid && __ldg(sino + lor[k].bin) != 0.0f);
-  }
-  column_setup(g, p, tr, c, lor, on, left, w, go);
-  column_lines(tr, go, w, img, line);
-  double value[2] = {0.0, 0.0};
+    const PackedPairs q = packed_pairs(smem, p);
+    const int n = pack_nonzero(s, p, c, subset, sino, q);
+    for (int i0 = c.warp * 64; i0 < n; i0 += p.warps * 64)
+    {
 #pragma unroll
-  for (int k = 0; k < 2; ++k)
-  {
-    go[k] = go[k] && osem_ratio<kWeighted>(line[k], lor[k].bin, sino, mult, bias, value[k]);
+      for (int k = 0; k < 2; ++k)
+      {
+        const int i = i0 + 32 * k + (int)(threadIdx.x & 31);
+        lor[k] = column_lor(s, t, p, c, subset, i < n, i < n ? c.begin + q.pairs[c.group * p.share + i] : 0);
+      }
+      trace(lor, on);
+    }
   }
-  column_scatter(tr, go, w, value, accumulator_of(g, *tr.head, acc));
+  else
+  {
+    column_lors(s, t, p, c, subset, lor);
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+    {
+      on[k] = kZero == ZeroBins::Trace || (lor[k].valid && __ldg(sino + lor[k].bin) != 0.0f);
+    }
+    trace(lor, on);
+  }
   column_leftover(s, t, p, subset, block, first, smem, left, [&](const ColumnLor& l, const Track& own) {
     const GeneralLine gl = general_line(g, *own.head, l.z1, l.z2, img, check);
     double q;
@@ -427,7 +522,7 @@ __device__ __forceinline__ void column_osem(const Grid& g, const Sino& s, const 
   });
 }
 
-template<bool kWeighted, bool kSkip>
+template<bool kWeighted, ZeroBins kZero>
 __global__ void __launch_bounds__(256, 5) k_column_osem(const __grid_constant__ Grid g,
                                                         const __grid_constant__ Sino s, Tables t, ColumnPlan p,
                                                         const double* __restrict__ img,
@@ -437,7 +532,7 @@ __global__ void __launch_bounds__(256, 5) k_column_osem(const __grid_constant__ 
                                                         LorQueue queue, int* check)
 {
   extern __shared__ __align__(16) unsigned char smem[];
-  column_osem<kWeighted, kSkip>(g, s, t, p, s.subset, (int)blockIdx.x, img, sino, mult, bias, acc, queue, check, smem);
+  column_osem<kWeighted, kZero>(g, s, t, p, s.subset, (int)blockIdx.x, img, sino, mult, bias, acc, queue, check, smem);
 }
 
 // The queue: the enumerated indices of the subset's non-zero bins, as far as
@@ -564,7 +659,7 @@ __global__ void __launch_bounds__(128, 8) k_queue_backward(const __grid_constant
 
 // The same for the items of a batch (batch.cu), whose work units are the
 // blocks of their problems' plans.
-template<bool kSkip>
+template<ZeroBins kZero>
 __global__ void __launch_bounds__(kBatchColumnBlock, 10)
   k_batch_column_osem(const BatchProblem* __restrict__ P, const BatchItem* __restrict__ items, int n_items, int* check)
 {
@@ -579,7 +674,7 @@ __global__ void __launch_bounds__(kBatchColumnBlock, 10)
       hi = mid;
   }
   const BatchProblem& pb = P[__ldg(&items[lo].problem)];
-  column_osem<false, kSkip>(pb.g, pb.s, pb.t, pb.plan, __ldg(&items[lo].subset),
+  column_osem<false, kZero>(pb.g, pb.s, pb.t, pb.plan, __ldg(&items[lo].subset),
                             (int)blockIdx.x - __ldg(&items[lo].unit_begin), pb.wide, pb.sino, nullptr, pb.bias, pb.bp,
                             LorQueue{}, check, smem);
 }
@@ -695,7 +790,9 @@ bool ask_shared(K kernel, size_t bytes)
 
 size_t column_smem(const ColumnPlan& p)
 {
-  return (size_t)p.per_block * (track_bytes(p.cap) + p.share * sizeof(unsigned)) + 4 * sizeof(int);
+  const size_t packed = 8 * sizeof(int) + (size_t)p.per_block * p.share * sizeof(unsigned short);
+  return (size_t)p.per_block * (track_bytes(p.cap) + p.share * sizeof(unsigned)) + 4 * sizeof(int) +
+         (p.skip != 0 && p.turn == kPackedTurn ? packed : 0);
 }
 
 int column_blocks(const ColumnPlan& p) { return (p.tracks + p.per_block - 1) / p.per_block * p.blocks; }
@@ -714,7 +811,8 @@ ColumnPlan column_plan(const Grid& g, const Sino& s, const double* z, int block,
   // a ring
   const double apart = s.n_rings > 1 ? std::fabs(z[2] - z[0]) * (s.span > 1 ? 0.5 : 1.0) : 0.0;
   p.interleave = apart >= 1.6 * g.ext[2] ? 1 : 0;
-  const int warps = std::max((p.pairs + 63) / 64, 1);
+  p.turn = skip && fixed ? kPackedTurn : 64;
+  const int warps = std::max((p.pairs + p.turn - 1) / p.turn, 1);
   // a track's warps in equal blocks of nearly the wanted size: the count
   // that leaves the fewest warps idle
   const int want = block / 32;
@@ -735,7 +833,7 @@ ColumnPlan column_plan(const Grid& g, const Sino& s, const double* z, int block,
   p.block = best * 32;
   p.blocks = std::max((warps + best - 1) / best, 1);
   p.warps = p.blocks > 1 ? best : warps;
-  p.share = p.blocks > 1 ? best * 64 : std::max(p.pairs, 1);
+  p.share = p.blocks > 1 ? best * p.turn : std::max(p.pairs, 1);
   p.per_block = best / p.warps;
   return p;
 }
@@ -791,7 +889,7 @@ double column_stops(const Grid& g, const Sino& s, const ColumnPlan& p, const dou
 }
 
 // Warps of the launch that have work.
-long long column_warps(const ColumnPlan& p) { return (long long)p.tracks * ((p.pairs + 63) / 64); }
+long long column_warps(const ColumnPlan& p) { return (long long)p.tracks * ((p.pairs + p.turn - 1) / p.turn); }
 
 // Tracks need ring pairs to share them: below 30 most of a warp's 64 slots
 // are idle.  They also need about six warps per scheduler (kColumnWarps) to hide the loops'
@@ -900,7 +998,7 @@ void launch_batch_column_osem(const BatchProblem* P, const BatchItem* items, int
   {
     return;
   }
-  auto* kernel = skip ? k_batch_column_osem<true> : k_batch_column_osem<false>;
+  auto* kernel = skip ? k_batch_column_osem<ZeroBins::Pack> : k_batch_column_osem<ZeroBins::Trace>;
   if (!ask_shared(kernel, bytes))
   {
     return;
@@ -917,9 +1015,13 @@ void launch_column_osem(const Grid& g, const Sino& s, const Tables& t, const Col
     return;
   }
   const size_t bytes = column_smem(p);
-  const bool skip = p.skip != 0;
-  auto* kernel = mult != nullptr ? (skip ? k_column_osem<true, true> : k_column_osem<true, false>)
-                                 : (skip ? k_column_osem<false, true> : k_column_osem<false, false>);
+  // (a plan that packs is a batch's, which has no multiplicative factors)
+  auto* kernel =
+    mult != nullptr
+      ? (p.skip != 0 ? k_column_osem<true, ZeroBins::Queue> : k_column_osem<true, ZeroBins::Trace>)
+      : (p.skip == 0 ? k_column_osem<false, ZeroBins::Trace>
+                     : (p.turn == kPackedTurn ? k_column_osem<false, ZeroBins::Pack>
+                                              : k_column_osem<false, ZeroBins::Queue>));
   if (!ask_shared(kernel, bytes))
   {
     return;

@@ -32,6 +32,7 @@ struct ColumnPlan
   int block;      // threads per block
   int blocks;     // blocks per track
   int share;      // ring pairs of a block's part of a track
+  int turn;       // ring pairs of a warp: 64, or 128 where it packs the non-zero bins
   int warps;      // warps of a block that serve one track
   int per_block;  // tracks per block
   int cap;        // crossings of a track: at most nx + ny
@@ -101,8 +102,8 @@ int queue_room(const Sino& s);
 // image as doubles in z columns ([y][x][z]) and add into two accumulators of
 // that layout, one after the other at acc, whose sum is the backprojection.
 // How a launch with blocks of about `block` threads deals the LORs of s (z: the
-// scanner's slice centres; skip: the projectors skip bins that are 0;
-// fixed: with blocks of exactly that size).
+// scanner's slice centres; skip: the projectors skip bins that are 0; fixed: a
+// batch's launch, of blocks of exactly that size and without a queue).
 ColumnPlan column_plan(const Grid& g, const Sino& s, const double* z, int block, bool skip, bool fixed = false);
 int column_blocks(const ColumnPlan& p);
 // Warps of the launch that have work; below kColumnWarps a launch alone is
