@@ -91,9 +91,10 @@ class TrackPlan(C.Structure):
     """fir_track_plan_info."""
 
     _fields_ = [
-        ("on_tracks", C.c_int), ("ring_pairs", C.c_int), ("tracks", C.c_int), ("threads", C.c_int),
+        ("forward_on_tracks", C.c_int), ("backward_on_tracks", C.c_int), ("osem_on_tracks", C.c_int),
+        ("ring_pairs", C.c_int), ("tracks", C.c_int), ("threads", C.c_int),
         ("block_pairs", C.c_int), ("block_tracks", C.c_int), ("shared_bytes", C.c_longlong),
-        ("warps", C.c_longlong), ("stops", C.c_double), ("clipped", C.c_double),
+        ("warps", C.c_longlong), ("stops", C.c_double), ("general", C.c_double),
     ]
 
 

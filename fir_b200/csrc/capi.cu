@@ -507,10 +507,11 @@ Widened widen_for_projection(fir_ctx& c, const Grid& g, const float* img)
 
 // The plan of a launch on transaxial tracks (column.cu), or tracks = 0 where
 // LOR by LOR is faster.
-ColumnPlan columns_for(const fir_ctx& c, const Grid& g, const Sino& s, bool skip)
+ColumnPlan columns_for(const fir_ctx& c, const Grid& g, const Sino& s, bool skip, TrackUse use)
 {
+  const HostTables t{c.scan_xy.data(), c.scan_z.data()};
   ColumnPlan p = column_plan(g, s, c.scan_z.data(), c.block, skip);
-  if (column_warps(p) < kColumnWarps || !columns_pay(g, s, p, c.scan_z.data(), c.scan_diameter))
+  if (column_warps(p) < kColumnWarps || !columns_pay(g, s, p, t, use))
   {
     p.tracks = 0;
   }
@@ -563,12 +564,13 @@ LorQueue queue_for(fir_ctx& c, const Sino& s, const ColumnPlan& p, const float* 
 }
 
 // The same plan for a launch of this context, which also needs scratch: the
-// image's double copy (image) and the accumulators (acc) in z columns.  Calls
+// image's double copy and the accumulators in z columns, as it uses them.  Calls
 // that the LOR-by-LOR kernels can serve without it must not fail for the lack
 // of it, so without room for it the plan has tracks = 0.
-ColumnPlan columns_here(fir_ctx& c, const Grid& g, const Sino& s, bool skip, bool image, bool acc)
+ColumnPlan columns_here(fir_ctx& c, const Grid& g, const Sino& s, bool skip, TrackUse use)
 {
-  ColumnPlan p = columns_for(c, g, s, skip);
+  ColumnPlan p = columns_for(c, g, s, skip, use);
+  const bool image = use != TrackUse::Backward, acc = use != TrackUse::Forward;
   const size_t n = (size_t)g.nxy * g.nz;
   const size_t queue = queue_bytes(s);
   if (p.tracks == 0)
@@ -626,7 +628,7 @@ Sino nonzero_bins(fir_ctx& c, const Sino& s, const float* sino)
 void project_image(fir_ctx& c, const Grid& g, const Sino& s, const Tables& t, const float* img, float* sino,
                    FwdEpilogue ep)
 {
-  const ColumnPlan plan = columns_here(c, g, s, false, true, false);
+  const ColumnPlan plan = columns_here(c, g, s, false, TrackUse::Forward);
   if (plan.tracks > 0)
   {
     const double* wide = to_columns(c, g, img, nullptr);
@@ -689,7 +691,7 @@ void backproject_subsets(fir_ctx& c, const ProjInfo& p, const VolInfo& v, const 
   ColumnPlan plan{};
   if (c.backproj == FIR_BACKPROJ_ATOMIC)
   {
-    plan = columns_here(c, g, sino_of(p, n_subsets, 0), skip, false, true);
+    plan = columns_here(c, g, sino_of(p, n_subsets, 0), skip, TrackUse::Backward);
   }
   for (int k = 0; k < n_subsets; ++k)
   {
@@ -713,7 +715,7 @@ ColumnPlan osem_columns(fir_ctx& c, const Grid& g, const Sino& s)
   {
     return ColumnPlan{};
   }
-  return columns_here(c, g, s, c.skip_zero != 0, true, true);
+  return columns_here(c, g, s, c.skip_zero != 0, TrackUse::Osem);
 }
 
 // The backprojection of ratio_backproject in z columns (context scratch).
@@ -1831,8 +1833,8 @@ fir_status fir_ctx_set_scanner(fir_ctx* ctx, const fir_scanner_desc* scanner)
     c.z.ensure(s.z.size() * sizeof(double));
     cuda_ok(cudaMemcpy(c.xy.p, s.xy.data(), s.xy.size() * sizeof(double), cudaMemcpyHostToDevice), "cudaMemcpy");
     cuda_ok(cudaMemcpy(c.z.p, s.z.data(), s.z.size() * sizeof(double), cudaMemcpyHostToDevice), "cudaMemcpy");
+    c.scan_xy = s.xy;
     c.scan_z = s.z;
-    c.scan_diameter = 2.0 * std::hypot(s.xy[0], s.xy[1]);
     c.scan_rings = s.n_rings;
     c.scan_cpr = s.n_cpr;
     c.have_scanner = true;
@@ -1869,12 +1871,15 @@ fir_status fir_track_plan(const fir_scanner_desc* scanner, const fir_proj_desc* 
     fir_ctx c;
     c.geometry = geometry;
     c.block = block_size > 0 ? block_size : c.block;
+    c.scan_xy = sc.xy;
     c.scan_z = sc.z;
-    c.scan_diameter = 2.0 * std::hypot(sc.xy[0], sc.xy[1]);
     const Grid g = grid_of(c, v);
     const Sino s = sino_of(p, n_subsets, subset);
     const ColumnPlan plan = column_plan(g, s, c.scan_z.data(), c.block, skip_zero != 0);
-    out->on_tracks = columns_for(c, g, s, skip_zero != 0).tracks > 0 ? 1 : 0;
+    auto on = [&](TrackUse use) { return columns_for(c, g, s, skip_zero != 0, use).tracks > 0 ? 1 : 0; };
+    out->forward_on_tracks = on(TrackUse::Forward);
+    out->backward_on_tracks = on(TrackUse::Backward);
+    out->osem_on_tracks = on(TrackUse::Osem);
     out->ring_pairs = plan.pairs;
     out->tracks = plan.tracks;
     out->threads = plan.block;
@@ -1882,8 +1887,9 @@ fir_status fir_track_plan(const fir_scanner_desc* scanner, const fir_proj_desc* 
     out->block_tracks = plan.per_block;
     out->shared_bytes = (long long)column_smem(plan);
     out->warps = column_warps(plan);
-    out->stops = column_stops(g, s, plan, c.scan_z.data(), c.scan_diameter);
-    out->clipped = column_clipped(g, s, c.scan_z.data(), c.scan_diameter);
+    const HostTables t{c.scan_xy.data(), c.scan_z.data()};
+    out->stops = column_stops(g, s, plan, t);
+    out->general = column_general(g, s, t);
   });
 }
 

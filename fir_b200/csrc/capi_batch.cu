@@ -492,7 +492,7 @@ fir_status fir_batch_create(fir_batch** out, fir_ctx* ctx, int n_problems, const
       {
         q.plan = plans[(size_t)k];  // (columns_pay has looked at this one)
       }
-      if (columns_pay(g, s, plans[(size_t)k], sc.z.data(), 2.0 * std::hypot(sc.xy[0], sc.xy[1])))
+      if (columns_pay(g, s, plans[(size_t)k], HostTables{sc.xy.data(), sc.z.data()}, TrackUse::Batch))
       {
         pays[(size_t)k] = 1;
         track_warps += column_warps(plans[(size_t)k]);

@@ -154,8 +154,7 @@ struct fir_ctx
 
   bool have_scanner = false;
   int scan_rings = 0, scan_cpr = 0;
-  std::vector<double> scan_z;  // slice centres (host copy)
-  double scan_diameter = 0.0;  // of the first crystal's circle
+  std::vector<double> scan_xy, scan_z;  // the scanner's tables (host copies)
   fir::abi::DevBuf xy, z;
 
   fir::abi::DevBuf check;     // device check word

@@ -838,38 +838,123 @@ ColumnPlan column_plan(const Grid& g, const Sino& s, const double* z, int block,
   return p;
 }
 
-// Share of the ring pairs whose LOR through the axis meets the volume but
-// enters or leaves it through an end face: those take the general walk.
-double column_clipped(const Grid& g, const Sino& s, const double* z, double diameter)
+// Where the tracks of view and tang run through the volume (track_setup, as a
+// fraction of the LOR); false where they miss it.
+static bool track_span(const Grid& g, const Sino& s, const double* xy, int view, int tang, double span[2])
 {
-  if (z[0] > g.low[2] && z[0] < g.high[2] && z[2 * s.n_rings - 2] > g.low[2] && z[2 * s.n_rings - 2] < g.high[2])
+  int c[2];
+  crystal_ang(s, view, tang, c[0], c[1]);
+  span[0] = 0.0;
+  span[1] = 1.0;
+  for (int d = 0; d < 2; ++d)
   {
-    return 0.0;
+    const double p1 = xy[2 * c[0] + d], df = xy[2 * c[1] + d] - p1;
+    if (std::fabs(df) <= kEps)
+    {
+      if (p1 < g.low[d] || p1 > g.high[d])
+      {
+        return false;
+      }
+      continue;
+    }
+    const double a = (g.low[d] - p1) / df, b = (g.high[d] - p1) / df;
+    span[0] = std::max(span[0], std::min(a, b));
+    span[1] = std::min(span[1], std::max(a, b));
   }
-  const double across = std::max(g.high[0] - g.low[0], g.high[1] - g.low[1]);
-  const double in = std::max(0.5 * (diameter - across) / diameter, 0.0);
-  long long all = 0, clipped = 0;
+  return span[0] < span[1];
+}
+
+// lane_setup's choice for a LOR between z1 and z2 on such a track, up to its
+// rounding.
+static LorKind lor_kind(const Grid& g, const double span[2], double z1, double z2)
+{
+  const double lo = g.low[2], hi = g.high[2];
+  const double diff = z2 - z1, df = std::fabs(diff) > kEps ? diff : kEps;
+  const bool moves = std::fabs(diff) > kEps, up = diff > kEps;
+  const double in = moves ? ((up ? lo : hi) - z1) / df : 0.0, out = moves ? ((up ? hi : lo) - z1) / df : 1.0;
+  if ((!moves && (z1 < lo || z1 > hi)) || std::max(in, span[0]) >= std::min(out, span[1]))
+  {
+    return kLorNone;
+  }
+  const double dz = std::fabs(g.ext[2] / df);
+  const double at = std::trunc((z1 + df * span[0] - lo) / g.ext[2]);
+  const double ind = std::min(std::max(at, 0.0), g.nz - 1.0);
+  const double next = (moves ? (lo + g.ext[2] * ind - z1) / df : 1.0) + (up ? dz : 0.0);
+  const double leaves = next + (up ? g.nz - 1 - ind : ind) * dz;
+  return in <= span[0] && out >= span[1] && dz > 4.0 * kEps && leaves > span[1] + 4.0 * kEps ? kLorColumn
+                                                                                           : kLorGeneral;
+}
+
+double column_general(const Grid& g, const Sino& s, const HostTables& t)
+{
+  const double *xy = t.xy, *z = t.z;
+  long long pairs = 0;
   for (int k = 0; k < s.n_segments; ++k)
   {
-    for (int axial = 0; axial < s.n_axial[k]; ++axial)
+    pairs += s.n_axial[k];
+  }
+  const double bottom = std::min(z[0], z[2 * s.n_rings - 2]), top = std::max(z[0], z[2 * s.n_rings - 2]);
+  // (the traversal's slices may be thinner than the voxels and end below the
+  // volume's top)
+  const double end = std::min(g.low[2] + g.nz * g.ext[2], g.high[2]), margin = 1e-4 * (top - bottom);
+  if (bottom > g.low[2] + margin && top < end - margin)
+  {
+    // z clips nothing.  The direct LORs of the lowest slice take the general
+    // walk where they end at a crystal within the volume.
+    int inside = 0;
+    for (int c = 0; c < s.n_cpr; ++c)
+    {
+      const double x = xy[2 * c], y = xy[2 * c + 1];
+      inside += x >= g.low[0] && x <= g.high[0] && y >= g.low[1] && y <= g.high[1] ? 1 : 0;
+    }
+    int direct = 0;
+    for (int axial = 0; inside > 0 && axial < s.n_axial[s.seg_offset]; ++axial)
     {
       int a1, a2;
-      crystal_axial(s, k - s.seg_offset, axial, a1, a2);
-      const double z1 = z[a1] + in * (z[a2] - z[a1]), z2 = z[a2] + in * (z[a1] - z[a2]);
-      const double lo = std::min(z1, z2), hi = std::max(z1, z2);
-      const bool meets = hi > g.low[2] && lo < g.high[2];
-      all += meets ? 1 : 0;
-      clipped += meets && (lo < g.low[2] || hi > g.high[2]) ? 1 : 0;
+      crystal_axial(s, 0, axial, a1, a2);
+      direct += z[a1] < g.low[2] + g.ext[2] ? 1 : 0;
+    }
+    return (double)inside / s.n_cpr * direct / pairs;
+  }
+  // sampled: 8 views x 5 tangential bins.  In a segment they are the first or
+  // the last planes, so it is read from both ends.
+  long long general = 0, meeting = 0;
+  for (int i = 0; i < 40; ++i)
+  {
+    double span[2];
+    if (!track_span(g, s, xy, i / 5 * s.n_views / 8, (2 * (i % 5) + 1) * s.n_tang / 10 - s.tang_offset, span))
+    {
+      continue;
+    }
+    meeting += pairs;
+    for (int k = 0; k < s.n_segments; ++k)
+    {
+      auto kind = [&](int axial) {
+        int a1, a2;
+        crystal_axial(s, k - s.seg_offset, axial, a1, a2);
+        return lor_kind(g, span, z[a1], z[a2]);
+      };
+      int first = 0, last = s.n_axial[k];
+      for (LorKind q; first < last && (q = kind(first)) != kLorColumn; ++first)
+      {
+        (q == kLorGeneral ? general : meeting) += q == kLorGeneral ? 1 : -1;
+      }
+      for (LorKind q; last > first && (q = kind(last - 1)) != kLorColumn; --last)
+      {
+        (q == kLorGeneral ? general : meeting) += q == kLorGeneral ? 1 : -1;
+      }
     }
   }
-  return all > 0 ? (double)clipped / all : 0.0;
+  return meeting > 0 ? (double)general / meeting : 0.0;
 }
 
 // Mean number of z crossings that stop a warp's turn per crossing of its
 // track: the LORs of a segment cross together where their planes lie whole
 // voxels apart, so a segment counts once per distinct offset.
-double column_stops(const Grid& g, const Sino& s, const ColumnPlan& p, const double* z, double diameter)
+double column_stops(const Grid& g, const Sino& s, const ColumnPlan& p, const HostTables& t)
 {
+  const double* z = t.z;
+  const double diameter = 2.0 * std::hypot(t.xy[0], t.xy[1]);
   const double apart = s.n_rings > 1 ? std::fabs(z[2] - z[0]) * (s.span > 1 ? 0.5 : 1.0) / g.ext[2] : 0.0;
   int offsets = 1;
   while (offsets < 64 && std::fabs(offsets * apart - std::round(offsets * apart)) > 1e-3)
@@ -891,21 +976,44 @@ double column_stops(const Grid& g, const Sino& s, const ColumnPlan& p, const dou
 // Warps of the launch that have work.
 long long column_warps(const ColumnPlan& p) { return (long long)p.tracks * ((p.pairs + p.turn - 1) / p.turn); }
 
-// Tracks need ring pairs to share them: below 30 most of a warp's 64 slots
-// are idle.  They also need about six warps per scheduler (kColumnWarps) to hide the loops'
-// latency (a turn waits for its entry and test): the LOR-by-LOR kernels, with
-// twice the warps, are faster below that (measured 0.63x to 0.98x below 3000
-// warps, 1.3x and more above 8000).  A LOR clipped by the volume's ends walks
-// alone in its block's last pass (0.65x at 11 %, 1.14x at 2 %), and a stop
-// makes a turn nearly twice as long (1.1x at 3.2 stops per turn on small
-// volumes, 0.96x at 2.3 on a 320x320x128 one).
-bool columns_pay(const Grid& g, const Sino& s, const ColumnPlan& p, const double* z, double diameter)
+// Tracks need ring pairs to share them, or most of a warp's 64 slots are idle:
+// with 36 pairs (6 rings) projection and fused kernel take 1.2 and 1.1 times as
+// long as LOR by LOR, with 49 0.96 and 0.85 times; the backprojection, bound by
+// its atomics, gains at 36 too (0.67).  They also need about six warps per
+// scheduler (kColumnWarps) to hide the loops' latency (a turn waits for its
+// entry and test): the LOR-by-LOR kernels, with twice the warps, are faster
+// below that (measured 0.63x to 0.98x below 3000 warps, 1.3x and more above
+// 8000).  A stop makes a turn nearly twice as long (1.1x at 3.2 stops per turn on
+// small volumes, 0.96x at 2.3 on a 320x320x128 one).
+//
+// A block with a LOR that z clips takes a whole walk longer, with most of its
+// warps idle, so the gain goes with the share of such LORs, and sooner where the
+// launch has few waves to fill the gaps.  Tracks against LOR by LOR:
+//   fused kernel, 25000 warps and more: 24 rings 1.73x unclipped, 1.31x at 1.7 %,
+//   1.06x at 5.8 %; 32 rings 1.15x at 1.5 %, 1.05x at 5 %, 0.99x at 8.7 %, 40 rings
+//   1.11x at 7.4 %; 24 rings 0.98x at 22 %
+//   12000 to 25000: 17 rings 1.57x, 1.04x at 1.7 %; span 3 1.38x, 1.10x at 0.2 %,
+//   1.0x at 1.5 %, 0.95x at 2.7 %
+//   fewer: 24 rings 1.38x, 0.97x at 1.7 %; 8 rings 1.15x, 0.88x at 0.13 %
+//   projection (all views): 1.04x at 8.7 %, 1.0x at 8.2 % (span 3), 1.0x at 22 %;
+//   with 64 pairs, whose blocks hold four tracks, 0.96x at 0.13 %, 0.5x at 12 %
+//   backprojection: 1.15x to 1.4x at 20 %, even at 45 % with 36 pairs.
+bool columns_pay(const Grid& g, const Sino& s, const ColumnPlan& p, const HostTables& t, TrackUse use)
 {
-  if (g.exact_only || p.pairs < 30 || column_smem(p) > kColumnSharedLimit || (long long)g.nxy * g.nz >= 1LL << 29)
+  const bool back = use == TrackUse::Backward;
+  if (g.exact_only || p.pairs < (back ? 30 : 44) || column_smem(p) > kColumnSharedLimit ||
+      (long long)g.nxy * g.nz >= 1LL << 29)
   {
     return false;
   }
-  return column_stops(g, s, p, z, diameter) <= 2.2 && column_clipped(g, s, z, diameter) <= 0.04;
+  if ((g.nz + kTile - 1) / kTile > 65535)
+  {
+    return false;  // beyond the tile grid of the z-column copies
+  }
+  const long long warps = use == TrackUse::Batch ? 12000 : column_warps(p);
+  const double most =
+    back ? 0.2 : (p.pairs <= 64 || warps < 12000 ? 3e-4 : (warps < 25000 ? 0.012 : 0.08));
+  return column_stops(g, s, p, t) <= 2.2 && column_general(g, s, t) <= most;
 }
 
 void launch_to_columns(const Grid& g, const float* in, double* out, float* acc, const LaunchCfg& cfg)

@@ -109,13 +109,28 @@ int column_blocks(const ColumnPlan& p);
 // Warps of the launch that have work; below kColumnWarps a launch alone is
 // faster LOR by LOR.
 long long column_warps(const ColumnPlan& p);
-// What columns_pay looks at: see there.
-double column_stops(const Grid& g, const Sino& s, const ColumnPlan& p, const double* z, double diameter);
-double column_clipped(const Grid& g, const Sino& s, const double* z, double diameter);
+// The scanner's tables in host memory.
+struct HostTables
+{
+  const double* xy;  // crystal centres of one ring
+  const double* z;   // slice centres
+};
+// Mean z crossings that stop a warp's turn per crossing of its track; share of
+// the LORs meeting the volume that take the general walk, because z clips them
+// or leaves the traversal's slices before they end.
+double column_stops(const Grid& g, const Sino& s, const ColumnPlan& p, const HostTables& t);
+double column_general(const Grid& g, const Sino& s, const HostTables& t);
 constexpr long long kColumnWarps = 6 * 592;
 // Whether a launch with enough warps is faster on tracks than LOR by LOR (z:
-// the scanner's slice centres, diameter: of a ring).
-bool columns_pay(const Grid& g, const Sino& s, const ColumnPlan& p, const double* z, double diameter);
+// Whether a launch with enough warps is faster on tracks than LOR by LOR.
+enum class TrackUse
+{
+  Forward,
+  Backward,
+  Osem,
+  Batch  // a problem's part of a batch's launches
+};
+bool columns_pay(const Grid& g, const Sino& s, const ColumnPlan& p, const HostTables& t, TrackUse use);
 // out = the image's double copy in z columns; the accumulators (or null) = 0.
 void launch_to_columns(const Grid& g, const float* in, double* out, float* acc, const LaunchCfg& cfg);
 // out = the accumulators' sum in [z][y][x].

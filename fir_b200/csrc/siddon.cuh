@@ -180,7 +180,7 @@ __host__ __device__ __forceinline__ void crystal_axial(const Sino& s, int seg, i
 }
 
 // ProjData::getCrystalAngCoord (ProjData.cc:301-340).
-__device__ __forceinline__ void crystal_ang(const Sino& s, int view, int tang, int& c1, int& c2)
+__host__ __device__ __forceinline__ void crystal_ang(const Sino& s, int view, int tang, int& c1, int& c2)
 {
   const int shift = tang >= 0 ? tang / 2 : (tang - 1) / 2;
   const int odd = (tang < 0 ? -tang : tang) & 1;

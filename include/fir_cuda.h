@@ -227,7 +227,9 @@ long long fir_ctx_track_launch_count(const fir_ctx* ctx);
  * projections bit for bit.  Host arithmetic only: no device is needed. */
 typedef struct fir_track_plan_info
 {
-  int on_tracks;          /* 1: the launch runs on tracks */
+  int forward_on_tracks;  /* 1: the projection runs on tracks, */
+  int backward_on_tracks; /* the backprojection, */
+  int osem_on_tracks;     /* the OSEM sub-iteration */
   int ring_pairs;         /* LORs that share a track */
   int tracks;             /* (view, tangential bin) pairs of the subset */
   int threads;            /* per block */
@@ -236,7 +238,7 @@ typedef struct fir_track_plan_info
   long long shared_bytes; /* shared memory of a block */
   long long warps;        /* of the launch */
   double stops;           /* axial crossings that stop a warp, per transaxial one */
-  double clipped;         /* share of the LORs that take the general walk */
+  double general;         /* share of the LORs traced one by one all the same */
 } fir_track_plan_info;
 /* geometry: FIR_GEOMETRY_*; block_size: FIR_OPT_BLOCK_SIZE (0: the default);
  * skip_zero: FIR_OPT_SKIP_ZERO_BINS. */

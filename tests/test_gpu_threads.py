@@ -99,7 +99,7 @@ def sizes():
 
 def test_plans_need_different_amounts():
     large, small = sizes()
-    assert large.on_tracks and small.on_tracks
+    assert large.forward_on_tracks and small.forward_on_tracks
     assert 96 * 1024 >= large.shared_bytes > small.shared_bytes > 48 * 1024
 
 

@@ -49,7 +49,7 @@ def test_outputs_are_overwritten_and_null_is_refused():
     add to it), and refuses a missing one."""
     scanner, proj, vol = (ScannerSpec.ring(13, 96, 130.0, 4.0), ProjSpec(13, 96, 25, 25),
                           VolSpec.centred((40, 40, 30), (4.0, 4.0, 2.0)))
-    assert capi.track_plan(scanner, proj, vol).on_tracks
+    assert capi.track_plan(scanner, proj, vol).osem_on_tracks
     nb = capi.proj_geometry(proj)["n_bins"]
     rng = np.random.default_rng(2)
     y = rng.poisson(1.0, nb).astype(np.float32)
@@ -91,7 +91,7 @@ def test_first_backprojection_may_be_captured_above_l2():
     l2 = torch.cuda.get_device_properties(0).L2_cache_size
     nz = int(l2 / 8 / (280 * 280)) + 2
     vol = VolSpec.centred((280, 280, nz), (2.0, 2.0, 2.0))
-    assert capi.track_plan(scanner, proj, vol).on_tracks
+    assert capi.track_plan(scanner, proj, vol).osem_on_tracks
     nb = capi.proj_geometry(proj)["n_bins"]
     y = torch.rand(nb, device="cuda")
     out = torch.zeros(vol.shape_zyx, device="cuda")
@@ -129,8 +129,8 @@ def test_captured_launch_keeps_its_scratch():
 
     scanner, proj, vol = (ScannerSpec.ring(13, 96, 130.0, 4.0), ProjSpec(13, 96, 25, 25),
                           VolSpec.centred((40, 40, 30), (4.0, 4.0, 2.0)))
-    assert capi.track_plan(scanner, proj, vol).on_tracks
-    assert not capi.track_plan(scanner, proj, vol, n_subsets=4).on_tracks
+    assert capi.track_plan(scanner, proj, vol).osem_on_tracks
+    assert not capi.track_plan(scanner, proj, vol, n_subsets=4).osem_on_tracks
     nb = capi.proj_geometry(proj)["n_bins"]
     rng = np.random.default_rng(3)
     y = torch.from_numpy(rng.poisson(2.0, nb).astype(np.float32)).cuda()
@@ -168,7 +168,7 @@ def test_skipped_bins_at_any_occupancy(occupied, span):
     else:
         scanner, proj, vol = (ScannerSpec.ring(16, 128, 160.0, 4.0), ProjSpec(16, 128, 9, 31, 3),
                               VolSpec.centred((47, 51, 17), (4.0, 4.0, 4.0)))
-    assert capi.track_plan(scanner, proj, vol, skip_zero=True).on_tracks
+    assert capi.track_plan(scanner, proj, vol, skip_zero=True).osem_on_tracks
     nb = capi.proj_geometry(proj)["n_bins"]
     rng = np.random.default_rng(4)
     y = rng.poisson(3.0, nb).astype(np.float32) + np.float32(1)
