@@ -223,12 +223,14 @@ __device__ __forceinline__ float take_backprojection(const Voxel& v, Tile& tile)
     const int k = tile_element(v, slice, column);
     if (k >= 0)
     {
+      const size_t n = (size_t)pb.nvox;
       float* const a = pb.bp + k;
-      float* const c = a + pb.nvox;
-      const float va = *a, vc = *c;
-      tile.v[slice][column] = __fadd_rn(va, vc);
-      *a = 0.0f;
-      *c = 0.0f;
+      const float v0 = a[0], v1 = a[n], v2 = a[2 * n], v3 = a[3 * n];
+      tile.v[slice][column] = __fadd_rn(__fadd_rn(v0, v2), __fadd_rn(v1, v3));
+      a[0] = 0.0f;
+      a[n] = 0.0f;
+      a[2 * n] = 0.0f;
+      a[3 * n] = 0.0f;
     }
     __syncthreads();
     const float b = tile.v[threadIdx.x >> 5][threadIdx.x & 31];

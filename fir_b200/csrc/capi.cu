@@ -579,7 +579,7 @@ ColumnPlan columns_here(fir_ctx& c, const Grid& g, const Sino& s, bool skip, Tra
   }
   const size_t had = c.wide.bytes;
   if ((image && !can_hold(c, c.wide, n * sizeof(double))) ||
-      (acc && !can_hold(c, c.column_acc, 2 * n * sizeof(float))) || (skip && !can_hold(c, c.compact, queue)))
+      (acc && !can_hold(c, c.column_acc, kColumnAccumulators * n * sizeof(float))) || (skip && !can_hold(c, c.compact, queue)))
   {
     if (c.wide.bytes > had)
     {
@@ -591,7 +591,7 @@ ColumnPlan columns_here(fir_ctx& c, const Grid& g, const Sino& s, bool skip, Tra
 }
 
 // Writes the image's double copy in z columns to context scratch and clears
-// the two accumulators at acc (or null).
+// the accumulators at acc (or null).
 const double* to_columns(fir_ctx& c, const Grid& g, const float* img, float* acc)
 {
   double* d = static_cast<double*>(c.wide.ensure((size_t)g.nxy * g.nz * sizeof(double)));
@@ -600,9 +600,11 @@ const double* to_columns(fir_ctx& c, const Grid& g, const float* img, float* acc
   return d;
 }
 
+size_t column_acc_bytes(const Grid& g) { return (size_t)kColumnAccumulators * g.nxy * g.nz * sizeof(float); }
+
 float* column_accumulators(fir_ctx& c, const Grid& g)
 {
-  return static_cast<float*>(c.column_acc.ensure(2 * (size_t)g.nxy * g.nz * sizeof(float)));
+  return static_cast<float*>(c.column_acc.ensure(column_acc_bytes(g)));
 }
 
 // s with the compacted list of its bins whose measured value is not 0
@@ -651,13 +653,13 @@ void backproject_subset(fir_ctx& c, const Grid& g, const Sino& s, const Tables& 
   if (plan.tracks > 0)
   {
     float* acc = column_accumulators(c, g);
-    cuda_ok(cudaMemsetAsync(acc, 0, 2 * (size_t)n * sizeof(float), c.stream), "cudaMemsetAsync");
+    cuda_ok(cudaMemsetAsync(acc, 0, column_acc_bytes(g), c.stream), "cudaMemsetAsync");
     const LorQueue queue = queue_for(c, s, plan, sino);
     timed_launch(c, [&] {
       launch_column_backward(g, s, t, plan, sino, acc, queue, cfg_of(c));
       if (queue.list != nullptr)
       {
-        launch_queue_backward(g, s, t, sino, acc, queue, cfg_of(c));
+        launch_queue_backward(g, s, t, plan, sino, acc, queue, cfg_of(c));
       }
     });
     c.launches += queue.list != nullptr ? 1 : 0;
@@ -730,7 +732,7 @@ const float* column_ratio_backproject(fir_ctx& c, const Grid& g, const Sino& s, 
     launch_column_osem(g, s, t, p, wide, sino, mult, bias, acc, queue, cfg_of(c));
     if (queue.list != nullptr)
     {
-      launch_queue_osem(g, s, t, wide, sino, mult, bias, acc, queue, cfg_of(c));
+      launch_queue_osem(g, s, t, p, wide, sino, mult, bias, acc, queue, cfg_of(c));
     }
   });
   c.launches += queue.list != nullptr ? 1 : 0;

@@ -515,7 +515,7 @@ fir_status fir_batch_create(fir_batch** out, fir_ctx* ctx, int n_problems, const
           !q.columns && !q.exchanged && !use_exchanged(c, g, 12.0) && use_exchanged(c, g, 8.0);
       }
       q.off_wide = take(q.gather_float ? 0 : nv * sizeof(double));
-      q.off_bp = take((q.columns ? 2 : 1) * nv * sizeof(float));
+      q.off_bp = take((q.columns ? kColumnAccumulators : 1) * nv * sizeof(float));
       q.off_wide_t = take(q.exchanged ? nv * sizeof(double) : 0);
       q.off_bp_t = take(q.exchanged || q.gather_float ? nv * sizeof(float) : 0);
       q.off_img_t = take(q.gather_float ? nv * sizeof(float) : 0);

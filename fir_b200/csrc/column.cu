@@ -375,11 +375,16 @@ __global__ void __launch_bounds__(256, 5) k_column_forward(const __grid_constant
   });
 }
 
-// A track's accumulator: tracks along x and along y add into one each, which
-// are summed at the end.  Each sum then rounds at half the size.
 __device__ __forceinline__ float* accumulator_of(const Grid& g, const TrackHead& h, float* acc)
 {
-  return acc + (h.crosses && h.along_x ? (size_t)g.nxy * g.nz : 0);
+  return acc + (h.crosses ? (size_t)h.acc * g.nxy * g.nz : 0);
+}
+
+// The sum of the accumulators' elements k (n each).
+__device__ __forceinline__ float accumulated(const float* __restrict__ acc, size_t n, size_t k)
+{
+  static_assert(kColumnAccumulators == 4, "");
+  return __fadd_rn(__fadd_rn(acc[k], acc[2 * n + k]), __fadd_rn(acc[n + k], acc[3 * n + k]));
 }
 
 // projections::backward (projections.cc:94-184) into the accumulators in z
@@ -613,22 +618,21 @@ template<bool kWeighted>
 __global__ void __launch_bounds__(128, 8) k_queue_osem(const __grid_constant__ Grid g, const __grid_constant__ Sino s,
                                                        Tables t, const double* __restrict__ img,
                                                        const float* __restrict__ sino, const float* __restrict__ mult,
-                                                       const float* __restrict__ bias, float* acc, LorQueue queue,
-                                                       int* check)
+                                                       const float* __restrict__ bias, float* acc, int views,
+                                                       LorQueue queue, int* check)
 {
   if (!queued(queue))
   {
     return;
   }
-  osem_lor_body<kWeighted, double, true>(g, s, s.subset, t, img, img, sino, mult, bias, acc,
-                                         acc + (size_t)g.nxy * g.nz, true, blockIdx.x * blockDim.x + threadIdx.x,
-                                         check);
+  osem_lor_body<kWeighted, double, true>(g, s, s.subset, t, img, img, sino, mult, bias, acc, acc, true,
+                                         blockIdx.x * blockDim.x + threadIdx.x, check, -1, views);
 }
 
 __global__ void __launch_bounds__(128, 8) k_queue_backward(const __grid_constant__ Grid g,
                                                            const __grid_constant__ Sino s, Tables t,
-                                                           const float* __restrict__ sino, float* acc, LorQueue queue,
-                                                           int* check)
+                                                           const float* __restrict__ sino, float* acc, int views,
+                                                           LorQueue queue, int* check)
 {
   if (!queued(queue))
   {
@@ -647,7 +651,8 @@ __global__ void __launch_bounds__(128, 8) k_queue_backward(const __grid_constant
     lor_ends(s, t, l, e);
     go = siddon_setup<true>(g, e, w);
     value = (double)__ldg(sino + l.bin);
-    to += fabs(dsub(e[3], e[0])) > fabs(dsub(e[4], e[1])) ? (size_t)g.nxy * g.nz : 0;
+    to += (size_t)column_accumulator(fabs(dsub(e[3], e[0])) > fabs(dsub(e[4], e[1])), l.view / s.n_subsets, views) *
+          g.nxy * g.nz;
   }
   const bool ok = siddon_walk<true>(
     g, w, go, [&](bool, int c, double len) { atomicAdd(to + c, __double2float_rn(dmul(len, value))); });
@@ -688,8 +693,8 @@ dim3 column_tiles(int np, int nz)
   return dim3((unsigned)((np + kTile - 1) / kTile), (unsigned)((nz + kTile - 1) / kTile));
 }
 
-// out = the double copy of in in z columns; both accumulators at acc (or
-// null) = 0.
+// out = the double copy of in in z columns; the accumulators at acc (or null)
+// = 0.
 __global__ void __launch_bounds__(kTile * kTileRows) k_to_columns(int np, int nz, const float* __restrict__ in,
                                                                   double* __restrict__ out, float* __restrict__ acc)
 {
@@ -713,8 +718,11 @@ __global__ void __launch_bounds__(kTile * kTileRows) k_to_columns(int np, int nz
       out[k] = (double)tile[threadIdx.x][j];
       if (acc != nullptr)
       {
-        acc[k] = 0.0f;
-        acc[(size_t)np * nz + k] = 0.0f;
+#pragma unroll
+        for (int a = 0; a < kColumnAccumulators; ++a)
+        {
+          acc[(size_t)a * np * nz + k] = 0.0f;
+        }
       }
     }
   }
@@ -731,7 +739,7 @@ __global__ void __launch_bounds__(kTile * kTileRows) k_from_columns(int np, int 
     const int z = z0 + threadIdx.x, p = p0 + j;
     if (p < np && z < nz)
     {
-      tile[j][threadIdx.x] = __fadd_rn(acc[(size_t)p * nz + z], acc[(size_t)np * nz + (size_t)p * nz + z]);
+      tile[j][threadIdx.x] = accumulated(acc, (size_t)np * nz, (size_t)p * nz + z);
     }
   }
   __syncthreads();
@@ -757,7 +765,7 @@ __global__ void __launch_bounds__(kTile * kTileRows) k_em_update_columns(int np,
     const int z = z0 + threadIdx.x, p = p0 + j;
     if (p < np && z < nz)
     {
-      tile[j][threadIdx.x] = __fadd_rn(acc[(size_t)p * nz + z], acc[(size_t)np * nz + (size_t)p * nz + z]);
+      tile[j][threadIdx.x] = accumulated(acc, (size_t)np * nz, (size_t)p * nz + z);
     }
   }
   __syncthreads();
@@ -1084,19 +1092,20 @@ static Sino queue_of(const Sino& s, const LorQueue& queue)
   return q;
 }
 
-void launch_queue_backward(const Grid& g, const Sino& s, const Tables& t, const float* sino, float* acc,
-                           const LorQueue& queue, const LaunchCfg& cfg)
+void launch_queue_backward(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p, const float* sino,
+                           float* acc, const LorQueue& queue, const LaunchCfg& cfg)
 {
   k_queue_backward<<<(unsigned)(queue.room + 127) / 128, 128, 0, cfg.stream>>>(g, queue_of(s, queue), t, sino, acc,
-                                                                                 queue, cfg.check);
+                                                                                 p.tracks / s.n_tang, queue, cfg.check);
 }
 
-void launch_queue_osem(const Grid& g, const Sino& s, const Tables& t, const double* img, const float* sino,
-                       const float* mult, const float* bias, float* acc, const LorQueue& queue, const LaunchCfg& cfg)
+void launch_queue_osem(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p, const double* img,
+                       const float* sino, const float* mult, const float* bias, float* acc, const LorQueue& queue,
+                       const LaunchCfg& cfg)
 {
   auto* kernel = mult != nullptr ? k_queue_osem<true> : k_queue_osem<false>;
   kernel<<<(unsigned)(queue.room + 127) / 128, 128, 0, cfg.stream>>>(g, queue_of(s, queue), t, img, sino, mult, bias,
-                                                                       acc, queue, cfg.check);
+                                                                       acc, p.tracks / s.n_tang, queue, cfg.check);
 }
 
 void launch_batch_column_osem(const BatchProblem* P, const BatchItem* items, int n_items, int n_blocks, size_t bytes,

@@ -63,7 +63,7 @@ struct TrackHead
   int col;     // first column
   int exit;    // index of the first crossing that leaves the volume
   int crosses; // 0: no LOR of the track crosses the volume
-  int along_x; // 1: the track runs mostly along x
+  int acc;     // number of the track's accumulator
   int shared;  // 1: the LORs may use the list
 };
 
@@ -86,6 +86,12 @@ __device__ __forceinline__ PlainCrossing plain_crossing(const Crossing& c)
   const int4 v = *reinterpret_cast<const int4*>(&c);
   return v.y == kExactHigh ? PlainCrossing{__hiloint2double(v.w, v.z), v.x}
                            : PlainCrossing{__hiloint2double(v.y, v.x), v.z >> 2};
+}
+
+// The accumulator of a track in view number sv of the subset's views.
+__device__ __forceinline__ int column_accumulator(bool along_x, int sv, int views)
+{
+  return (along_x ? 1 : 0) + (2 * sv >= views ? 2 : 0);
 }
 
 // x and y parts of siddon_setup for one track.
@@ -233,7 +239,7 @@ __device__ __forceinline__ void build_tracks(const Grid& g, const Sino& s, const
       h.y1 = p1.y;
       h.x2 = p2.x;
       h.y2 = p2.y;
-      h.along_x = fabs(dsub(p2.x, p1.x)) > fabs(dsub(p2.y, p1.y)) ? 1 : 0;
+      h.acc = column_accumulator(fabs(dsub(p2.x, p1.x)) > fabs(dsub(p2.y, p1.y)), sv, p.tracks / s.n_tang);
       track_setup(g, h);
     }
   }

@@ -41,6 +41,13 @@ struct ColumnPlan
 };
 // Shared memory of one block.
 size_t column_smem(const ColumnPlan& p);
+// The projectors on tracks add into one of this many float accumulators, by the
+// track's direction (mostly along x or y) and half of the subset's views: in
+// each the sums, and so their roundings, are smaller.  Error of a clinical
+// sub-iteration against 64 bits: one accumulator 3e-7, two 1.72e-7 (LOR by LOR,
+// whose warps add up some of their atomics first, 1.58e-7), four 1.2e-7
+// (and 10 us of 1.27 ms more).
+constexpr int kColumnAccumulators = 4;
 // The most that a plan may ask for.
 constexpr size_t kColumnSharedLimit = 96 * 1024;
 
@@ -99,7 +106,7 @@ struct LorQueue
 };
 int queue_room(const Sino& s);
 // column.cu: the projectors on transaxial tracks (column.cuh), which read the
-// image as doubles in z columns ([y][x][z]) and add into two accumulators of
+// image as doubles in z columns ([y][x][z]) and add into accumulators of
 // that layout, one after the other at acc, whose sum is the backprojection.
 // How a launch with blocks of about `block` threads deals the LORs of s (z: the
 // scanner's slice centres; skip: the projectors skip bins that are 0; fixed: a
@@ -149,10 +156,11 @@ void launch_column_osem(const Grid& g, const Sino& s, const Tables& t, const Col
 // LORs, where the launch on tracks leaves them to it.
 void launch_list_nonzero(const Sino& s, const ColumnPlan& p, const float* sino, const LorQueue& queue,
                          const LaunchCfg& cfg);
-void launch_queue_backward(const Grid& g, const Sino& s, const Tables& t, const float* sino, float* acc,
-                           const LorQueue& queue, const LaunchCfg& cfg);
-void launch_queue_osem(const Grid& g, const Sino& s, const Tables& t, const double* img, const float* sino,
-                       const float* mult, const float* bias, float* acc, const LorQueue& queue, const LaunchCfg& cfg);
+void launch_queue_backward(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p, const float* sino,
+                           float* acc, const LorQueue& queue, const LaunchCfg& cfg);
+void launch_queue_osem(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p, const double* img,
+                       const float* sino, const float* mult, const float* bias, float* acc, const LorQueue& queue,
+                       const LaunchCfg& cfg);
 // compact.cu: the enumerated indices of s (list null) whose bin of sino is
 // not 0, ascending, into list (s.n_enum entries), their number into *count
 // (device memory).  With temp null only *temp_bytes is set (CUB convention).
@@ -269,7 +277,7 @@ struct BatchProblem
   // wide, img and bp with x and y exchanged ([z][x][y]), for LORs running
   // mostly along x; bp_t is added into bp by the EM step.  Problems with the
   // double copy have wide_t, those that gather floats img_t (null: none).
-  // With columns (column.cu) wide is in z columns, bp the two accumulators
+  // With columns (column.cu) wide is in z columns, bp the accumulators
   // there, and these are null.
   double* wide_t;
   float* bp_t;

@@ -39,14 +39,14 @@ __device__ __forceinline__ void flag(int* check, int bit)
 // image itself (widened per step, exact; for volumes whose double copy does
 // not fit in L2 beside the accumulator).
 //
-// kColumns: the images are in z columns (column.cuh); img_t is img, and bp_t
-// the second of the two accumulators.
+// kColumns: the images are in z columns (column.cuh); img_t is img, bp_t is bp,
+// the accumulators, and views the number of the subset's views.
 template<bool kWeighted, typename TImg = double, bool kColumns = false>
 __device__ __forceinline__ void osem_lor_body(const Grid& g, const Sino& s, int subset, const Tables& t,
                                               const TImg* __restrict__ img, const TImg* __restrict__ img_t,
                                               const float* __restrict__ sino, const float* __restrict__ mult,
                                               const float* __restrict__ bias, float* bp, float* bp_t,
-                                              bool skip_zero, int i, int* check, int orient = -1)
+                                              bool skip_zero, int i, int* check, int orient = -1, int views = 0)
 {
   bool valid = false;
   const int ie = enum_index(s, i, valid);
@@ -75,6 +75,10 @@ __device__ __forceinline__ void osem_lor_body(const Grid& g, const Sino& s, int 
   }
   const TImg* im = tr ? img_t : img;
   float* b = tr ? bp_t : bp;
+  if (kColumns)
+  {
+    b += (size_t)((tr ? 1 : 0) + (2 * (l.view / s.n_subsets) >= views ? 2 : 0)) * g.nxy * g.nz;
+  }
   // b may come from a descriptor in memory, not a kernel parameter: without
   // this the compiler cannot tell the atomic's address space and tests it at
   // every step.

@@ -191,3 +191,116 @@ def test_skipped_bins_at_any_occupancy(occupied, span):
     for a, b in zip(*out):
         assert np.linalg.norm(a - b) <= 1e-6 * np.linalg.norm(b)
         assert np.array_equal(a > 0, b > 0)
+
+
+# rings, crystals, segments, span, tangential bins, size, voxel, z offset, geometry, block size
+REF, EXACT = capi.FIR_GEOMETRY_REFERENCE, capi.FIR_GEOMETRY_EXACT
+PATHS = {
+    # z clips 2 to 3 % of the LORs, at both ends of the volume or at one
+    "clipped": (16, 192, 31, 1, 71, (50, 46, 28), (4.0, 4.0, 2.0), 0.0, REF, 0),
+    "clipped_one_end": (16, 192, 31, 1, 71, (50, 46, 30), (4.0, 4.0, 2.0), 2.5, REF, 0),
+    "clipped_blocks_of_256": (16, 192, 31, 1, 71, (50, 46, 28), (4.0, 4.0, 2.0), 0.0, REF, 256),
+    "clipped_blocks_of_32": (16, 192, 31, 1, 71, (50, 46, 28), (4.0, 4.0, 2.0), 0.0, REF, 32),
+    # two tracks per block
+    "clipped_two_tracks": (10, 384, 19, 1, 71, (90, 90, 18), (3.0, 3.0, 2.0), 0.0, REF, 0),
+    # extents truncated to whole millimetres: paths leave the slices early
+    "truncated": (16, 192, 31, 1, 71, (50, 46, 27), (3.3, 3.7, 2.4), 0.0, REF, 0),
+    # extents that are not whole, two plane offsets per segment
+    "fractional": (16, 192, 31, 1, 71, (51, 45, 40), (3.3, 2.7, 1.6), 0.0, EXACT, 0),
+    "span_3_clipped": (20, 192, 13, 3, 71, (47, 51, 37), (4.0, 4.0, 2.0), 0.0, REF, 0),
+}
+
+
+def path_case(name):
+    r, n, seg, span, tang, size, voxel, off, geometry, block = PATHS[name]
+    scanner = ScannerSpec.ring(r, n, 170.0, 4.0)
+    proj, vol = ProjSpec(r, n, seg, tang, span), VolSpec.centred(size, voxel, off)
+    plan = capi.track_plan(scanner, proj, vol, geometry=geometry, block_size=block)
+    assert plan.forward_on_tracks and plan.backward_on_tracks and plan.osem_on_tracks
+    assert (plan.general > 1e-3) == (name != "fractional")
+    assert plan.block_tracks == {"clipped_two_tracks": 2, "clipped_blocks_of_256": 2}.get(name, 1)
+    track, single = contexts(scanner, geometry)
+    track.set_option(capi.FIR_OPT_BLOCK_SIZE, block)
+    return track, single, proj, vol
+
+
+@pytest.mark.parametrize("name", sorted(PATHS))
+def test_projection_is_bit_identical(name):
+    track, single, proj, vol = path_case(name)
+    x = np.random.default_rng(5).random(vol.shape_zyx, dtype=np.float32)
+    got, want = forward_both(track, single, proj, vol, x)
+    np.testing.assert_array_equal(got, want)
+    track.forward_exp(vol, x * np.float32(0.01), proj, got)
+    single.forward_exp(vol, x * np.float32(0.01), proj, want)
+    np.testing.assert_array_equal(got, want)
+
+
+# A voxel sums some 1e4 floats: 1e-6 of the norm as in the repository's other
+# comparisons of float atomics, here against sums in 64 bits of the same terms
+# (the multi-frame backprojection, which traces LOR by LOR).
+@pytest.mark.parametrize("name", sorted(PATHS))
+@pytest.mark.parametrize("skip", [0, 1])
+def test_backprojections_agree(name, skip):
+    track, single, proj, vol = path_case(name)
+    nb = capi.proj_geometry(proj)["n_bins"]
+    rng = np.random.default_rng(6)
+    y = rng.poisson(1.0, nb).astype(np.float32)  # 37 % of the bins are 0
+    m = rng.random(nb, dtype=np.float32) + np.float32(0.2)
+    bias = rng.random(nb, dtype=np.float32)
+    x = rng.random(vol.shape_zyx, dtype=np.float32) + np.float32(0.1)
+    track.set_option(capi.FIR_OPT_SKIP_ZERO_BINS, skip)
+    sens = np.ones((1,) + vol.shape_zyx, np.float32)
+    back, ones, ratio = (np.zeros(vol.shape_zyx, np.float32) for _ in range(3))
+    track.backward(proj, y, vol, back)
+    track.sensitivity(proj, vol, ones)
+    track.ratio_backprojection(proj, y, vol, x, ratio, bias=bias)
+    osem = x.copy()
+    track.osem(proj, y, vol, osem, sens, OSEMParams(n_iterations=1, n_subsets=1), bias=bias, mult=m)
+    assert track.track_launch_count == 4
+
+    def wide(bins):
+        out = np.zeros((1,) + vol.shape_zyx)
+        single.backward_frames(proj, bins[None].astype(np.float64), vol, out)
+        return out[0]
+
+    def over(estimate):
+        with np.errstate(divide="ignore", invalid="ignore"):
+            return np.where(estimate > 1e-5, y / estimate, np.float32(0))
+
+    line = np.zeros(nb, np.float32)
+    single.forward(vol, x, proj, line)
+    want_osem = wide(over(line * m + bias) * m)
+    want_osem = np.where(want_osem > 1e-5, x * want_osem, 0.0)
+    assert single.track_launch_count == 0
+    for got, want in ((back, wide(y)), (ones, wide(np.ones(nb, np.float32))), (ratio, wide(over(line + bias))),
+                      (osem, want_osem)):
+        assert np.linalg.norm(got.astype(np.float64) - want) <= 1e-6 * np.linalg.norm(want)
+        assert np.array_equal(got != 0, want != 0)
+
+
+def test_rounding_is_no_larger_than_lor_by_lor():
+    """The backprojection's distance from sums in 64 bits, on a subset of the
+    clinical scanner's bins."""
+    import torch
+
+    scanner, proj = ScannerSpec.ring(32, 512, 400.0, 4.0), ProjSpec(32, 512, 63, 125)
+    vol = VolSpec.centred((200, 200, 64), (3.0, 3.0, 3.0))
+    assert capi.track_plan(scanner, proj, vol, n_subsets=16).backward_on_tracks
+    track, single = contexts(scanner)
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    nb = capi.proj_geometry(proj)["n_bins"]
+    y = 0.5 + torch.rand(nb, generator=gen, device="cuda")
+    wide = torch.zeros((1,) + vol.shape_zyx, device="cuda", dtype=torch.float64)
+    at, only = 0, torch.zeros_like(y)
+    for seg in range(-31, 32):  # the views of subset 3
+        n = (32 - abs(seg)) * 125
+        only[at:at + 256 * n].view(256, n)[3::16] = y[at:at + 256 * n].view(256, n)[3::16]
+        at += 256 * n
+    single.backward_frames(proj, only[None].double(), vol, wide)
+    error = []
+    for c in (track, single):
+        out = torch.zeros((16,) + vol.shape_zyx, device="cuda")
+        c.backward(proj, y, vol, out, 16)
+        c.synchronize()
+        error.append(float((out[3].double() - wide[0]).norm() / wide.norm()))
+    assert error[0] <= error[1] <= 1e-6, error
