@@ -154,18 +154,26 @@ class _Penalty(torch.autograd.Function):
         return g * gy, None
 
 
+def _outside_transforms(x) -> bool:
+    """Whether x is outside function transforms, forward-mode duals, dispatch
+    and torch-function modes and tracing.  torch tells some of these by names
+    of its own, which a release may change: without them the answer is no."""
+    try:
+        return (torch._C._functorch.peek_interpreter_stack() is None
+                and not torch._C._functorch.is_functorch_wrapped_tensor(x)
+                and torch.autograd.forward_ad._current_level < 0
+                and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
+                and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
+    except (AttributeError, TypeError):
+        return False
+
+
 def _plain_cuda_image(x, beta) -> bool:
-    """Whether x is an ordinary CUDA image outside every transform (function
-    transforms, forward-mode duals, dispatch and torch-function modes, tracing)
-    and beta a number: only then a kernel may stand in for the operations."""
+    """Whether x is an ordinary CUDA image outside every transform and beta a
+    number: only then a kernel may stand in for the operations."""
     return (type(x) in (torch.Tensor, torch.nn.Parameter) and x.is_cuda and x.layout == torch.strided
             and x.dtype in (torch.float32, torch.float64) and x.dim() >= 3 and 0 < x.numel() < 2 ** 31
-            and isinstance(beta, (int, float))
-            and torch._C._functorch.peek_interpreter_stack() is None
-            and not torch._C._functorch.is_functorch_wrapped_tensor(x)
-            and torch.autograd.forward_ad._current_level < 0
-            and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
-            and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
+            and isinstance(beta, (int, float)) and _outside_transforms(x))
 
 
 def quadratic_penalty(x: torch.Tensor, beta: float) -> torch.Tensor:
