@@ -172,6 +172,7 @@ def _plain_cuda_image(x, beta) -> bool:
     """Whether x is an ordinary CUDA image outside every transform and beta a
     number: only then a kernel may stand in for the operations."""
     return (type(x) in (torch.Tensor, torch.nn.Parameter) and x.is_cuda and x.layout == torch.strided
+            and not x.is_neg()  # (a view whose memory holds the negated values)
             and x.dtype in (torch.float32, torch.float64) and x.dim() >= 3 and 0 < x.numel() < 2 ** 31
             and isinstance(beta, (int, float)) and _outside_transforms(x))
 

@@ -24,3 +24,11 @@ def test_a_torch_without_its_private_names_takes_the_operations(claims_cuda, mon
     monkeypatch.delattr(holder, name)
     assert not autograd._plain_cuda_image(x, 0.5)
     assert torch.equal(autograd.quadratic_penalty(x, 0.5), want)
+
+
+def test_a_negated_view_takes_the_operations(claims_cuda):
+    """Its memory holds the other signs, and contiguous() leaves it so."""
+    x = torch._neg_view(torch.rand(2, 3, 4))
+    assert x.contiguous().data_ptr() == x.data_ptr()
+    assert not autograd._plain_cuda_image(x, 0.5)
+    assert autograd._plain_cuda_image(x.resolve_neg(), 0.5)
