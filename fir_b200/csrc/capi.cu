@@ -518,31 +518,20 @@ ColumnPlan columns_for(const fir_ctx& c, const Grid& g, const Sino& s, bool skip
   return p;
 }
 
-// Whether b holds n bytes, or can be made to: not while the stream is being
+// Whether the context may allocate n bytes: not while its stream is being
 // captured (an allocation would end the capture), nor where the device has no
 // room for them.
-bool can_hold(const fir_ctx& c, DevBuf& b, size_t n)
+bool can_allocate(const fir_ctx& c, size_t n)
 {
-  if (b.bytes >= n)
-  {
-    return true;
-  }
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(c.stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone)
+  size_t room = 0, all = 0;
+  const bool yes = cudaStreamIsCapturing(c.stream, &capture) == cudaSuccess &&
+                   capture == cudaStreamCaptureStatusNone && cudaMemGetInfo(&room, &all) == cudaSuccess && room >= n;
+  if (!yes)
   {
     cudaGetLastError();
-    return false;
   }
-  try
-  {
-    b.ensure(n);
-    return true;
-  }
-  catch (const Failure&)
-  {
-    cudaGetLastError();
-    return false;
-  }
+  return yes;
 }
 
 // The queue of a launch on tracks, in context scratch; none without skipped
@@ -564,26 +553,51 @@ LorQueue queue_for(fir_ctx& c, const Sino& s, const ColumnPlan& p, const float* 
 }
 
 // The same plan for a launch of this context, which also needs scratch: the
-// image's double copy and the accumulators in z columns, as it uses them.  Calls
-// that the LOR-by-LOR kernels can serve without it must not fail for the lack
-// of it, so without room for it the plan has tracks = 0.
+// image's double copy, the accumulators in z columns and the queue, as it uses
+// them.  Calls that the LOR-by-LOR kernels can serve without it must not fail
+// for the lack of it, nor of what they allocate next (the backprojection, the
+// blurred image and the filter's two, 16 bytes per voxel), so without room for
+// all of it the plan has tracks = 0.
 ColumnPlan columns_here(fir_ctx& c, const Grid& g, const Sino& s, bool skip, TrackUse use)
 {
   ColumnPlan p = columns_for(c, g, s, skip, use);
-  const bool image = use != TrackUse::Backward, acc = use != TrackUse::Forward;
-  const size_t n = (size_t)g.nxy * g.nz;
-  const size_t queue = queue_bytes(s);
   if (p.tracks == 0)
   {
     return p;
   }
-  const size_t had = c.wide.bytes;
-  if ((image && !can_hold(c, c.wide, n * sizeof(double))) ||
-      (acc && !can_hold(c, c.column_acc, kColumnAccumulators * n * sizeof(float))) || (skip && !can_hold(c, c.compact, queue)))
+  const size_t n = (size_t)g.nxy * g.nz;
+  const std::pair<DevBuf*, size_t> scratch[] = {
+    {&c.wide, use != TrackUse::Backward ? n * sizeof(double) : 0},
+    {&c.column_acc, use != TrackUse::Forward ? kColumnAccumulators * n * sizeof(float) : 0},
+    {&c.compact, skip ? queue_bytes(s) : 0}};
+  size_t missing = 0;
+  for (const auto& b : scratch)
   {
-    if (c.wide.bytes > had)
+    missing += b.second > b.first->bytes ? b.second : 0;
+  }
+  if (missing == 0)
+  {
+    return p;
+  }
+  if (!can_allocate(c, missing + 4 * n * sizeof(float)))
+  {
+    p.tracks = 0;
+    return p;
+  }
+  const size_t had = c.column_acc.bytes;
+  try
+  {
+    for (const auto& b : scratch)
     {
-      c.wide.release();  // the other kernels may need the room
+      b.first->ensure(b.second);
+    }
+  }
+  catch (const Failure&)
+  {
+    cudaGetLastError();
+    if (c.column_acc.bytes > had)
+    {
+      c.column_acc.release();  // the other kernels may need the room
     }
     p.tracks = 0;
   }

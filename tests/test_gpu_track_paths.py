@@ -155,6 +155,45 @@ def test_captured_launch_keeps_its_scratch():
     assert float((x.double() - want).norm()) <= 1e-6 * float(want.norm())
 
 
+def test_scratch_leaves_room_for_the_rest_of_the_call():
+    """Where the device has room for the tracks' scratch but not for the
+    filter's as well, the sub-iteration runs LOR by LOR."""
+    import torch
+
+    scanner, proj = ScannerSpec.ring(16, 192, 170.0, 4.0), ProjSpec(16, 192, 31, 71)
+    vol = VolSpec.centred((256, 256, 256), (1.0, 1.0, 1.0))
+    assert capi.track_plan(scanner, proj, vol).osem_on_tracks
+    voxels = 256 ** 3
+    y = torch.ones(capi.proj_geometry(proj)["n_bins"], device="cuda")
+    sens = torch.ones(vol.shape_zyx, device="cuda")
+    prm = OSEMParams(n_subsets=1, convolution_interval=1, fwhm_xyz=(4.0, 4.0, 4.0))
+
+    def run(limit, launches_on_tracks):
+        ctx = capi.Context(scanner)
+        if limit:
+            ctx.set_option(capi.FIR_OPT_STEP_LIMIT, 1 << 20)
+        x = torch.ones(vol.shape_zyx, device="cuda")
+        ctx.osem_subiteration(proj, y, vol, x, sens, prm, 0, 1)
+        ctx.synchronize()
+        assert ctx.track_launch_count == launches_on_tracks
+        return x.cpu().double()
+
+    run(False, 1)  # (loads the kernels)
+    want = run(True, 0)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    # the image takes 4 bytes per voxel, the tracks' scratch 24, the filter's 8;
+    # LOR by LOR it is 12 and 8
+    free = torch.cuda.mem_get_info()[0]
+    hog = torch.empty(free - (4 + 28) * voxels, dtype=torch.uint8, device="cuda")
+    try:
+        got = run(False, 0)
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    assert float((got - want).norm()) <= 1e-6 * float(want.norm())
+
+
 # Sums of floats in another order: 1e-6 as in the repository's other
 # comparisons of float atomics.
 @pytest.mark.parametrize("occupied", [0.0, 1e-4, 0.1, 0.49, 0.51, 1.0])
