@@ -499,31 +499,30 @@ fir_status fir_batch_create(fir_batch** out, fir_ctx* ctx, int n_problems, const
       }
     }
     const bool use_columns = c.step_limit == 0 && track_warps >= kColumnWarps;
-    auto columns_of = [&](int k) { return pays[(size_t)k] != 0; };
-    for (int k = 0; k < n_problems; ++k)
-    {
-      fir_batch::Problem& q = b->pr[(size_t)k];
-      const size_t nv = (size_t)q.v.nvox;
-      q.off_sino = take((size_t)q.p.g.n_bins * sizeof(float));
-      q.off_sens = take(nv * q.n_subsets * sizeof(float));
-      q.off_img = take(nv * sizeof(float));
+    auto lay_out = [&](bool on_tracks) {
+      off = 0;
+      for (int k = 0; k < n_problems; ++k)
       {
+        fir_batch::Problem& q = b->pr[(size_t)k];
+        const size_t nv = (size_t)q.v.nvox;
+        q.off_sino = take((size_t)q.p.g.n_bins * sizeof(float));
+        q.off_sens = take(nv * q.n_subsets * sizeof(float));
+        q.off_img = take(nv * sizeof(float));
         const Grid g = grid_of(c, q.v);
-        q.columns = use_columns && columns_of(k);
+        q.columns = on_tracks && pays[(size_t)k] != 0;
         q.exchanged = !q.columns && use_exchanged(c, g);
-        q.gather_float =
-          !q.columns && !q.exchanged && !use_exchanged(c, g, 12.0) && use_exchanged(c, g, 8.0);
+        q.gather_float = !q.columns && !q.exchanged && !use_exchanged(c, g, 12.0) && use_exchanged(c, g, 8.0);
+        q.off_wide = take(q.gather_float ? 0 : nv * sizeof(double));
+        q.off_bp = take((q.columns ? kColumnAccumulators : 1) * nv * sizeof(float));
+        q.off_wide_t = take(q.exchanged ? nv * sizeof(double) : 0);
+        q.off_bp_t = take(q.exchanged || q.gather_float ? nv * sizeof(float) : 0);
+        q.off_img_t = take(q.gather_float ? nv * sizeof(float) : 0);
+        q.off_t1 = take(q.filter ? nv * sizeof(float) : 0);
+        q.off_t2 = take(q.filter ? nv * sizeof(float) : 0);
+        q.off_xy = take(scan[(size_t)k].xy.size() * sizeof(double));
+        q.off_z = take(scan[(size_t)k].z.size() * sizeof(double));
       }
-      q.off_wide = take(q.gather_float ? 0 : nv * sizeof(double));
-      q.off_bp = take((q.columns ? kColumnAccumulators : 1) * nv * sizeof(float));
-      q.off_wide_t = take(q.exchanged ? nv * sizeof(double) : 0);
-      q.off_bp_t = take(q.exchanged || q.gather_float ? nv * sizeof(float) : 0);
-      q.off_img_t = take(q.gather_float ? nv * sizeof(float) : 0);
-      q.off_t1 = take(q.filter ? nv * sizeof(float) : 0);
-      q.off_t2 = take(q.filter ? nv * sizeof(float) : 0);
-      q.off_xy = take(scan[(size_t)k].xy.size() * sizeof(double));
-      q.off_z = take(scan[(size_t)k].z.size() * sizeof(double));
-    }
+    };
     b->desc_host.resize((size_t)n_problems);
     cuda_ok(cudaDeviceGetAttribute(&b->n_sms, cudaDevAttrMultiProcessorCount, c.device), "cudaDeviceGetAttribute");
     try
@@ -534,6 +533,19 @@ fir_status fir_batch_create(fir_batch** out, fir_ctx* ctx, int n_problems, const
       cuda_ok(cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming), "cudaEventCreate");
       cuda_ok(cudaEventCreateWithFlags(&b->ev_in, cudaEventDisableTiming), "cudaEventCreate");
       cuda_ok(cudaEventCreateWithFlags(&b->ev_out, cudaEventDisableTiming), "cudaEventCreate");
+      // LOR by LOR where the device has no room for the tracks' accumulators and
+      // the biases that may follow
+      lay_out(use_columns);
+      size_t room = 0, all = 0, later = 0;
+      for (const fir_batch::Problem& q : b->pr)
+      {
+        later += (size_t)q.p.g.n_bins * sizeof(float);
+      }
+      cuda_ok(cudaMemGetInfo(&room, &all), "cudaMemGetInfo");
+      if (use_columns && room < off + later)
+      {
+        lay_out(false);
+      }
       auto* base = static_cast<unsigned char*>(b->arena.ensure(std::max<size_t>(off, 256)));
       cuda_ok(cudaMemsetAsync(base, 0, off, c.stream), "cudaMemsetAsync");
       for (int k = 0; k < n_problems; ++k)

@@ -194,6 +194,37 @@ def test_scratch_leaves_room_for_the_rest_of_the_call():
     assert float((got - want).norm()) <= 1e-6 * float(want.norm())
 
 
+def test_a_batch_without_room_for_the_accumulators():
+    """It runs LOR by LOR: 20 bytes per voxel, on tracks 32."""
+    import torch
+
+    scanner, proj = ScannerSpec.ring(16, 192, 170.0, 4.0), ProjSpec(16, 192, 31, 71)
+    vol = VolSpec.centred((256, 256, 256), (1.0, 1.0, 1.0))
+    assert capi.track_plan(scanner, proj, vol).osem_on_tracks
+    y = np.random.default_rng(8).poisson(3.0, capi.proj_geometry(proj)["n_bins"]).astype(np.float32)
+    ones = np.ones(vol.shape_zyx, np.float32)
+    ctx = capi.Context(scanner)
+
+    def run():
+        batch = capi.Batch(ctx, [(scanner, proj, vol, OSEMParams())])
+        batch.set_data(0, y, ones)
+        batch.set_image(0, ones)
+        batch.osem()
+        out = batch.get_image(0).astype(np.float64)
+        batch.close()
+        return out
+
+    want = run()
+    torch.cuda.empty_cache()
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - 26 * 256 ** 3, dtype=torch.uint8, device="cuda")
+    try:
+        got = run()
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    assert np.linalg.norm(got - want) <= 1e-6 * np.linalg.norm(want)
+
+
 # Sums of floats in another order: 1e-6 as in the repository's other
 # comparisons of float atomics.
 @pytest.mark.parametrize("occupied", [0.0, 1e-4, 0.1, 0.49, 0.51, 1.0])
