@@ -1250,12 +1250,10 @@ void check_osem_params(const fir_osem_params* prm, const ProjInfo& p)
 }
 
 // Device-pointer body of one OSEM sub-iteration.
-void osem_subiteration_device(fir_ctx& c, const ProjInfo& p, const Tables& t, const Grid& g, const ColumnPlan& plan,
+void osem_subiteration_device(fir_ctx& c, const Sino& s, const Tables& t, const Grid& g, const ColumnPlan& plan,
                               const VolInfo& v, const float* sino, const float* mult, const float* bias, float* img,
-                              const float* sens_frame, const fir_osem_params* prm, int subset,
-                              int subiter)
+                              const float* sens_frame, const fir_osem_params* prm, int subiter)
 {
-  const Sino s = sino_of(p, prm->n_subsets, subset);
   Filter f;
   if (prm->convolution_interval > 0 && subiter % prm->convolution_interval == 0)
   {
@@ -1309,16 +1307,15 @@ void osem_subiteration_device(fir_ctx& c, const ProjInfo& p, const Tables& t, co
 // One sub-iteration of the resolution-modelling OSEM: the Gaussian B of the
 // parameters is part of the system model (projection of B x, B applied to
 // the backprojection, sens_frame already blurred).
-void osem_psf_subiteration_device(fir_ctx& c, const ProjInfo& p, const Tables& t, const Grid& g,
-                                  const ColumnPlan& plan, const VolInfo& v, const float* sino, const float* mult, const float* bias, float* img,
-                                  const float* sens_frame, const fir_osem_params* prm, int subset, int subiter)
+void osem_psf_subiteration_device(fir_ctx& c, const Sino& s, const Tables& t, const Grid& g, const ColumnPlan& plan,
+                                  const VolInfo& v, const float* sino, const float* mult, const float* bias,
+                                  float* img, const float* sens_frame, const fir_osem_params* prm, int subiter)
 {
   const size_t bytes = (size_t)v.nvox * sizeof(float);
   float* bp = static_cast<float*>(c.bp.ensure(bytes));
   float* blur = static_cast<float*>(c.psf_blur.ensure(bytes));
   cuda_ok(cudaMemcpyAsync(blur, img, bytes, cudaMemcpyDeviceToDevice, c.stream), "cudaMemcpyAsync");
   convolve_device(c, v, blur, prm->fwhm_xyz, prm->cut_radius);
-  const Sino s = sino_of(p, prm->n_subsets, subset);
   ratio_backproject(c, g, s, t, plan, blur, sino, mult, bias, bp, v.nvox);
   convolve_device(c, v, bp, prm->fwhm_xyz, prm->cut_radius);
   launch_em_update(v.nvox, img, img, bp, sens_frame, cfg_of(c));
@@ -1480,13 +1477,14 @@ void osem_run(fir_ctx& c, const fir_proj_desc* proj, const float* sino, const fl
       {
         feed->feed(subset);
       }
+      const Sino s = sino_of(p, params->n_subsets, subset);
       if (psf)
       {
-        osem_psf_subiteration_device(c, p, t, g, plan, v, dsino, dmult, dbias, dimg, sframe, params, subset, subiter);
+        osem_psf_subiteration_device(c, s, t, g, plan, v, dsino, dmult, dbias, dimg, sframe, params, subiter);
       }
       else
       {
-        osem_subiteration_device(c, p, t, g, plan, v, dsino, dmult, dbias, dimg, sframe, params, subset, subiter);
+        osem_subiteration_device(c, s, t, g, plan, v, dsino, dmult, dbias, dimg, sframe, params, subiter);
       }
       if (save != nullptr && params->save_interval > 0 && subiter % params->save_interval == 0 &&
           subiter != nsub_total)
@@ -2104,8 +2102,8 @@ fir_status fir_osem_subiteration(fir_ctx* ctx, const fir_proj_desc* proj, const 
     const float* dbias = st.in(bias, p.g.n_bins);
     const float* dsens = st.in(sens_frame, v.nvox);
     float* dimg = st.inout(img, v.nvox);
-    const ColumnPlan plan = osem_columns(c, g, sino_of(p, params->n_subsets, subset));
-    osem_subiteration_device(c, p, t, g, plan, v, dsino, nullptr, dbias, dimg, dsens, params, subset, subiter);
+    const Sino s = sino_of(p, params->n_subsets, subset);
+    osem_subiteration_device(c, s, t, g, osem_columns(c, g, s), v, dsino, nullptr, dbias, dimg, dsens, params, subiter);
     finish(c, st);
   });
 }
