@@ -1183,14 +1183,16 @@ struct Filter
   bool wanted = false;
 };
 
+bool filter_wanted(const float fwhm[3]) { return fwhm[0] > 0.0 && fwhm[1] > 0.0 && fwhm[2] > 0.0; }
+
 Filter filter_of(const VolInfo& v, const float fwhm[3])
 {
   Filter f;
-  if (!(fwhm[0] > 0.0 && fwhm[1] > 0.0 && fwhm[2] > 0.0))
+  f.wanted = filter_wanted(fwhm);
+  if (!f.wanted)
   {
     return f;
   }
-  f.wanted = true;
   f.x = gauss_taps(fwhm[0], v.d.voxel_x, false);
   f.y = gauss_taps(fwhm[1], v.d.voxel_y, false);
   f.z = gauss_taps(fwhm[2], v.d.voxel_z, true);
@@ -1198,13 +1200,19 @@ Filter filter_of(const VolInfo& v, const float fwhm[3])
   return f;
 }
 
+// The filter's two images, in one allocation: a captured fir_convolve finds them
+// after any sub-iteration that filters, in one launch or in passes.
+float* filter_scratch(fir_ctx& c, const VolInfo& v)
+{
+  return static_cast<float*>(c.conv.ensure(2 * (size_t)v.nvox * sizeof(float)));
+}
+
 // One frame filtered in place in three passes; where r >= restore - 5 fwhm it
 // is kept (restore <= 0: nowhere), then 0 where r > cut (<= 0: nowhere).
 void filter_passes(fir_ctx& c, const VolInfo& v, const Filter& f, float restore, float cut, float* img)
 {
-  const size_t bytes = (size_t)v.nvox * sizeof(float);
-  float* t1 = static_cast<float*>(c.conv1.ensure(bytes));
-  float* t2 = static_cast<float*>(c.conv2.ensure(bytes));
+  float* t1 = filter_scratch(c, v);
+  float* t2 = t1 + v.nvox;
   const LaunchCfg cfg = cfg_of(c);
   launch_conv_pass(v.d.nx, v.d.ny, v.d.nz, 0, f.x, img, t1, cfg);
   launch_conv_pass(v.d.nx, v.d.ny, v.d.nz, 1, f.y, t1, t2, cfg);
@@ -1261,14 +1269,7 @@ void osem_subiteration_device(fir_ctx& c, const Sino& s, const Tables& t, const 
   }
   // a small volume is filtered in one launch, from the EM step's scratch image
   const bool fused = f.wanted && conv_fused_fits(g.nx, g.ny, g.nz, f.x, f.y, f.z);
-  float* out = img;
-  if (fused)
-  {
-    out = static_cast<float*>(c.conv1.ensure((size_t)v.nvox * sizeof(float)));
-    // (a captured fir_convolve after this call finds its scratch, as after one
-    // that filters in passes)
-    c.conv2.ensure((size_t)v.nvox * sizeof(float));
-  }
+  float* out = fused ? filter_scratch(c, v) : img;
   if (plan.tracks > 0)
   {
     const float* acc = column_ratio_backproject(c, g, s, t, plan, img, sino, mult, bias);
@@ -1276,7 +1277,12 @@ void osem_subiteration_device(fir_ctx& c, const Sino& s, const Tables& t, const 
   }
   else
   {
-    float* bp = static_cast<float*>(c.bp.ensure((size_t)v.nvox * sizeof(float)));
+    // the filter does not need its second image before the EM step has read the
+    // backprojection
+    const bool filters = prm->convolution_interval > 0 && filter_wanted(prm->fwhm_xyz);
+    float* bp = filters || c.conv.bytes >= 2 * (size_t)v.nvox * sizeof(float)
+                  ? filter_scratch(c, v) + v.nvox
+                  : static_cast<float*>(c.bp.ensure((size_t)v.nvox * sizeof(float)));
     const float* bp_t = ratio_backproject(c, g, s, t, plan, img, sino, mult, bias, bp, v.nvox, true);
     if (bp_t != nullptr)
     {
@@ -1683,7 +1689,7 @@ fir_status fir_ctx_destroy(fir_ctx* c)
     }
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
-    for (DevBuf* b : {&c->xy, &c->z, &c->check, &c->bp, &c->conv1, &c->conv2, &c->mu, &c->wide,
+    for (DevBuf* b : {&c->xy, &c->z, &c->check, &c->bp, &c->conv, &c->mu, &c->wide,
                       &c->det, &c->det_pairs, &c->ratio, &c->frames_il, &c->frames_acc, &c->psf_blur, &c->psf_sens, &c->rebin,
                       &c->wide_t, &c->bp_t, &c->column_acc, &c->img_t, &c->frames_il_t, &c->frames_acc_t, &c->compact})
     {

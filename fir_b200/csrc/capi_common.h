@@ -160,7 +160,7 @@ struct fir_ctx
   fir::abi::DevBuf check;     // device check word
   int* check_host = nullptr;  // pinned mirror
 
-  fir::abi::DevBuf bp, conv1, conv2, mu, wide, det, det_pairs, ratio, frames_il, frames_acc, psf_blur, psf_sens, rebin;
+  fir::abi::DevBuf bp, conv, mu, wide, det, det_pairs, ratio, frames_il, frames_acc, psf_blur, psf_sens, rebin;
   fir::abi::DevBuf wide_t, bp_t;  // x/y-exchanged double image and accumulator of the fused kernel
   fir::abi::DevBuf column_acc;    // accumulators in z columns (column.cu)
   fir::abi::DevBuf img_t;         // x/y-exchanged float image (float traversal, float gathers)

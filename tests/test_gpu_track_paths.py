@@ -155,6 +155,30 @@ def test_captured_launch_keeps_its_scratch():
     assert float((x.double() - want).norm()) <= 1e-6 * float(want.norm())
 
 
+def test_a_filtered_subiteration_leaves_the_filter_its_scratch():
+    """A context whose sub-iteration filtered in one launch captures its first
+    fir_convolve, as after one that filtered in passes."""
+    import torch
+
+    scanner, proj = ScannerSpec.ring(4, 64, 120.0, 4.0), ProjSpec(4, 64, 7, 21)
+    vol = VolSpec.centred((32, 32, 8), (4.0, 4.0, 4.0))
+    fwhm = [4.0, 4.0, 4.0]
+    y = torch.ones(capi.proj_geometry(proj)["n_bins"], device="cuda")
+    x = torch.rand(vol.shape_zyx, generator=torch.Generator(device="cuda").manual_seed(9), device="cuda")
+    want = x.clone()
+    eager, ctx = capi.Context(scanner), capi.Context(scanner)
+    eager.convolve(vol, want, fwhm)
+    image = torch.ones_like(x)
+    ctx.osem_subiteration(proj, y, vol, image, torch.ones_like(x), OSEMParams(convolution_interval=1, fwhm_xyz=fwhm),
+                          0, 1)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ctx.convolve(vol, x, fwhm)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(x, want)
+
+
 def test_scratch_leaves_room_for_the_rest_of_the_call():
     """Where the device has room for the tracks' scratch but not for the
     filter's as well, the sub-iteration runs LOR by LOR."""
@@ -182,8 +206,8 @@ def test_scratch_leaves_room_for_the_rest_of_the_call():
     want = run(True, 0)
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
-    # the image takes 4 bytes per voxel, the tracks' scratch 24, the filter's 8;
-    # LOR by LOR it is 12 and 8
+    # the image takes 4 bytes per voxel, the tracks' scratch 24, the filter's 8; LOR
+    # by LOR it is 8, and 8 for the filter and the backprojection
     free = torch.cuda.mem_get_info()[0]
     hog = torch.empty(free - (4 + 28) * voxels, dtype=torch.uint8, device="cuda")
     try:
