@@ -80,7 +80,7 @@ def peaks():
 
 def profile_traffic():
     """Per-launch DRAM bytes of the OSEM kernel from the committed ncu summary."""
-    path = os.path.join(ROOT, "profiles", "osem_subset_clinical.json")
+    path = os.path.join(ROOT, "profiles", "osem_column_clinical.json")
     try:
         with open(path) as f:
             d = json.load(f)

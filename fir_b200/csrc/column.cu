@@ -6,7 +6,8 @@
 // holds twice the warps (clinical forward projection 10.96 against 10.4 ms).
 // The projections run at 48 registers, the backprojection at 64: the gathers'
 // latency wants the warps (10.0 against 10.4 ms), the atomics do not (12.1
-// against 11.9).
+// against 11.9).  48 registers cost 92 to 356 bytes of spills a thread, at the
+// edges of the walks: local accesses are 1.7 % of the instructions.
 #include "column.cuh"
 
 #include <algorithm>
@@ -450,9 +451,7 @@ __device__ __forceinline__ bool osem_ratio(float line, int bin, const float* __r
   return true;
 }
 
-// The LORs of block number `block` of one OSEM sub-iteration
-// (reconAlgos.cc:119-158, see osem_lor_body): image and accumulators in z
-// columns.
+// What becomes of bins that are 0.
 enum class ZeroBins
 {
   Trace,  // not skipped
@@ -460,6 +459,9 @@ enum class ZeroBins
   Pack    // the others packed
 };
 
+// The LORs of block number `block` of one OSEM sub-iteration
+// (reconAlgos.cc:119-158, see osem_lor_body): image and accumulators in z
+// columns.
 template<bool kWeighted, ZeroBins kZero>
 __device__ __forceinline__ void column_osem(const Grid& g, const Sino& s, const Tables& t, const ColumnPlan& p,
                                             int subset, int block, const double* __restrict__ img,

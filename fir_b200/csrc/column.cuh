@@ -30,12 +30,13 @@
 // nothing and leaves the volume after alphaMax).  Others take the general
 // walk, 32 to a warp, at the end of their block.
 //
-// Bound by instruction issue (69 % of the slots; 22 instructions per LOR and
-// step with the gather, 20 with the atomic, against 45 of the general walk),
-// then by the atomics' sectors.  Clinical scanner (32 rings x 512 crystals,
+// Bound by instruction issue (74 % of the slots in the projection, 68 % in the
+// fused kernel; 22 instructions per LOR and step with the gather, 20 with the
+// atomic, against 45 of the general walk), the backprojection by its atomics'
+// sectors (L1 78 %, L2 63 %, issue 57 %).  Clinical scanner (32 rings x 512 crystals,
 // 3.28e7 LORs, 200x200x64 voxels): forward projection 16.15 -> 9.5 ms,
 // backprojection of 16 subsets 23.0 -> 12.0 ms, OSEM sub-iteration 2.08 ->
-// 1.26 ms.
+// 1.28 ms.
 #pragma once
 
 #include "lor_body.cuh"

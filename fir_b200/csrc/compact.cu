@@ -1,5 +1,6 @@
 // The non-zero bins of a subset as a compacted enumeration (Sino::list), for
-// FIR_OPT_SKIP_ZERO_BINS.  A bin whose measured value is 0 has a ratio of
+// FIR_OPT_SKIP_ZERO_BINS where LORs are traced one by one (launches on tracks
+// have a list of their own, column.cu).  A bin whose measured value is 0 has a ratio of
 // exactly 0 in reconAlgos.cc:152-157, so its backprojection adds nothing and
 // skipping it is exact.  Skipped inside the fused kernel, such a bin still
 // holds its lane while the other lanes of the warp trace; listed out, the

@@ -128,8 +128,6 @@ struct HostTables
 double column_stops(const Grid& g, const Sino& s, const ColumnPlan& p, const HostTables& t);
 double column_general(const Grid& g, const Sino& s, const HostTables& t);
 constexpr long long kColumnWarps = 6 * 592;
-// Whether a launch with enough warps is faster on tracks than LOR by LOR (z:
-// Whether a launch with enough warps is faster on tracks than LOR by LOR.
 enum class TrackUse
 {
   Forward,
@@ -137,6 +135,7 @@ enum class TrackUse
   Osem,
   Batch  // a problem's part of a batch's launches
 };
+// Whether a launch with enough warps is faster on tracks than LOR by LOR.
 bool columns_pay(const Grid& g, const Sino& s, const ColumnPlan& p, const HostTables& t, TrackUse use);
 // out = the image's double copy in z columns; the accumulators (or null) = 0.
 void launch_to_columns(const Grid& g, const float* in, double* out, float* acc, const LaunchCfg& cfg);
@@ -277,8 +276,8 @@ struct BatchProblem
   // wide, img and bp with x and y exchanged ([z][x][y]), for LORs running
   // mostly along x; bp_t is added into bp by the EM step.  Problems with the
   // double copy have wide_t, those that gather floats img_t (null: none).
-  // With columns (column.cu) wide is in z columns, bp the accumulators
-  // there, and these are null.
+  // With columns (column.cu) wide is in z columns, bp the
+  // kColumnAccumulators there, and these are null.
   double* wide_t;
   float* bp_t;
   float* img_t;
