@@ -986,15 +986,27 @@ double column_stops(const Grid& g, const Sino& s, const ColumnPlan& p, const Hos
 // Warps of the launch that have work.
 long long column_warps(const ColumnPlan& p) { return (long long)p.tracks * ((p.pairs + p.turn - 1) / p.turn); }
 
-// Tracks need ring pairs to share them, or most of a warp's 64 slots are idle:
-// with 36 pairs (6 rings) projection and fused kernel take 1.2 and 1.1 times as
-// long as LOR by LOR, with 49 0.96 and 0.85 times; the backprojection, bound by
-// its atomics, gains at 36 too (0.67).  They also need about six warps per
-// scheduler (kColumnWarps) to hide the loops' latency (a turn waits for its
-// entry and test): the LOR-by-LOR kernels, with twice the warps, are faster
-// below that (measured 0.63x to 0.98x below 3000 warps, 1.3x and more above
-// 8000).  A stop makes a turn nearly twice as long (1.1x at 3.2 stops per turn on
-// small volumes, 0.96x at 2.3 on a 320x320x128 one).
+// Tracks need about six warps per scheduler (kColumnWarps) to hide the loops'
+// latency (a turn waits for its entry and test): the LOR-by-LOR kernels, with
+// twice the warps, are faster below that (measured 0.63x to 0.98x below 3000
+// warps, 1.3x and more above 8000).
+//
+// They also need ring pairs to fill a warp's 64 slots, and a z crossing that stops
+// a turn costs as much as the turn.  The backprojection, bound by its atomics,
+// gains all the same (1.2x to 1.6x with 25 pairs, 1.06x to 2.6x at 3 to 11 stops).
+// Projection and fused kernel, 600 geometries, tracks against LOR by LOR by the
+// share of slots filled:
+//   full (16, 32, 40, 64 rings): projection 1.3x to 1.6x at one stop, 1.1x to 1.3x
+//   at 2.2, 0.9x to 1.05x at 3 to 10; fused kernel 1.3x to 1.8x, 1.04x to 1.45x,
+//   1.0x to 1.5x
+//   0.75 (12 rings): projection 1.06x at 0.8, 0.99x at 1.5, 0.92x at 2.7; fused
+//   kernel 1.25x, 1.09x, 0.95x
+//   0.63 (9 rings): projection 1.15x at 0.3, 1.0x at 0.8, 0.92x at 1.3; fused
+//   kernel 1.24x, 1.15x, 1.05x
+// A track of one warp shares its block with others, whose walks differ in
+// length: 8 rings (full) 1.03x and 1.16x at 0.8 stops, 10 (0.78) 1.11x and 1.24x;
+// 7 rings (0.77) 0.96x and 1.03x, 6 (0.56) 0.85x and 0.9x.
+// The lines below are where these cross 1.
 //
 // A block with a LOR that z clips takes a whole walk longer, with most of its
 // warps idle, so the gain goes with the share of such LORs, and sooner where the
@@ -1008,10 +1020,12 @@ long long column_warps(const ColumnPlan& p) { return (long long)p.tracks * ((p.p
 //   projection (all views): 1.04x at 8.7 %, 1.0x at 8.2 % (span 3), 1.0x at 22 %;
 //   with 64 pairs, whose blocks hold four tracks, 0.96x at 0.13 %, 0.5x at 12 %
 //   backprojection: 1.15x to 1.4x at 20 %, even at 45 % with 36 pairs.
+// Beyond 2.2 stops too little is gained to pay for clipped LORs (64 rings, fused
+// kernel: 1.05x at 2.3 stops unclipped, 0.94x at 1 %; 1.2x and 0.92x at 3.7).
 bool columns_pay(const Grid& g, const Sino& s, const ColumnPlan& p, const HostTables& t, TrackUse use)
 {
   const bool back = use == TrackUse::Backward;
-  if (g.exact_only || p.pairs < (back ? 30 : 44) || column_smem(p) > kColumnSharedLimit ||
+  if (g.exact_only || p.pairs < 30 || column_smem(p) > kColumnSharedLimit ||
       (long long)g.nxy * g.nz >= 1LL << 29)
   {
     return false;
@@ -1021,9 +1035,18 @@ bool columns_pay(const Grid& g, const Sino& s, const ColumnPlan& p, const HostTa
     return false;  // beyond the tile grid of the z-column copies
   }
   const long long warps = use == TrackUse::Batch ? 12000 : column_warps(p);
-  const double most =
-    back ? 0.2 : (p.pairs <= 64 || warps < 12000 ? 3e-4 : (warps < 25000 ? 0.012 : 0.08));
-  return column_stops(g, s, p, t) <= 2.2 && column_general(g, s, t) <= most;
+  double most = 0.2;
+  if (!back)
+  {
+    const double fill = p.pairs / (64.0 * ((p.pairs + 63) / 64)) * (p.pairs <= 64 ? 0.78 : 1.0);
+    const double stops = column_stops(g, s, p, t);
+    if (stops > (use == TrackUse::Forward ? 6.3 * (fill - 0.55) : 9.0 * (fill - 0.5)))
+    {
+      return false;
+    }
+    most = p.pairs <= 64 || warps < 12000 || stops > 2.2 ? 3e-4 : (warps < 25000 ? 0.012 : 0.08);
+  }
+  return column_general(g, s, t) <= most;
 }
 
 void launch_to_columns(const Grid& g, const float* in, double* out, float* acc, const LaunchCfg& cfg)

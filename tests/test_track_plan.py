@@ -173,3 +173,24 @@ def test_few_rings_and_long_volumes():
     for nz, on in ((65535 * 32, 1), (65535 * 32 + 1, 0)):
         plan = capi.track_plan(scanner, proj, VolSpec.centred((1, 1, nz), (2.0, 2.0, 2.0)))
         assert plan.backward_on_tracks == on and plan.osem_on_tracks == on
+
+
+# rings, crystals, radius, pitch, size, voxel; routes (forward, backward, fused).
+# Exact geometry, span 1, nothing clipped but where named.
+@pytest.mark.parametrize("rings,crystals,radius,pitch,size,voxel,routes", [
+    (16, 256, 250.0, 4.0, (64, 64, 43), (4.0, 4.0, 1.6), (1, 1, 1)),        # full warps, 1.8 stops
+    (16, 256, 250.0, 4.0, (64, 64, 38), (4.0, 4.0, 1.8181818), (0, 1, 1)),  # 3.2
+    (16, 256, 250.0, 4.0, (64, 64, 54), (4.0, 4.0, 1.3), (0, 1, 0)),        # 6.5
+    (12, 320, 250.0, 4.0, (64, 64, 19), (4.0, 4.0, 3.0), (1, 1, 1)),        # three quarters of the slots, 0.9
+    (12, 320, 250.0, 4.0, (64, 64, 29), (4.0, 4.0, 1.8181818), (0, 1, 1)),  # 2.1
+    (9, 384, 250.0, 4.0, (128, 128, 12), (2.5, 2.5, 4.0), (1, 1, 1)),       # 0.63 of the slots, 0.1
+    (9, 384, 250.0, 4.0, (64, 64, 15), (4.0, 4.0, 3.0), (0, 1, 1)),         # 0.7
+    (7, 384, 250.0, 4.0, (64, 64, 13), (4.0, 4.0, 2.4), (0, 1, 0)),         # one warp per track, 1.0
+    (64, 640, 410.0, 3.2, (320, 320, 144), (1.5, 1.5, 1.5), (1, 1, 1)),     # 2.3
+    (64, 640, 410.0, 3.2, (320, 320, 128), (1.5, 1.5, 1.5), (0, 1, 0)),     # the same, 1 % clipped
+])
+def test_routes_by_fill_and_stops(rings, crystals, radius, pitch, size, voxel, routes):
+    plan = capi.track_plan(ScannerSpec.ring(rings, crystals, radius, pitch),
+                           ProjSpec(rings, crystals, 2 * rings - 1, crystals // 4 - 5), VolSpec.centred(size, voxel),
+                           geometry=1)
+    assert (plan.forward_on_tracks, plan.backward_on_tracks, plan.osem_on_tracks) == routes, (plan.stops, plan.general)
