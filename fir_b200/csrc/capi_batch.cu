@@ -488,9 +488,11 @@ fir_status fir_batch_create(fir_batch** out, fir_ctx* ctx, int n_problems, const
       const ScannerInfo& sc = scan[(size_t)k];
       plans[(size_t)k] = column_plan(g, s, sc.z.data(), kBatchColumnBlock, b->skip_zero, true);
       q.plan = column_plan(g, s, sc.z.data(), c.block, b->skip_zero);
-      if (column_smem(q.plan) > kColumnSharedLimit)
+      // (a batch has no queue, so where it skips bins its blocks pack the others;
+      // columns_pay has looked at this plan's shared memory)
+      if (b->skip_zero || column_smem(q.plan) > kColumnSharedLimit)
       {
-        q.plan = plans[(size_t)k];  // (columns_pay has looked at this one)
+        q.plan = plans[(size_t)k];
       }
       if (columns_pay(g, s, plans[(size_t)k], HostTables{sc.xy.data(), sc.z.data()}, TrackUse::Batch))
       {

@@ -398,3 +398,34 @@ def test_rounding_is_no_larger_than_lor_by_lor():
         c.synchronize()
         error.append(float((out[3].double() - wide[0]).norm() / wide.norm()))
     assert error[0] <= error[1] <= 1e-6, error
+
+
+@pytest.mark.parametrize("occupied", [0.01, 0.6])
+def test_a_large_problem_of_a_batch_skips_bins(occupied):
+    """Above 2^22 LORs per subset a problem has launches of its own; they pack
+    the non-zero bins of their blocks too."""
+    scanner, proj = ScannerSpec.ring(32, 256, 300.0, 4.0), ProjSpec(32, 256, 63, 65)
+    vol = VolSpec.centred((60, 56, 64), (4.0, 4.0, 2.0))
+    nb = capi.proj_geometry(proj)["n_bins"]
+    assert nb >= 1 << 22 and capi.track_plan(scanner, proj, vol, skip_zero=True).osem_on_tracks
+    rng = np.random.default_rng(10)
+    y = np.where(rng.random(nb) < occupied, rng.integers(1, 5, nb), 0).astype(np.float32)
+    ones = np.ones(vol.shape_zyx, np.float32)
+    ctx, single = capi.Context(scanner), capi.Context(scanner)
+    single.set_option(capi.FIR_OPT_STEP_LIMIT, 1 << 20)
+    ctx.set_option(capi.FIR_OPT_SKIP_ZERO_BINS, 1)
+    batch = capi.Batch(ctx, [(scanner, proj, vol, OSEMParams())])
+    batch.set_data(0, y, ones)
+    batch.set_image(0, ones)
+    batch.osem()
+    got = batch.get_image(0).astype(np.float64)
+    batch.close()
+    # (sums in 64 bits, as above: LOR by LOR, float sums of this many LORs differ
+    # from them by more than those on tracks)
+    line, want = np.zeros(nb, np.float32), np.zeros((1,) + vol.shape_zyx)
+    single.forward(vol, ones, proj, line)
+    ratio = np.divide(y, line, out=np.zeros_like(y), where=line > 1e-5)
+    single.backward_frames(proj, ratio[None].astype(np.float64), vol, want)
+    want = np.where(want[0] > 1e-5, want[0], 0.0)
+    assert np.linalg.norm(got - want) <= 1e-6 * np.linalg.norm(want)
+    assert np.array_equal(got > 0, want > 0)
