@@ -926,8 +926,10 @@ double column_general(const Grid& g, const Sino& s, const HostTables& t)
     }
     return (double)inside / s.n_cpr * direct / pairs;
   }
-  // sampled: 8 views x 5 tangential bins.  In a segment they are the first or
-  // the last planes, so it is read from both ends.
+  // sampled: 8 views x 5 tangential bins, 32 or a few more segments where there
+  // are more (the calls' host time: 127 segments 0.11 ms, sampled 0.03).  In a
+  // segment they are the first or the last planes, so it is read from both ends.
+  const int step = std::max(s.n_segments / 32, 1);
   long long general = 0, meeting = 0;
   for (int i = 0; i < 40; ++i)
   {
@@ -936,9 +938,9 @@ double column_general(const Grid& g, const Sino& s, const HostTables& t)
     {
       continue;
     }
-    meeting += pairs;
-    for (int k = 0; k < s.n_segments; ++k)
+    for (int k = (s.n_segments - 1) % step / 2; k < s.n_segments; k += step)
     {
+      meeting += s.n_axial[k];
       auto kind = [&](int axial) {
         int a1, a2;
         crystal_axial(s, k - s.seg_offset, axial, a1, a2);
