@@ -510,8 +510,12 @@ Widened widen_for_projection(fir_ctx& c, const Grid& g, const float* img)
 ColumnPlan columns_for(const fir_ctx& c, const Grid& g, const Sino& s, bool skip, TrackUse use)
 {
   const HostTables t{c.scan_xy.data(), c.scan_z.data()};
-  ColumnPlan p = column_plan(g, s, c.scan_z.data(), c.block, skip);
-  if (column_warps(p) < kColumnWarps || !columns_pay(g, s, p, t, use))
+  ColumnPlan p = column_plan(g, s, c.scan_z.data(), c.block, skip, use == TrackUse::Backward);
+  // (a packing warp has two turns where most bins are not 0; 16 rings, 4544 warps
+  // of one turn, backprojection at 20, 50, 100 % non-zero bins: 54, 69, 72 us on
+  // tracks, 57, 82, 108 LOR by LOR)
+  const long long turns = (long long)p.tracks * ((p.pairs + 63) / 64);
+  if (turns < kColumnWarps || !columns_pay(g, s, p, t, use))
   {
     p.tracks = 0;
   }
@@ -536,17 +540,18 @@ bool can_allocate(const fir_ctx& c, size_t n)
 
 // The queue of a launch on tracks, in context scratch; none without skipped
 // bins.
-size_t queue_bytes(const Sino& s) { return ((size_t)queue_room(s) + 1) * sizeof(int); }
+size_t queue_bytes(const Sino& s, TrackUse use) { return (size_t)queue_room(s, use) * sizeof(int); }
 
-LorQueue queue_for(fir_ctx& c, const Sino& s, const ColumnPlan& p, const float* sino)
+// acc: the launch's accumulators, cleared.
+LorQueue queue_for(fir_ctx& c, const Grid& g, const Sino& s, const ColumnPlan& p, TrackUse use, const float* sino,
+                   float* acc)
 {
   if (p.skip == 0)
   {
     return LorQueue{};
   }
-  int* base = static_cast<int*>(c.compact.ensure(queue_bytes(s)));
-  const LorQueue q{base + 1, base, queue_room(s)};
-  cuda_ok(cudaMemsetAsync(base, 0, sizeof(int), c.stream), "cudaMemsetAsync");
+  const LorQueue q{static_cast<int*>(c.compact.ensure(queue_bytes(s, use))),
+                   queue_count(acc, (size_t)g.nxy * g.nz), queue_room(s, use)};
   launch_list_nonzero(s, p, sino, q, cfg_of(c));
   after_launch(c);
   return q;
@@ -568,8 +573,8 @@ ColumnPlan columns_here(fir_ctx& c, const Grid& g, const Sino& s, bool skip, Tra
   const size_t n = (size_t)g.nxy * g.nz;
   const std::pair<DevBuf*, size_t> scratch[] = {
     {&c.wide, use != TrackUse::Backward ? n * sizeof(double) : 0},
-    {&c.column_acc, use != TrackUse::Forward ? kColumnAccumulators * n * sizeof(float) : 0},
-    {&c.compact, skip ? queue_bytes(s) : 0}};
+    {&c.column_acc, use != TrackUse::Forward ? column_acc_bytes(n) : 0},
+    {&c.compact, skip ? queue_bytes(s, use) : 0}};
   size_t missing = 0;
   for (const auto& b : scratch)
   {
@@ -614,11 +619,9 @@ const double* to_columns(fir_ctx& c, const Grid& g, const float* img, float* acc
   return d;
 }
 
-size_t column_acc_bytes(const Grid& g) { return (size_t)kColumnAccumulators * g.nxy * g.nz * sizeof(float); }
-
 float* column_accumulators(fir_ctx& c, const Grid& g)
 {
-  return static_cast<float*>(c.column_acc.ensure(column_acc_bytes(g)));
+  return static_cast<float*>(c.column_acc.ensure(column_acc_bytes((size_t)g.nxy * g.nz)));
 }
 
 // s with the compacted list of its bins whose measured value is not 0
@@ -667,8 +670,8 @@ void backproject_subset(fir_ctx& c, const Grid& g, const Sino& s, const Tables& 
   if (plan.tracks > 0)
   {
     float* acc = column_accumulators(c, g);
-    cuda_ok(cudaMemsetAsync(acc, 0, column_acc_bytes(g), c.stream), "cudaMemsetAsync");
-    const LorQueue queue = queue_for(c, s, plan, sino);
+    cuda_ok(cudaMemsetAsync(acc, 0, column_acc_bytes((size_t)n), c.stream), "cudaMemsetAsync");
+    const LorQueue queue = queue_for(c, g, s, plan, TrackUse::Backward, sino, acc);
     timed_launch(c, [&] {
       launch_column_backward(g, s, t, plan, sino, acc, queue, cfg_of(c));
       if (queue.list != nullptr)
@@ -741,7 +744,7 @@ const float* column_ratio_backproject(fir_ctx& c, const Grid& g, const Sino& s, 
 {
   float* acc = column_accumulators(c, g);
   const double* wide = to_columns(c, g, img, acc);
-  const LorQueue queue = queue_for(c, s, p, sino);
+  const LorQueue queue = queue_for(c, g, s, p, TrackUse::Osem, sino, acc);
   timed_launch(c, [&] {
     launch_column_osem(g, s, t, p, wide, sino, mult, bias, acc, queue, cfg_of(c));
     if (queue.list != nullptr)
@@ -1895,7 +1898,7 @@ fir_status fir_track_plan(const fir_scanner_desc* scanner, const fir_proj_desc* 
     c.scan_z = sc.z;
     const Grid g = grid_of(c, v);
     const Sino s = sino_of(p, n_subsets, subset);
-    const ColumnPlan plan = column_plan(g, s, c.scan_z.data(), c.block, skip_zero != 0);
+    const ColumnPlan plan = column_plan(g, s, c.scan_z.data(), c.block, skip_zero != 0, false);
     auto on = [&](TrackUse use) { return columns_for(c, g, s, skip_zero != 0, use).tracks > 0 ? 1 : 0; };
     out->forward_on_tracks = on(TrackUse::Forward);
     out->backward_on_tracks = on(TrackUse::Backward);

@@ -486,8 +486,8 @@ fir_status fir_batch_create(fir_batch** out, fir_ctx* ctx, int n_problems, const
       const Grid g = grid_of(geo, q.v);
       const Sino s = sino_of(q.p, q.n_subsets, 0);
       const ScannerInfo& sc = scan[(size_t)k];
-      plans[(size_t)k] = column_plan(g, s, sc.z.data(), kBatchColumnBlock, b->skip_zero, true);
-      q.plan = column_plan(g, s, sc.z.data(), c.block, b->skip_zero);
+      plans[(size_t)k] = column_plan(g, s, sc.z.data(), kBatchColumnBlock, b->skip_zero, true, true);
+      q.plan = column_plan(g, s, sc.z.data(), c.block, b->skip_zero, true);
       // (a batch has no queue, so where it skips bins its blocks pack the others;
       // columns_pay has looked at this plan's shared memory)
       if (b->skip_zero || column_smem(q.plan) > kColumnSharedLimit)

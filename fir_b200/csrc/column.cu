@@ -134,24 +134,27 @@ __device__ __forceinline__ void column_lors(const Sino& s, const Tables& t, cons
   }
 }
 
-// Ring pairs of a warp where a batch skips zero bins.
+// Where bins that are 0 are skipped and less than a share of them is left, the
+// launch leaves those to the queue, one LOR per thread of its own kernel: a
+// block would build its tracks for a few LORs, most of its warps' lanes idle.
+// (Decided block by block, the two kernels of a launch are each too short to fill
+// the GPU: 58 % of a span-3 subset, 281 us against 245 and 239.)  Listing and the
+// launch that finds nothing to do cost about 10 us.  Above the share
+// * the fused kernel traces all LORs as without skipping, those of zero bins
+//   idle.  Sub-iterations at 20, 40, 60 % non-zero bins, queue; packed as below;
+//   idle at any share: clinical 0.65, 0.97, 1.34 ms; 0.92, 1.03, 1.52; 1.43; 24 rings
+//   355, 521, 702 us; 506, 556, 871; 770; 64 rings 2.2, 3.2, 4.5 ms; 3.0, 3.5, 5.2; 6.0.
+// * the backprojection, which gains twice as much on tracks, packs the other
+//   ring pairs of a block's tracks: at 12, 20, 50 %, queue; packed; idle: clinical
+//   335, 448, 928 us; 352, 386, 580; 750; 24 rings 203, 264, 531; 235, 244, 323; 390; 64
+//   rings 1.05, 1.47, 3.2 ms; 1.28, 1.37, 2.1; 3.1.
+constexpr int kQueuePercent = 65, kQueuePercentBackward = 16;
+
+// A packing block has twice the ring pairs, as half of the bins are often 0.  A
+// batch, which has no queue, packs too (12 problems of 1e5 counts: 11.1 ms; with
+// the zero bins' lanes idle 13.2).
 constexpr int kPackedTurn = 128;
 
-// Where bins that are 0 are skipped and less than this share of them is left,
-// the launch leaves those to the queue, one LOR per thread of its own kernel: a
-// block would build its tracks for a few LORs, most of its warps' lanes idle.
-// Otherwise all LORs go along their tracks as without skipping, those of zero
-// bins idle.  (Decided block by block, the two kernels of a launch are each too
-// short to fill the GPU: 58 % of a span-3 subset, 281 us against 245 and 239.)
-// Sub-iterations of Poisson data, tracks against queue: clinical scanner
-// 1.21 ms against 0.44 at 10 % non-zero, 0.69 at 25 %, 1.32 at 61 %; 17 rings
-// 365 us against 158 at 9 %, 246 at 25 %, 415 at 55 %; 24 rings 770 us against
-// 479 at 25 %, 862 at 59 %.
-constexpr int kQueuePercent = 50;
-
-// A batch has no queue.  Its blocks pack the ring pairs of their tracks'
-// non-zero bins instead, and have twice the pairs, as half of the bins are often
-// 0 (12 problems of 1e5 counts: 11.1 ms; with the zero bins' lanes idle 13.2).
 // counts and pairs are in shared memory.
 struct PackedPairs
 {
@@ -211,6 +214,28 @@ __device__ __forceinline__ int pack_nonzero(const Sino& s, const ColumnPlan& p, 
   }
   __syncthreads();
   return all;
+}
+
+// Calls trace(lor) for the LORs that the warp's group has packed, 64 at a time,
+// two per lane.  Every thread of the block calls this.
+template<class Trace>
+__device__ __forceinline__ void packed_each(const Sino& s, const Tables& t, const ColumnPlan& p,
+                                            const ColumnShare& c, int subset, const float* __restrict__ sino,
+                                            unsigned char* smem, Trace&& trace)
+{
+  const PackedPairs q = packed_pairs(smem, p);
+  const int n = pack_nonzero(s, p, c, subset, sino, q);
+  for (int i0 = c.warp * 64; i0 < n; i0 += p.warps * 64)
+  {
+    ColumnLor lor[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+    {
+      const int i = i0 + 32 * k + (int)(threadIdx.x & 31);
+      lor[k] = column_lor(s, t, p, c, subset, i < n, i < n ? c.begin + q.pairs[c.group * p.share + i] : 0);
+    }
+    trace(lor);
+  }
 }
 
 // Whether the launch that skips zero bins leaves the others to the queue.
@@ -406,20 +431,29 @@ __global__ void __launch_bounds__(256, 4) k_column_backward(const __grid_constan
   const Leftover left = leftover(smem, p);
   build_tracks(g, s, t, p, s.subset, first, smem, left.count);
   const Track tr = track_at(smem, p.cap, c.group);
-  ColumnLor lor[2];
-  column_lors(s, t, p, c, s.subset, lor);
-  ColumnLane w[2] = {};
-  bool go[2];
-  double value[2];
-  bool on[2] = {true, true};
+  auto trace = [&](const ColumnLor lor[2]) {
+    ColumnLane w[2] = {};
+    bool go[2];
+    double value[2];
+    const bool on[2] = {true, true};
 #pragma unroll
-  for (int k = 0; k < 2; ++k)
+    for (int k = 0; k < 2; ++k)
+    {
+      value[k] = lor[k].valid && sino != nullptr ? (double)__ldg(sino + lor[k].bin) : 1.0;
+    }
+    column_setup(g, p, tr, c, lor, on, left, w, go);
+    column_scatter(tr, go, w, value, accumulator_of(g, *tr.head, acc));
+  };
+  if constexpr (kSkip)
   {
-    value[k] = lor[k].valid && sino != nullptr ? (double)__ldg(sino + lor[k].bin) : 1.0;
-    on[k] = !kSkip || value[k] != 0.0;
+    packed_each(s, t, p, c, s.subset, sino, smem, trace);
   }
-  column_setup(g, p, tr, c, lor, on, left, w, go);
-  column_scatter(tr, go, w, value, accumulator_of(g, *tr.head, acc));
+  else
+  {
+    ColumnLor lor[2];
+    column_lors(s, t, p, c, s.subset, lor);
+    trace(lor);
+  }
   column_leftover(s, t, p, s.subset, (int)blockIdx.x, first, smem, left, [&](const ColumnLor& l, const Track& own) {
     const double v = sino != nullptr ? (double)__ldg(sino + l.bin) : 1.0;
     general_scatter(g, *own.head, l.z1, l.z2, v, accumulator_of(g, *own.head, acc), check);
@@ -492,25 +526,14 @@ __device__ __forceinline__ void column_osem(const Grid& g, const Sino& s, const 
     }
     column_scatter(tr, go, w, value, accumulator_of(g, *tr.head, acc));
   };
-  ColumnLor lor[2];
   bool on[2] = {true, true};
   if constexpr (kZero == ZeroBins::Pack)
   {
-    const PackedPairs q = packed_pairs(smem, p);
-    const int n = pack_nonzero(s, p, c, subset, sino, q);
-    for (int i0 = c.warp * 64; i0 < n; i0 += p.warps * 64)
-    {
-#pragma unroll
-      for (int k = 0; k < 2; ++k)
-      {
-        const int i = i0 + 32 * k + (int)(threadIdx.x & 31);
-        lor[k] = column_lor(s, t, p, c, subset, i < n, i < n ? c.begin + q.pairs[c.group * p.share + i] : 0);
-      }
-      trace(lor, on);
-    }
+    packed_each(s, t, p, c, subset, sino, smem, [&](const ColumnLor lor[2]) { trace(lor, on); });
   }
   else
   {
+    ColumnLor lor[2];
     column_lors(s, t, p, c, subset, lor);
 #pragma unroll
     for (int k = 0; k < 2; ++k)
@@ -696,12 +719,16 @@ dim3 column_tiles(int np, int nz)
 }
 
 // out = the double copy of in in z columns; the accumulators at acc (or null)
-// = 0.
+// and the queue's count behind them = 0.
 __global__ void __launch_bounds__(kTile * kTileRows) k_to_columns(int np, int nz, const float* __restrict__ in,
                                                                   double* __restrict__ out, float* __restrict__ acc)
 {
   __shared__ float tile[kTile][kTile + 1];
   const int p0 = blockIdx.x * kTile, z0 = blockIdx.y * kTile;
+  if (acc != nullptr && blockIdx.x + blockIdx.y + threadIdx.x + threadIdx.y == 0)
+  {
+    *queue_count(acc, (size_t)np * nz) = 0;
+  }
   for (int j = threadIdx.y; j < kTile; j += kTileRows)
   {
     const int p = p0 + threadIdx.x, z = z0 + j;
@@ -807,7 +834,7 @@ size_t column_smem(const ColumnPlan& p)
 
 int column_blocks(const ColumnPlan& p) { return (p.tracks + p.per_block - 1) / p.per_block * p.blocks; }
 
-ColumnPlan column_plan(const Grid& g, const Sino& s, const double* z, int block, bool skip, bool fixed)
+ColumnPlan column_plan(const Grid& g, const Sino& s, const double* z, int block, bool skip, bool pack, bool fixed)
 {
   ColumnPlan p{};
   for (int k = 0; k < s.n_segments; ++k)
@@ -821,7 +848,7 @@ ColumnPlan column_plan(const Grid& g, const Sino& s, const double* z, int block,
   // a ring
   const double apart = s.n_rings > 1 ? std::fabs(z[2] - z[0]) * (s.span > 1 ? 0.5 : 1.0) : 0.0;
   p.interleave = apart >= 1.6 * g.ext[2] ? 1 : 0;
-  p.turn = skip && fixed ? kPackedTurn : 64;
+  p.turn = skip && pack ? kPackedTurn : 64;
   const int warps = std::max((p.pairs + p.turn - 1) / p.turn, 1);
   // a track's warps in equal blocks of nearly the wanted size: the count
   // that leaves the fewest warps idle
@@ -1100,7 +1127,10 @@ void launch_column_backward(const Grid& g, const Sino& s, const Tables& t, const
   kernel<<<(unsigned)column_blocks(p), p.block, bytes, cfg.stream>>>(g, s, t, p, sino, acc, queue, cfg.check);
 }
 
-int queue_room(const Sino& s) { return (int)((long long)s.n_enum * kQueuePercent / 100) + 1; }
+int queue_room(const Sino& s, TrackUse use)
+{
+  return (int)((long long)s.n_enum * (use == TrackUse::Backward ? kQueuePercentBackward : kQueuePercent) / 100) + 1;
+}
 
 void launch_list_nonzero(const Sino& s, const ColumnPlan& p, const float* sino, const LorQueue& queue,
                          const LaunchCfg& cfg)

@@ -32,7 +32,7 @@ struct ColumnPlan
   int block;      // threads per block
   int blocks;     // blocks per track
   int share;      // ring pairs of a block's part of a track
-  int turn;       // ring pairs of a warp: 64, or 128 where it packs the non-zero bins
+  int turn;       // ring pairs of a warp: 64, or 128 where the block packs the non-zero bins
   int warps;      // warps of a block that serve one track
   int per_block;  // tracks per block
   int cap;        // crossings of a track: at most nx + ny
@@ -48,6 +48,13 @@ size_t column_smem(const ColumnPlan& p);
 // whose warps add up some of their atomics first, 1.58e-7), four 1.2e-7
 // (and 10 us of 1.27 ms more).
 constexpr int kColumnAccumulators = 4;
+// The accumulators of nvox voxels and, behind them, the count of the queue that
+// a launch with skipped bins may leave LORs to (LorQueue): cleared together.
+constexpr size_t column_acc_bytes(size_t nvox) { return (kColumnAccumulators * nvox + 4) * sizeof(float); }
+__host__ __device__ inline int* queue_count(float* acc, size_t nvox)
+{
+  return reinterpret_cast<int*>(acc + kColumnAccumulators * nvox);
+}
 // The most that a plan may ask for.
 constexpr size_t kColumnSharedLimit = 96 * 1024;
 
@@ -104,14 +111,15 @@ struct LorQueue
   int* count;
   int room;
 };
-int queue_room(const Sino& s);
 // column.cu: the projectors on transaxial tracks (column.cuh), which read the
 // image as doubles in z columns ([y][x][z]) and add into accumulators of
 // that layout, one after the other at acc, whose sum is the backprojection.
 // How a launch with blocks of about `block` threads deals the LORs of s (z: the
-// scanner's slice centres; skip: the projectors skip bins that are 0; fixed: a
-// batch's launch, of blocks of exactly that size and without a queue).
-ColumnPlan column_plan(const Grid& g, const Sino& s, const double* z, int block, bool skip, bool fixed = false);
+// scanner's slice centres; skip: the projector skips bins that are 0; pack: its
+// blocks pack the others, as the backprojection's and a batch's do; fixed: a
+// batch's launch, of blocks of exactly that size).
+ColumnPlan column_plan(const Grid& g, const Sino& s, const double* z, int block, bool skip, bool pack,
+                       bool fixed = false);
 int column_blocks(const ColumnPlan& p);
 // Warps of the launch that have work; below kColumnWarps a launch alone is
 // faster LOR by LOR.
@@ -135,9 +143,11 @@ enum class TrackUse
   Osem,
   Batch  // a problem's part of a batch's launches
 };
+int queue_room(const Sino& s, TrackUse use);
 // Whether a launch with enough warps is faster on tracks than LOR by LOR.
 bool columns_pay(const Grid& g, const Sino& s, const ColumnPlan& p, const HostTables& t, TrackUse use);
-// out = the image's double copy in z columns; the accumulators (or null) = 0.
+// out = the image's double copy in z columns; the accumulators and the queue's
+// count behind them (acc null: none) = 0.
 void launch_to_columns(const Grid& g, const float* in, double* out, float* acc, const LaunchCfg& cfg);
 // out = the accumulators' sum in [z][y][x].
 void launch_from_columns(const Grid& g, const float* acc, float* out, const LaunchCfg& cfg);

@@ -146,10 +146,11 @@ typedef enum fir_option
   /* 1: skip sinogram bins whose value is exactly 0 in backprojection and
    * OSEM (their contribution is exactly 0).  Default 0.  In the atomic mode
    * the OSEM sub-iteration and fir_backward first list a subset's non-zero
-   * bins on the device (5 bytes of context scratch per LOR of the subset, 2 on
+   * bins on the device (5 bytes of context scratch per LOR of the subset, 2.6 on
    * transaxial tracks) and trace only those; on tracks (fir_track_plan) they do
-   * so where fewer than half of the bins are non-zero, and otherwise leave the
-   * zero bins' lanes idle.  The result equals the full enumeration's up to the
+   * so where few enough are (65 % of the bins, 16 % for fir_backward), and
+   * otherwise trace all with the zero bins' lanes idle, or pack the others block
+   * by block.  The result equals the full enumeration's up to the
    * order of the float atomic additions. */
   FIR_OPT_SKIP_ZERO_BINS = 3,
   /* Threads per block of the projector kernels (32..256, multiple of 32);

@@ -251,11 +251,12 @@ def test_a_batch_without_room_for_the_accumulators():
 
 # Sums of floats in another order: 1e-6 as in the repository's other
 # comparisons of float atomics.
-@pytest.mark.parametrize("occupied", [0.0, 1e-4, 0.1, 0.49, 0.51, 1.0])
+@pytest.mark.parametrize("occupied", [0.0, 1e-4, 0.1, 0.159, 0.161, 0.4, 0.649, 0.651, 1.0])
 @pytest.mark.parametrize("span", [1, 3])
 def test_skipped_bins_at_any_occupancy(occupied, span):
-    """Below half of the bins non-zero a launch on tracks leaves them to the
-    general walk, above it traces all; both equal the LOR-by-LOR route."""
+    """Below 65 % of the bins non-zero (backprojection: 16 %) a launch on tracks
+    leaves them to the general walk, above it traces all (packs them); both equal
+    the LOR-by-LOR route."""
     if span == 1:
         scanner, proj, vol = (ScannerSpec.ring(15, 96, 150.0, 5.0), ProjSpec(15, 96, 29, 27),
                               VolSpec.centred((50, 46, 40), (3.0, 3.0, 2.0)))
